@@ -112,19 +112,19 @@ __device__ double block_sum(const double *v, int n, double *part /* >= 33 */)
     return r;
 }
 
-// FP32 block reductions (max, sum) over ADAPT_NT threads; f = shared scratch
-// of >= 33 floats.  Result broadcast to all threads.
-template <int ADAPT_NT, bool MAX>
+// FP32 block reductions (max, sum) over the first RED_NT threads; f = shared
+// scratch of >= 33 floats.  Result broadcast to all threads.
+template <int RED_NT, bool MAX>
 __device__ float block_reduce_f(float v, float *f)
 {
-    constexpr int NW = ADAPT_NT / 32;
+    constexpr int NW = RED_NT / 32;
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
         const float o = __shfl_xor_sync(0xffffffffu, v, off);
         v = MAX ? fmaxf(v, o) : v + o;
     }
-    if (lane == 0) f[w] = v;
+    if (lane == 0 && w < NW) f[w] = v;
     __syncthreads();
     if (w == 0) {
         float z = lane < NW ? f[lane] : 0.f;
@@ -143,11 +143,12 @@ __device__ float block_reduce_f(float v, float *f)
 
 // FP32 mode, alpha > 0 with training data: the weights of one axis (average,
 // 3-tap smoothing, normalisation, damping; pyx:539-562) in FP32 on the MUFU,
-// written to avg[] as doubles.  A normalised weight outside the float range
+// written to avg[] as doubles.  The FP32 sum is formed by SUM_NT threads, so that
+// it does not depend on the size of the CTA that adapts.  A normalised weight outside the float range
 // (or within 1e-5 of 1) is formed and damped in FP64, so tiny weights keep
 // the reference's ((1 - v) / -ln v)^alpha.  The cumulative sums and the new
 // nodes (regrid) stay FP64.
-template <int ADAPT_NT>
+template <int ADAPT_NT, int SUM_NT>
 __device__ void adapt_weights_fast(const AdaptArgs &a, int d, int K, double *avg, double *tmp, double *part)
 {
     const int t = threadIdx.x;
@@ -176,8 +177,9 @@ __device__ void adapt_weights_fast(const AdaptArgs &a, int d, int K, double *avg
     mx = block_reduce_f<ADAPT_NT, true>(mx, pf);
     const float rmx = mx > 0.f ? 1.f / mx : 0.f;   // sum of values scaled by the max: no overflow
     float sp = 0.f;
-    for (int i = t; i < K; i += ADAPT_NT) sp += sf[i] * rmx;
-    sp = block_reduce_f<ADAPT_NT, false>(sp, pf);
+    if (t < SUM_NT)
+        for (int i = t; i < K; i += SUM_NT) sp += sf[i] * rmx;
+    sp = block_reduce_f<SUM_NT, false>(sp, pf);
     const float rs = sp > 0.f ? 1.f / sp : 0.f;
     const float alf = (float)a.alpha;
     for (int i = t; i < K; i += ADAPT_NT) {
@@ -202,7 +204,7 @@ __device__ void adapt_weights_fast(const AdaptArgs &a, int d, int K, double *avg
 // memory, max_old + 1 and max_old doubles) the axis' old nodes and
 // increments are staged there first, so new_grid / new_inc may be the grid
 // itself (adapt in place).
-template <int ADAPT_NT>
+template <int ADAPT_NT, int SUM_NT = ADAPT_NT>
 __device__ void adapt_axis(const AdaptArgs &a, int d, double *avg, double *tmp, double *part,
                            double *gs = nullptr, double *is = nullptr)
 {
@@ -211,7 +213,7 @@ __device__ void adapt_axis(const AdaptArgs &a, int d, double *avg, double *tmp, 
     const int t = threadIdx.x;
     const double alpha = a.alpha;
     if (alpha > 0 && K > 1 && a.fast && a.sum_f != nullptr) {
-        adapt_weights_fast<ADAPT_NT>(a, d, K, avg, tmp, part);
+        adapt_weights_fast<ADAPT_NT, SUM_NT>(a, d, K, avg, tmp, part);
     } else if (alpha != 0 && K > 1) {
         if (a.sum_f != nullptr) {
             for (int i = t; i < K; i += ADAPT_NT) {

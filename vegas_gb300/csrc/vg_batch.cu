@@ -49,6 +49,14 @@ size_t smem_budget(int minb)
     return b < cap ? b : cap;
 }
 
+size_t range_smem(int ntb, int dim, int maxK, int tab_len, int train, size_t budget, int *table, int *copies)
+{
+    if (ntb == 256) return vg::range_fit<256>(dim, maxK, tab_len, train, 1, budget, table, copies).total;
+    if (ntb == 512) return vg::range_fit<512>(dim, maxK, tab_len, train, 1, budget, table, copies).total;
+    if (ntb == 768) return vg::range_fit<768>(dim, maxK, tab_len, train, 1, budget, table, copies).total;
+    return vg::range_fit<1024>(dim, maxK, tab_len, train, 1, budget, table, copies).total;
+}
+
 int bucket_of(int dim) { return dim <= 4 ? 0 : (dim <= 8 ? 1 : 2); }
 
 int occupancy_dispatch(int b, int kind, int cfg, size_t smem, int *per_sm)
@@ -176,31 +184,26 @@ extern "C" int vg_batch_prepare(const vg_integrator *its, int njobs, int kind, c
         J.bucket = b;
         present[b] = 1;
         IterArgs &a = J.a;
-        const int TT = vg::NT * C.S;
         const size_t budget = smem_budget(C.minb);
-        a.tab_len = tab_len;
-        a.T = TT;
         a.ncta = 1;
-        const int bins = a.train;
-        // over budget: the grid table goes first (read through L1), then the
-        // training histogram (global atomics)
-        a.table_smem = 1;
-        a.hist_smem = bins;
-        auto plan = [&](int table, int hist) {
-            return f64 ? vg::smem_plan<double>(dim, a.maxK, TT, table, hist, tab_len, bins, 1)
-                       : vg::smem_plan<float>(dim, a.maxK, TT, table, hist, tab_len, bins, 1);
-        };
-        vg::SmemPlan p = plan(1, a.hist_smem);
-        if (p.total > budget) {
-            a.table_smem = 0;
-            p = plan(0, a.hist_smem);
+        size_t need;
+        if (f64) {
+            const int TT = vg::NT * F64_S;
+            a.T = TT;
+            // over budget: the grid table goes first (read through L1), then the
+            // training histogram (global atomics)
+            a.table_smem = 1;
+            a.hist_smem = a.train;
+            vg::SmemPlan p = vg::smem_plan<vg::NT>(dim, a.maxK, TT, 1, a.hist_smem, a.train, 1);
+            if (p.total > budget) p = vg::smem_plan<vg::NT>(dim, a.maxK, TT, a.table_smem = 0, a.hist_smem, a.train, 1);
+            if (p.total > budget && a.hist_smem)
+                p = vg::smem_plan<vg::NT>(dim, a.maxK, TT, 0, a.hist_smem = 0, a.train, 1);
+            need = p.total;
+        } else {
+            a.tab_len = tab_len;
+            need = range_smem(C.ntb, dim, a.maxK, tab_len, a.train, budget, &a.table_smem, &a.hist_smem);
         }
-        if (p.total > budget && a.hist_smem) {
-            a.hist_smem = 0;
-            p = plan(0, 0);
-        }
-        if (p.total > 220 * 1024) return vg_fail(VG_ERR_UNSUPPORTED, "shared memory plan too large");
-        size_t need = p.total;
+        if (need > 220 * 1024) return vg_fail(VG_ERR_UNSUPPORTED, "shared memory plan too large");
         J.adapt = (it->adapt && it->alpha > 0) ? 1 : 0;
         if (J.adapt) {
             vgadapt::AdaptArgs &ad = J.ad;
@@ -224,7 +227,7 @@ extern "C" int vg_batch_prepare(const vg_integrator *its, int njobs, int kind, c
             ad.max_old = max_old;
             ad.sequential = 1;
             ad.fast = f64 ? 0 : 1;
-            const size_t an = sizeof(double) * (2 * (size_t)max_old + vg::NT);
+            const size_t an = sizeof(double) * (2 * (size_t)max_old + 64);
             need = an > need ? an : need;
         }
         J.out = out + (size_t)j * 3 * nitn;

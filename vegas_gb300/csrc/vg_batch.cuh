@@ -1,9 +1,8 @@
 // vg_batch.cuh -- many independent vegas+ integrals in one persistent launch.
 //
 // One CTA runs one integral at a time, all of its iterations back to back:
-// allocation of evaluations to hypercubes (pyx:1692-1706), the fused tile
-// body of the single-integral kernel over all of the integral's tiles
-// (sampling, map, integrand, two-pass per-hypercube reduction, training
+// allocation of evaluations to hypercubes (pyx:1692-1706), the fused body of
+// the single-integral kernel over all of the integral's samples (sampling, map, integrand, two-pass per-hypercube reduction, training
 // histogram), the merge of hypercubes cut by tile boundaries and the
 // iteration sums (finalize), AdaptiveMap.adapt (pyx:467-594), and at the end
 // the weighted average over the iterations after the warm-up ones
@@ -13,7 +12,7 @@
 // grid-wide synchronisation.
 #pragma once
 #include "vg_adapt.cuh"
-#include "vg_tile.cuh"
+#include "vg_range.cuh"
 
 namespace vgbatch {
 using namespace vg;
@@ -74,13 +73,15 @@ __device__ __forceinline__ bool group_barrier(unsigned int *ctr, unsigned int ta
 }
 
 constexpr int APER = 4;          // hypercubes per thread and pass of the allocation
+constexpr int F64_S = 2;         // samples per thread of the FP64 tiles
 
 // Allocation of one iteration by one CTA: neval_h, offsets, tile heads,
 // totals in the integral's stats (the three allocation kernels' work).
-static __device__ __noinline__ void cta_alloc(const IterArgs &a, int64_t *scan)
+template <int NTB>
+static __device__ __noinline__ void cta_alloc(const IterArgs &a, int64_t *scan /* NTB/32 */)
 {
     const int tid = threadIdx.x;
-    build_tablef(a, tid, NT);   // the FP32 grid table of this iteration
+    build_tablef(a, tid, NTB);   // the FP32 grid table of this iteration
     vg_stats *st = a.stats;
     const double sum_sigf = st->sum_sigf;
     const double nsf = (a.beta > 0 && sum_sigf > 0)
@@ -89,7 +90,7 @@ static __device__ __noinline__ void cta_alloc(const IterArgs &a, int64_t *scan)
     const int64_t mx = a.max_neval_hcube > a.min_neval_hcube ? a.max_neval_hcube : a.min_neval_hcube;
     const int64_t avg = (int64_t)((double)a.neval / (double)a.H);
     int64_t run = 0, mxn = 0;
-    for (int64_t base = 0; base < a.H; base += (int64_t)NT * APER) {
+    for (int64_t base = 0; base < a.H; base += (int64_t)NTB * APER) {
         int64_t loc[APER];
         int64_t s = 0;
 #pragma unroll
@@ -108,16 +109,8 @@ static __device__ __noinline__ void cta_alloc(const IterArgs &a, int64_t *scan)
             loc[k] = n;
             s += n;
         }
-        scan[tid] = s;
-        __syncthreads();
-        for (int off = 1; off < NT; off <<= 1) {
-            const int64_t add = tid >= off ? scan[tid - off] : 0;
-            __syncthreads();
-            scan[tid] += add;
-            __syncthreads();
-        }
-        int64_t off = run + scan[tid] - s;
-        const int64_t total = scan[NT - 1];
+        int64_t total;
+        int64_t off = run + block_excl_scan<NTB>(s, scan, &total);
 #pragma unroll
         for (int k = 0; k < APER; k++) {
             const int64_t h = base + (int64_t)tid * APER + k;
@@ -130,15 +123,8 @@ static __device__ __noinline__ void cta_alloc(const IterArgs &a, int64_t *scan)
             off += n;
         }
         run += total;
-        __syncthreads();
     }
-    // block maximum of the counts
-    scan[tid] = mxn;
-    __syncthreads();
-    for (int o = NT / 2; o > 0; o >>= 1) {
-        if (tid < o) scan[tid] = scan[tid + o] > scan[tid] ? scan[tid + o] : scan[tid];
-        __syncthreads();
-    }
+    mxn = block_max<NTB>(mxn, scan);
     if (tid == 0) {
         const int64_t N = run;
         int64_t ntiles = (N + BASE_TILE - 1) / BASE_TILE;
@@ -146,7 +132,7 @@ static __device__ __noinline__ void cta_alloc(const IterArgs &a, int64_t *scan)
         st->neval = N;
         st->neval_sigf = nsf;
         st->range_lo = a.min_neval_hcube;
-        st->range_hi = a.adaptive_alloc ? (scan[0] > a.min_neval_hcube ? scan[0] : a.min_neval_hcube)
+        st->range_hi = a.adaptive_alloc ? (mxn > a.min_neval_hcube ? mxn : a.min_neval_hcube)
                                         : a.min_neval_hcube;
         if (N > a.ncap || ntiles + 1 > a.ntiles_cap) {
             st->status = VG_ERR_MEMORY;
@@ -162,34 +148,24 @@ static __device__ __noinline__ void cta_alloc(const IterArgs &a, int64_t *scan)
     __syncthreads();
 }
 
-// Iteration sums of one integral by one CTA: the tile body's partial sums
-// (parts[0]) plus the Chan et al. merge of every hypercube cut by tile
-// boundaries (the finalize kernels' work); sum_sigf and the constant-integrand
+// Iteration sums of one integral by one CTA: the partial sums of the group's
+// CTAs plus the Chan et al. merge of every hypercube cut by the ends of the
+// warps' ranges (the finalize kernels' work); sum_sigf and the constant-integrand
 // reset (pyx:2209-2215).
-static __device__ __noinline__ void cta_finalize(const IterArgs &a, int ngroup, VgKSum *red, int *flag)
+template <int NTB>
+static __device__ __noinline__ void cta_finalize(const IterArgs &a, int ngroup, int *flag)
 {
-    // the group CTAs' float-float partials and the cut hypercubes, merged
-    // and summed in float-float, converted to FP64 once (FP32 mode)
     const int tid = threadIdx.x;
     vg_stats *st = a.stats;
-    const int64_t N = st->neval;
-    const int64_t ntiles = st->ntiles ? (N + a.T - 1) / a.T : 0;
-    float r6[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (tid < ngroup && ntiles > 0) {   // the partial sums of each CTA of the group
-        const TilePart p = a.parts[tid];
-        ff_unpack(p.mean.s, r6[0], r6[1]);
-        ff_unpack(p.var.s, r6[2], r6[3]);
-        ff_unpack(p.sigf.s, r6[4], r6[5]);
-    }
-    for (int64_t t = tid; t < ntiles; t += NT) merge_cut_ff(a, t, ntiles, r6[0], r6[1], r6[2], r6[3], r6[4], r6[5]);
-    ff_block_reduce6<NT>(r6, reinterpret_cast<float *>(red));
+    float s6[6];
+    finalize_ranges<NTB>(a, ngroup, (int64_t)ngroup * (NTB / 32 / GROUP), ngroup > 1, s6);
     if (tid == 0) {
-        st->mean = vg_ff_value(r6[0], r6[1]);
-        st->var = vg_ff_value(r6[2], r6[3]);
+        st->mean = vg_ff_value(s6[0], s6[1]);
+        st->var = vg_ff_value(s6[2], s6[3]);
         st->sigf_reset = 0;
         *flag = 0;
         if (a.adaptive) {
-            const double ss = vg_ff_value(r6[4], r6[5]);
+            const double ss = vg_ff_value(s6[4], s6[5]);
             if (ss > 0) {
                 st->sum_sigf = ss;
             } else {
@@ -201,7 +177,7 @@ static __device__ __noinline__ void cta_finalize(const IterArgs &a, int ngroup, 
     }
     __syncthreads();
     if (*flag)
-        for (int64_t h = tid; h < a.H; h += NT) a.sigf[h] = 1.0;
+        for (int64_t h = tid; h < a.H; h += NTB) a.sigf[h] = 1.0;
     __syncthreads();
 }
 
@@ -282,6 +258,7 @@ static __device__ __noinline__ void cta_finalize_f64(const IterArgs &a, int ngro
 
 // End of iteration: adapt the map (one axis after another), copy the new
 // grid back, clear the training histogram (vg_end_iteration's work).
+template <int NTB>
 static __device__ __noinline__ void cta_adapt(const BatchJob &J, const IterArgs &a, unsigned char *smem)
 {
     const int tid = threadIdx.x;
@@ -289,16 +266,16 @@ static __device__ __noinline__ void cta_adapt(const BatchJob &J, const IterArgs 
     double *avg = (double *)smem;
     double *tmp = avg + ad.max_old;
     double *part = tmp + ad.max_old;
-    for (int i = tid; i < ad.max_old; i += NT) avg[i] = 1.0;
+    for (int i = tid; i < ad.max_old; i += NTB) avg[i] = 1.0;
     __syncthreads();
-    for (int d = 0; d < ad.dim; d++) vgadapt::adapt_axis<NT>(ad, d, avg, tmp, part);
+    for (int d = 0; d < ad.dim; d++) vgadapt::adapt_axis<NTB, 256>(ad, d, avg, tmp, part);
     __syncthreads();
     for (int d = 0; d < ad.dim; d++) {
         const int K = ad.old_ninc[d];
         double *g = const_cast<double *>(ad.grid) + d * ad.ldg;
         double *inc = const_cast<double *>(ad.inc) + d * ad.ldi;
-        for (int i = tid; i <= K; i += NT) g[i] = ad.new_grid[d * ad.ldg_new + i];
-        for (int i = tid; i < K; i += NT) {
+        for (int i = tid; i <= K; i += NTB) g[i] = ad.new_grid[d * ad.ldg_new + i];
+        for (int i = tid; i < K; i += NTB) {
             inc[i] = ad.new_inc[d * ad.ldi_new + i];
             a.sum_f[d * a.ldi + i] = 0.0;
             a.n_f[d * a.ldi + i] = 0ull;
@@ -336,18 +313,16 @@ static __device__ __noinline__ void cta_ravg(const BatchJob &J, int nitn, int nw
 
 // The persistent kernel of one dimension bucket (every integral it takes has
 // dim <= DIMB): sampling, map and evaluation in T (float; double in the
-// FP64 parity configuration), S samples per thread and MINB CTAs per SM it is compiled for
-// (the tile shape and occupancy the autotuner picks per bucket; one kernel
-// per bucket lets the small-dimension integrals run at the occupancy their
-// registers and shared memory allow).
+// FP64 parity configuration), NTB threads per CTA and MINB CTAs per SM (the
+// occupancy the autotuner picks per bucket).
 //
 // Queue mode (group <= 1): each CTA takes whole integrals from the queue.
 // Group mode (group = G >= 2, cooperative launch): CTA c works on integral
 // order[c / G] as rank c % G; rank 0 allocates, finalizes and adapts, all G
 // ranks share the tiles (rank r takes tiles r, r + G, ...), with two group
 // barriers per iteration.
-template <typename T, int KIND, int DIMB, int S, int MINB>
-__global__ void __launch_bounds__(NT, MINB) batch_kernel(const BatchJob *__restrict__ jobs,
+template <typename T, int KIND, int DIMB, int NTB, int MINB>
+__global__ void __launch_bounds__(NTB, MINB) batch_kernel(const BatchJob *__restrict__ jobs,
                                                    const VgParams *__restrict__ params,
                                                    const int *__restrict__ order, int njobs, int nitn,
                                                    int nwarm, uint32_t itn0, unsigned int *queue,
@@ -355,8 +330,8 @@ __global__ void __launch_bounds__(NT, MINB) batch_kernel(const BatchJob *__restr
 {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ IterArgs sa;
-    __shared__ int64_t scan[NT];
-    __shared__ VgKSum red[NT / 32 + 4];   // also 6 floats per warp for float-float reductions
+    __shared__ int64_t scan[NTB / 32];
+    __shared__ VgKSum red[NTB / 32];
     __shared__ int s_q, s_flag;
     const int tid = threadIdx.x;
     const int G = group > 1 ? group : 1;
@@ -385,7 +360,7 @@ __global__ void __launch_bounds__(NT, MINB) batch_kernel(const BatchJob *__restr
             const int nw = (int)(sizeof(IterArgs) / 4);
             const uint32_t *src = reinterpret_cast<const uint32_t *>(&J.a);
             uint32_t *dst = reinterpret_cast<uint32_t *>(&sa);
-            for (int i = tid; i < nw; i += NT) dst[i] = src[i];
+            for (int i = tid; i < nw; i += NTB) dst[i] = src[i];
         }
         __syncthreads();
         unsigned int rounds = 0;
@@ -393,20 +368,27 @@ __global__ void __launch_bounds__(NT, MINB) batch_kernel(const BatchJob *__restr
         for (int it = 0; it < nitn && ok; it++) {
             if (tid == 0) sa.itn = itn0 + (uint32_t)it;
             __syncthreads();
-            if (rank == 0) cta_alloc(sa, scan);
+            if (rank == 0) cta_alloc<NTB>(sa, scan);
             if (G > 1 && !(ok = group_barrier(J.sync, (unsigned)G * ++rounds, sa.wait_iters))) break;
-            if (sa.stats->ntiles > 0) tile_body<T, MODE_FUSED, KIND, DIMB, S>(sa, params[j], smem, rank, G, rank);
+            if (sa.stats->ntiles > 0) {
+                if constexpr (sizeof(T) == 8)
+                    tile_body<MODE_FUSED, KIND, DIMB, F64_S, NTB>(sa, params[j], smem, rank, G, rank);
+                else if (G > 1)
+                    range_body<MODE_FUSED, KIND, DIMB, NTB, true>(sa, params[j], smem, rank, G);
+                else
+                    range_body<MODE_FUSED, KIND, DIMB, NTB, false>(sa, params[j], smem, 0, 1);
+            }
             __syncthreads();
             if (G > 1 && !(ok = group_barrier(J.sync, (unsigned)G * ++rounds, sa.wait_iters))) break;
             if (rank == 0) {
                 if constexpr (sizeof(T) == 8) cta_finalize_f64(sa, G, red, &s_flag);
-                else cta_finalize(sa, G, red, &s_flag);
+                else cta_finalize<NTB>(sa, G, &s_flag);
                 if (tid == 0) {
                     J.out[3 * it] = sa.stats->mean;
                     J.out[3 * it + 1] = sa.stats->var;
                     J.out[3 * it + 2] = (double)sa.stats->neval;
                 }
-                if (J.adapt) cta_adapt(J, sa, smem);
+                if (J.adapt) cta_adapt<NTB>(J, sa, smem);
             }
             __syncthreads();
         }
@@ -422,48 +404,48 @@ __global__ void __launch_bounds__(NT, MINB) batch_kernel(const BatchJob *__restr
 
 // Launch (queue mode, or cooperative for co-resident groups) and occupancy
 // of one instantiation; the bucket files dispatch to these.
-template <typename T, int KIND, int DIMB, int S, int MINB>
+template <typename T, int KIND, int DIMB, int NTB, int MINB>
 int launch_one(const BatchJob *jobs, const VgParams *prm, const int *order, int njobs, int nitn, int nwarm,
                uint32_t itn0, unsigned int *queue, size_t smem, int grid, int group, int *status, cudaStream_t st)
 {
-    auto k = batch_kernel<T, KIND, DIMB, S, MINB>;
+    auto k = batch_kernel<T, KIND, DIMB, NTB, MINB>;
     if (group > 1) {
         void *args[] = {(void *)&jobs, (void *)&prm, (void *)&order, (void *)&njobs, (void *)&nitn, (void *)&nwarm,
                         (void *)&itn0, (void *)&queue, (void *)&group, (void *)&status};
-        VG_CUDA_CHECK(cudaLaunchCooperativeKernel((const void *)k, dim3((unsigned)grid), dim3(NT), args, smem, st));
+        VG_CUDA_CHECK(cudaLaunchCooperativeKernel((const void *)k, dim3((unsigned)grid), dim3(NTB), args, smem, st));
         return VG_OK;
     }
-    k<<<grid, NT, smem, st>>>(jobs, prm, order, njobs, nitn, nwarm, itn0, queue, group, status);
+    k<<<grid, NTB, smem, st>>>(jobs, prm, order, njobs, nitn, nwarm, itn0, queue, group, status);
     VG_LAUNCH_CHECK();
     return VG_OK;
 }
 
 // sets the kernel's shared-memory attribute (outside any stream capture)
-template <typename T, int KIND, int DIMB, int S, int MINB>
+template <typename T, int KIND, int DIMB, int NTB, int MINB>
 int occupancy_one(size_t smem, int *per_sm)
 {
-    auto k = batch_kernel<T, KIND, DIMB, S, MINB>;
+    auto k = batch_kernel<T, KIND, DIMB, NTB, MINB>;
     VG_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    VG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k, NT, smem));
+    VG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k, NTB, smem));
     return VG_OK;
 }
 
-// Tile configurations of each bucket: samples per thread and CTAs per SM.
+// Configurations of each bucket: threads per CTA and CTAs per SM.
 struct BucketConfig {
-    int S, minb;
+    int ntb, minb;
 };
 constexpr int NCONFIG = 3;
 constexpr int NBUCKET = 3;
 constexpr int BUCKET_DIM[NBUCKET] = {4, 8, 16};
 // FP64 parity configuration (cfg VG_BATCH_CFG_F64): Lorentzian products of
-// dim <= 8 (buckets 0 and 1 share the one instantiation), 2 samples per
-// thread, one CTA per SM -- the single-integral FP64 kernel's tile shape.
-constexpr BucketConfig F64_CONFIG = {2, 1};
+// dim <= 8 (buckets 0 and 1 share the one instantiation), the large tiles of
+// the single-integral FP64 kernel, one CTA per SM.
+constexpr BucketConfig F64_CONFIG = {NT, 1};
 constexpr int F64_DIMB = 8;
 constexpr BucketConfig BUCKET_CONFIGS[NBUCKET][NCONFIG] = {
-    {{2, 4}, {4, 2}, {2, 2}},   // dim <= 4
-    {{2, 2}, {4, 1}, {2, 3}},   // dim <= 8
-    {{2, 1}, {1, 2}, {2, 2}},   // dim <= 16
+    {{1024, 1}, {512, 2}, {256, 4}},   // dim <= 4
+    {{512, 2}, {1024, 1}, {768, 1}},   // dim <= 8
+    {{768, 1}, {512, 1}, {1024, 1}},   // dim <= 16
 };
 
 // One bucket's launch and occupancy for configuration cfg (instantiated by
@@ -477,13 +459,13 @@ int bucket_launch(int cfg, const BatchJob *jobs, const VgParams *prm, const int 
     constexpr BucketConfig c0 = BUCKET_CONFIGS[b][0], c1 = BUCKET_CONFIGS[b][1], c2 = BUCKET_CONFIGS[b][2];
     switch (cfg) {
     case 0:
-        return launch_one<float, KIND, DIMB, c0.S, c0.minb>(jobs, prm, order, njobs, nitn, nwarm, itn0, queue, smem, grid,
+        return launch_one<float, KIND, DIMB, c0.ntb, c0.minb>(jobs, prm, order, njobs, nitn, nwarm, itn0, queue, smem, grid,
                                                      group, status, st);
     case 1:
-        return launch_one<float, KIND, DIMB, c1.S, c1.minb>(jobs, prm, order, njobs, nitn, nwarm, itn0, queue, smem, grid,
+        return launch_one<float, KIND, DIMB, c1.ntb, c1.minb>(jobs, prm, order, njobs, nitn, nwarm, itn0, queue, smem, grid,
                                                      group, status, st);
     default:
-        return launch_one<float, KIND, DIMB, c2.S, c2.minb>(jobs, prm, order, njobs, nitn, nwarm, itn0, queue, smem, grid,
+        return launch_one<float, KIND, DIMB, c2.ntb, c2.minb>(jobs, prm, order, njobs, nitn, nwarm, itn0, queue, smem, grid,
                                                      group, status, st);
     }
 }
@@ -494,9 +476,9 @@ int bucket_occupancy(int cfg, size_t smem, int *per_sm)
     constexpr int b = DIMB == 4 ? 0 : (DIMB == 8 ? 1 : 2);
     constexpr BucketConfig c0 = BUCKET_CONFIGS[b][0], c1 = BUCKET_CONFIGS[b][1], c2 = BUCKET_CONFIGS[b][2];
     switch (cfg) {
-    case 0: return occupancy_one<float, KIND, DIMB, c0.S, c0.minb>(smem, per_sm);
-    case 1: return occupancy_one<float, KIND, DIMB, c1.S, c1.minb>(smem, per_sm);
-    default: return occupancy_one<float, KIND, DIMB, c2.S, c2.minb>(smem, per_sm);
+    case 0: return occupancy_one<float, KIND, DIMB, c0.ntb, c0.minb>(smem, per_sm);
+    case 1: return occupancy_one<float, KIND, DIMB, c1.ntb, c1.minb>(smem, per_sm);
+    default: return occupancy_one<float, KIND, DIMB, c2.ntb, c2.minb>(smem, per_sm);
     }
 }
 

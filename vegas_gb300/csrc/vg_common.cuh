@@ -34,14 +34,14 @@ __device__ __forceinline__ VgU4 vg_philox(uint32_t c0, uint32_t c1, uint32_t c2,
 {
 #pragma unroll
     for (int r = 0; r < 10; r++) {
-        uint32_t hi0 = __umulhi(0xD2511F53u, c0), lo0 = 0xD2511F53u * c0;
-        uint32_t hi1 = __umulhi(0xCD9E8D57u, c2), lo1 = 0xCD9E8D57u * c2;
-        uint32_t n0 = hi1 ^ c1 ^ k0;
-        uint32_t n2 = hi0 ^ c3 ^ k1;
+        const uint64_t p0 = (uint64_t)0xD2511F53u * c0;   // one wide multiply for both halves
+        const uint64_t p1 = (uint64_t)0xCD9E8D57u * c2;
+        const uint32_t n0 = (uint32_t)(p1 >> 32) ^ c1 ^ k0;
+        const uint32_t n2 = (uint32_t)(p0 >> 32) ^ c3 ^ k1;
         c0 = n0;
-        c1 = lo1;
+        c1 = (uint32_t)p1;
         c2 = n2;
-        c3 = lo0;
+        c3 = (uint32_t)p0;
         k0 += 0x9E3779B9u;
         k1 += 0xBB67AE85u;
     }
@@ -79,6 +79,18 @@ struct VgUniform<double> {
 
 template <>
 struct VgUniform<float> {
+    // the uniforms of axes 4g .. 4g+3
+    static __device__ __forceinline__ void group(uint64_t seed, uint32_t stream, uint32_t itn, uint64_t i, int g,
+                                                 float (&u)[4])
+    {
+        const float s = 1.0f / 16777216.0f;
+        const VgU4 r = vg_philox((uint32_t)i, (uint32_t)(i >> 32), itn, (stream << 8) | (uint32_t)g, (uint32_t)seed,
+                                 (uint32_t)(seed >> 32));
+        u[0] = (float)(r.x >> 8) * s;
+        u[1] = (float)(r.y >> 8) * s;
+        u[2] = (float)(r.z >> 8) * s;
+        u[3] = (float)(r.w >> 8) * s;
+    }
     template <int DIMB>
     static __device__ __forceinline__ void draw(uint64_t seed, uint32_t stream, uint32_t itn,
                                                 uint64_t i, int dim, float *u)

@@ -186,7 +186,8 @@ __device__ __forceinline__ float vg_ex2(float x)
 
 template <int KIND, int DIMB>
 __device__ __forceinline__ float vg_eval_f32(const VgF32Consts &k, const float *__restrict__ tab,
-                                             int nterm, int dim, const float *x)
+                                             int nterm, int dim, const float *x,
+                                             unsigned long long *term_count = nullptr)
 {
     if (KIND == VG_F_GAUSS) {
         float s = 0.f;
@@ -234,6 +235,7 @@ __device__ __forceinline__ float vg_eval_f32(const VgF32Consts &k, const float *
                 if (j > jend) j = jend;
             }
         }
+        if (term_count != nullptr) atomicAdd(term_count, (unsigned long long)(jend - j));   // instrumentation
         for (; j + 4 <= jend; j += 4) {
             float4 v = *reinterpret_cast<const float4 *>(tab + j);
             float d0 = w - v.x, d1 = w - v.y, d2 = w - v.z, d3 = w - v.w;

@@ -29,61 +29,12 @@
 #include <mutex>
 
 #include "vg_adapt.cuh"
-#include "vg_tile.cuh"
+#include "vg_range.cuh"
 
 namespace {
 using namespace vg;
 
 // ======================================================== allocation
-// Block-wide exclusive prefix sum of one int64 per thread (warp shuffles,
-// then a scan of the warp totals); *total = the block's sum.
-template <int NTB>
-__device__ __forceinline__ int64_t block_excl_scan(int64_t v, int64_t *wtot /* NTB/32 */, int64_t *total)
-{
-    constexpr int NW = NTB / 32;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int64_t x = v;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const int64_t y = __shfl_up_sync(0xffffffffu, x, off);
-        if (lane >= off) x += y;
-    }
-    if (lane == 31) wtot[w] = x;
-    __syncthreads();
-    if (w == 0) {
-        int64_t z = lane < NW ? wtot[lane] : 0;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const int64_t y = __shfl_up_sync(0xffffffffu, z, off);
-            if (lane >= off) z += y;
-        }
-        if (lane < NW) wtot[lane] = z;
-    }
-    __syncthreads();
-    *total = wtot[NW - 1];
-    const int64_t r = (w > 0 ? wtot[w - 1] : 0) + x - v;
-    __syncthreads();
-    return r;
-}
-
-template <int NTB>
-__device__ __forceinline__ int64_t block_max(int64_t v, int64_t *wtot /* NTB/32 */)
-{
-    constexpr int NW = NTB / 32;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const int64_t o = __shfl_xor_sync(0xffffffffu, v, off);
-        v = o > v ? o : v;
-    }
-    if (lane == 0) wtot[w] = v;
-    __syncthreads();
-    int64_t m = wtot[0];
-    for (int i = 1; i < NW; i++) m = wtot[i] > m ? wtot[i] : m;
-    __syncthreads();
-    return m;
-}
-
 // Allocation, pyx:1692-1706, in one pass over the hypercubes: block b
 // (numbered by the order in which blocks start, so it only waits on blocks
 // already running) counts neval_h for its ALLOC_NT * ALLOC_PER hypercubes,
@@ -278,6 +229,7 @@ __global__ void tablef_kernel(IterArgs a)
 }
 
 // ========================================================== finalize
+// FP64 mode.
 // Stage 1 (one thread per tile, FIN_TILES tiles per block): the tile's
 // partial sums plus, for a tile whose last hypercube continues into later
 // tiles, the Chan et al. merge of that hypercube's partial records; a
@@ -347,29 +299,19 @@ __device__ __forceinline__ void finalize_store(const IterArgs &a, double mean, d
         for (int64_t h = threadIdx.x; h < a.H; h += blockDim.x) a.sigf[h] = 1.0;
 }
 
-// FP32 mode, stage 2: the blocks' float-float partials summed in float-float
-// in block order (lane-strided, then a fixed tree), converted to FP64 once.
-__device__ __forceinline__ void finalize_totals_ff(const IterArgs &a, int64_t nblk, int *reset)
+// FP32 mode: one CTA.
+constexpr int FIN32_NT = 256;
+__global__ void __launch_bounds__(FIN32_NT) finalize32_kernel(const __grid_constant__ IterArgs a)
 {
-    float r6[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int64_t b = threadIdx.x; b < nblk; b += FIN_TILES) {
-        const TilePart p = a.part2[b];
-        float h, l;
-        ff_unpack(p.mean.s, h, l);
-        ff_add_pair(r6[0], r6[1], h, l);
-        ff_unpack(p.var.s, h, l);
-        ff_add_pair(r6[2], r6[3], h, l);
-        ff_unpack(p.sigf.s, h, l);
-        ff_add_pair(r6[4], r6[5], h, l);
-    }
-    ff_block_reduce6<FIN_TILES>(r6, nullptr);
-    finalize_store(a, vg_ff_value(r6[0], r6[1]), vg_ff_value(r6[2], r6[3]), vg_ff_value(r6[4], r6[5]), reset);
+    __shared__ int s_reset;
+    float s6[6];
+    finalize_ranges<FIN32_NT>(a, a.ncta, a.ngroups, false, s6);
+    finalize_store(a, vg_ff_value(s6[0], s6[1]), vg_ff_value(s6[2], s6[3]), vg_ff_value(s6[4], s6[5]), &s_reset);
 }
 
 // Stage 1, and stage 2 in the block that finishes last (a counter the
 // allocation resets; the partials are read back in block order, so the
 // result does not depend on which block that is).
-template <int FAST>
 __global__ void __launch_bounds__(FIN_TILES) finalize1_kernel(IterArgs a)
 {
     __shared__ VgKSum red[1];
@@ -379,28 +321,7 @@ __global__ void __launch_bounds__(FIN_TILES) finalize1_kernel(IterArgs a)
     const int64_t ntiles = st->ntiles ? (N + a.T - 1) / a.T : 0;
     const int64_t nwork = ntiles > a.ncta ? ntiles : a.ncta;
     const int64_t nblk = (nwork + FIN_TILES - 1) / FIN_TILES;
-    if (FAST && (int64_t)blockIdx.x < nblk) {
-        // FP32 mode: the tile partials and the cut hypercubes' records hold
-        // packed float-float values; merged and summed in float-float
-        // (FP32 pipe, no FP64 instruction on the path)
-        float r6[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        const int64_t t = (int64_t)blockIdx.x * FIN_TILES + threadIdx.x;
-        if (t < a.ncta && ntiles > 0) {   // partial sums of the reduction CTA t
-            const TilePart p = a.parts[t];
-            ff_unpack(p.mean.s, r6[0], r6[1]);
-            ff_unpack(p.var.s, r6[2], r6[3]);
-            ff_unpack(p.sigf.s, r6[4], r6[5]);
-        }
-        if (t < ntiles) merge_cut_ff(a, t, ntiles, r6[0], r6[1], r6[2], r6[3], r6[4], r6[5]);
-        ff_block_reduce6<FIN_TILES>(r6, nullptr);
-        if (threadIdx.x == 0) {
-            TilePart p;
-            p.mean = VgKSum{ff_pack(r6[0], r6[1]), 0.0};
-            p.var = VgKSum{ff_pack(r6[2], r6[3]), 0.0};
-            p.sigf = VgKSum{ff_pack(r6[4], r6[5]), 0.0};
-            a.part2[blockIdx.x] = p;
-        }
-    } else if ((int64_t)blockIdx.x < nblk) {
+    if ((int64_t)blockIdx.x < nblk) {
         const double beta_half = a.beta_half;
         VgKSum cm = {0.0, 0.0}, cv = {0.0, 0.0}, cs = {0.0, 0.0};
         const int64_t t = (int64_t)blockIdx.x * FIN_TILES + threadIdx.x;
@@ -418,18 +339,15 @@ __global__ void __launch_bounds__(FIN_TILES) finalize1_kernel(IterArgs a)
                     const TileRec q = a.recs[2 * t2];
                     if (q.h != r.h) break;
                     const double n2 = n + q.n;
-                    // Chan et al. merge; FP32 mode: reciprocal-multiply divisions
-                    const double delta = FAST ? vgadapt::div_fast(q.S, q.n) - vgadapt::div_fast(Sx, n)
-                                              : q.S / q.n - Sx / n;
-                    Q = Q + q.Q + delta * delta * (FAST ? vgadapt::div_fast(n * q.n, n2) : n * q.n / n2);
+                    const double delta = q.S / q.n - Sx / n;   // Chan et al. merge
+                    Q = Q + q.Q + delta * delta * (n * q.n / n2);
                     Sx += q.S;
                     D += q.D;
                     n = n2;
                     if (!q.spans) break;
                 }
                 const double num = __dsub_rn(__dmul_rn(n, Q), __dmul_rn(D, D));
-                const double vh = FAST ? vgadapt::div_fast(num, __dsub_rn(n, 1.))
-                                       : __ddiv_rn(num, __dsub_rn(n, 1.));
+                const double vh = __ddiv_rn(num, __dsub_rn(n, 1.));
                 if (a.train_hc) {   // adapt_to_errors: train at the hypercube's last sample
                     unsigned short b[VG_MAX_DIM];
                     last_sample_bins<double>(a, r.h, b);
@@ -438,7 +356,7 @@ __global__ void __launch_bounds__(FIN_TILES) finalize1_kernel(IterArgs a)
                 cm.add(__dadd_rn(Sx, D));
                 cv.add(vh);
                 if (a.adaptive) {
-                    const double sg = FAST ? vg_pow_fast(fabs(vh), beta_half) : pow(fabs(vh), beta_half);
+                    const double sg = pow(fabs(vh), beta_half);
                     a.sigf[r.h] = sg;
                     cs.add(sg);
                 }
@@ -463,15 +381,14 @@ __global__ void __launch_bounds__(FIN_TILES) finalize1_kernel(IterArgs a)
     if (!s_last) return;
     __threadfence();
     if (threadIdx.x == 0) *a.fin_counter = 0u;
-    if (FAST) finalize_totals_ff(a, nblk, &s_reset);
-    else finalize_totals(a, nblk, red, &s_reset);
+    finalize_totals(a, nblk, red, &s_reset);
 }
 
 // ================================================================ host
 struct WorkLayout {
     size_t neval_h, offsets, bsum, tile_h0, counter, recs, parts, part2, feval, newgrid,
         newinc, tablef, total;
-    int64_t nblk, ntiles_cap, ncap;
+    int64_t nblk, ntiles_cap, ncap, rec_cap, part_cap;
 };
 
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -498,9 +415,17 @@ WorkLayout layout(const vg_integrator *it, int64_t ncap)
     L.bsum = o;    o = align256(o + sizeof(int64_t) * L.nblk);
     L.tile_h0 = o; o = align256(o + sizeof(int64_t) * (L.ntiles_cap + 1));
     L.counter = o; o = align256(o + 16 + sizeof(AllocSync));
-    L.recs = o;    o = align256(o + sizeof(TileRec) * 2 * L.ntiles_cap);
-    L.parts = o;   o = align256(o + sizeof(TilePart) * L.ntiles_cap);
-    L.part2 = o;   o = align256(o + sizeof(TilePart) * (L.ntiles_cap / FIN_TILES + 4096 / FIN_TILES + 2));
+    // FP64: two records per tile of 256 or more samples; FP32: per CTA or dealt unit
+    const int f64 = it->precision == VG_F64;
+    const int64_t tiles = (ncap + 255) / 256 + 1;
+    L.part_cap = L.ntiles_cap < MAX_PARTS ? L.ntiles_cap : (int64_t)MAX_PARTS;
+    if (L.part_cap < 1024) L.part_cap = 1024;   // the batched launch's groups of CTAs, whatever the integral's size
+    const int64_t units = L.ntiles_cap / DEAL_CHUNKS + 2;
+    L.rec_cap = f64 ? tiles : (units > L.part_cap ? units : L.part_cap);
+    const int64_t fin = L.rec_cap > L.part_cap ? L.rec_cap : L.part_cap;
+    L.recs = o;    o = align256(o + (f64 ? sizeof(TileRec) : sizeof(RangeRec)) * 2 * L.rec_cap);
+    L.parts = o;   o = align256(o + sizeof(TilePart) * L.part_cap);
+    L.part2 = o;   o = align256(o + sizeof(TilePart) * (fin / FIN_TILES + 2));
     L.feval = o;   o = align256(o + sizeof(float) * ncap);
     L.ncap = ncap;
     L.newgrid = o; o = align256(o + sizeof(double) * it->dim * it->ldg);
@@ -524,6 +449,16 @@ int fill_args(IterArgs &a, const vg_integrator *it, uint32_t itn, const double *
             return vg_fail(VG_ERR_VALUE, "bad geometry (ninc must be in 1..65534)");
         a.nstrat[d] = (int)it->nstrat[d];
         a.ninc[d] = (int)it->ninc[d];
+        AxisArgs &x = a.ax[d];
+        x.nstrat = a.nstrat[d];
+        x.ninc = a.ninc[d];
+        x.Kf = (float)a.ninc[d];
+        x.rstrat = 1.f / (float)a.nstrat[d];
+        int sh = 0;   // 2^sh >= nstrat: h * (dmul * nstrat - 2^(31+sh)) < 2^(31+sh) for h < 2^31
+        while (((int64_t)1 << sh) < a.nstrat[d]) sh++;
+        x.dshift = sh;
+        x.dmul = (unsigned int)((((uint64_t)1 << (31 + sh)) + (uint64_t)a.nstrat[d] - 1) / (uint64_t)a.nstrat[d]);
+        a.wide |= a.nstrat[d] >= (1 << 24);
         maxK = a.ninc[d] > maxK ? a.ninc[d] : maxK;
         if (it->ninc[d] + 1 > it->ldg || it->ninc[d] > it->ldi)
             return vg_fail(VG_ERR_VALUE, "grid arrays too small");
@@ -534,6 +469,7 @@ int fill_args(IterArgs &a, const vg_integrator *it, uint32_t itn, const double *
     a.ldg = it->ldg;
     a.ldi = it->ldi;
     a.H = it->nhcube;
+    a.wide |= it->nhcube > 0x7fffffff;
     a.ncap = neval_cap(it);
     WorkLayout L = layout(it, a.ncap);
     if (it->work_bytes < L.total)
@@ -559,6 +495,7 @@ int fill_args(IterArgs &a, const vg_integrator *it, uint32_t itn, const double *
     a.fin_counter = (unsigned int *)(w + L.counter + sizeof(unsigned long long));
     a.alloc_sync = (unsigned int *)(w + L.counter + 16);
     a.recs = (TileRec *)(w + L.recs);
+    a.rrecs = (RangeRec *)(w + L.recs);
     a.parts = (TilePart *)(w + L.parts);
     a.part2 = (TilePart *)(w + L.part2);
     a.f_eval = (float *)(w + L.feval);
@@ -583,12 +520,15 @@ int fill_args(IterArgs &a, const vg_integrator *it, uint32_t itn, const double *
 namespace vg {
 int finalize_launch(IterArgs &a, cudaStream_t st, int fast)
 {
-    // tiles of the launched kernel, bounded by the capacity
-    const int64_t tcap = (a.ntiles_cap * BASE_TILE + a.T - 1) / a.T;
-    const int64_t nwork = tcap > a.ncta ? tcap : a.ncta;
-    const int64_t nblk = (nwork + FIN_TILES - 1) / FIN_TILES;
-    if (fast) finalize1_kernel<1><<<(unsigned)nblk, FIN_TILES, 0, st>>>(a);
-    else finalize1_kernel<0><<<(unsigned)nblk, FIN_TILES, 0, st>>>(a);
+    if (fast) {
+        finalize32_kernel<<<1, FIN32_NT, 0, st>>>(a);
+    } else {
+        // tiles of the launched kernel, bounded by the capacity
+        const int64_t tcap = (a.ncap + a.T - 1) / a.T;
+        const int64_t nwork = tcap > a.ncta ? tcap : a.ncta;
+        const int64_t nblk = (nwork + FIN_TILES - 1) / FIN_TILES;
+        finalize1_kernel<<<(unsigned)nblk, FIN_TILES, 0, st>>>(a);
+    }
     VG_LAUNCH_CHECK();
     return VG_OK;
 }
@@ -682,8 +622,9 @@ extern "C" int vg_sample(const vg_integrator *it, uint32_t itn, const double *u,
     a.train = 0;
     a.train_hc = 0;
     a.adaptive = 0;
+    a.x_vec = (a.dim % 4 == 0) && ((uintptr_t)x & 15) == 0;
     cudaStream_t st = (cudaStream_t)stream;
-    if ((rc = reset_counter(a, st))) return rc;
+    if (it->precision == VG_F64 && (rc = reset_counter(a, st))) return rc;   // FP64 tiles are taken from a counter
     return vg::launch_points(a, it->precision == VG_F64, st);
 }
 
@@ -775,8 +716,9 @@ extern "C" int vg_sample_keep(const vg_integrator *it, uint32_t itn, const doubl
     a.train = 0;
     a.train_hc = 0;
     a.adaptive = 0;
+    a.x_vec = (a.dim % 4 == 0) && ((uintptr_t)x & 15) == 0;
     cudaStream_t st = (cudaStream_t)stream;
-    if ((rc = reset_counter(a, st))) return rc;
+    if (it->precision == VG_F64 && (rc = reset_counter(a, st))) return rc;   // FP64 tiles are taken from a counter
     return vg::launch_points(a, it->precision == VG_F64, st);
 }
 
@@ -801,19 +743,17 @@ static unsigned long long *g_term_count = nullptr;
 namespace vg {
 uint32_t g_wait_iters = VG_WAIT_ITERS_DEFAULT;
 int g_eval_split = 0;
-int g_tile_s4 = 0, g_tile_table = -1, g_tile_hist = -1;
+int g_tile_table = -1, g_tile_hist = -1;
 }
 
-// Tuning of the tile kernels: samples per thread of the fused FP32 ridge for
-// dim <= 4 (0 automatic = 2, with 4 CTAs per SM; or 4), grid table and
-// training histogram in shared memory (-1 automatic, 0 off, 1 on where it
-// fits).
+// Tuning of the iteration kernels: grid table and training histogram in
+// shared memory (-1 automatic, 0 off, 1 on where it fits).  s_dim4, samples
+// per thread of an earlier FP32 kernel, is checked and has no effect.
 extern "C" int vg_set_tile_tuning(int s_dim4, int table_smem, int hist_smem)
 {
     if (s_dim4 != 0 && s_dim4 != 2 && s_dim4 != 4) return vg_fail(VG_ERR_VALUE, "s_dim4 %d", s_dim4);
     if (table_smem < -1 || table_smem > 1 || hist_smem < -1 || hist_smem > 1)
         return vg_fail(VG_ERR_VALUE, "shared-memory policy");
-    vg::g_tile_s4 = s_dim4;
     vg::g_tile_table = table_smem;
     vg::g_tile_hist = hist_smem;
     return VG_OK;
