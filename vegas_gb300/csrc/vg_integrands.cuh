@@ -214,17 +214,23 @@ __device__ __forceinline__ float vg_eval_f32(const VgF32Consts &k, const float *
         const float E0 = -k.c[0] * R;
         const float w = m * k.c[1];
         float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-        // terms with E0 - (w - v_j)^2 < -127 are exactly zero (ex2.approx.ftz
-        // flushes them): evaluate the window of the others only, aligned to
-        // the 4-way accumulator pattern -- the sum is bit-identical
+        // Terms that can count, aligned to the 4-way accumulator pattern: a
+        // term below 2^-30 of the largest one (the nearest centre's) leaves the
+        // FP32 sum as it is (all of those together are below 2^-29 of it, its own
+        // rounding is 2^-24), one with E0 - (w - v_j)^2 < -127 is exactly zero
+        // (ex2.approx.ftz flushes it).  The first bound makes the window as wide
+        // for every sample of a warp: 68 terms of M = 1000, s = 0.01 at dim 4 where
+        // the second alone left 96 on average and 132 for the warp's widest.
         int j = 0, jend = nterm & ~3;
         {
             const float rad2 = E0 + 127.f;
             if (rad2 <= 0.f) {
                 jend = 0;
             } else {
-                const float delta = sqrtf(rad2) * 1.0001f + 1e-3f;
                 const float rc = 1.f / k.c[4];
+                const float jw = fmaf(w, rc, -0.5f);
+                const float dn = fmaf(-(rintf(fminf(fmaxf(jw, 0.f), (float)(nterm - 1))) + 0.5f), k.c[4], w);
+                const float delta = sqrtf(fminf(rad2, fmaf(dn, dn, 30.f))) * 1.0001f + 1e-3f;
                 int jlo = (int)floorf((w - delta) * rc - 0.5f) - 1;
                 int jhi = (int)ceilf((w + delta) * rc - 0.5f) + 1;
                 jlo = jlo < 0 ? 0 : jlo;
