@@ -511,11 +511,12 @@ class Integrator(object):
         corr = 1 if self.correlate_integrals else 0
         need = int(L.vg_reduce_array_work_bytes(s, corr))
         work = torch.empty(need, dtype=torch.uint8, device=self.device)
-        mean = torch.empty(s, dtype=torch.float64, device=self.device)
-        var = torch.empty((s, s), dtype=torch.float64, device=self.device)
+        out = torch.empty(s + s * s, dtype=torch.float64, device=self.device)
+        mean, var = out[:s], out[s:]
         N.check(L.vg_reduce_array(ctypes.byref(it), N.ptr(f), fdt, s, corr, N.ptr(w), N.ptr(mean),
                                   N.ptr(var), N.ptr(work), need, N.stream_ptr(self.device)))
-        return mean.cpu().numpy(), var.cpu().numpy()
+        host = out.cpu().numpy()   # one copy and one wait for both
+        return host[:s], host[s:].reshape(s, s)
 
     def __call__(self, fcn, save=None, saveall=None, **kargs):
         """Integrate ``fcn``; returns an :class:`RAvg` (pyx:1912-2230)."""
