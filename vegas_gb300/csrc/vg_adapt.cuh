@@ -1,8 +1,8 @@
 // vg_adapt.cuh -- AdaptiveMap.adapt for one axis as a block-level device
 // function (src/vegas/_vegas.pyx:467-594: average of the training data,
 // 3-tap smoothing, normalisation, damping ((1-f)/-ln f)^alpha, regrid).
-// Templated on the block size: the adapt kernel runs it with 1024 threads
-// per axis, the batched kernel with the 256 threads of its CTA.
+// The adapt kernel runs it with 1024 threads per axis, the batched kernel with
+// the threads of its CTA.
 #pragma once
 #include "vg_common.cuh"
 
@@ -49,12 +49,11 @@ __device__ __forceinline__ double div_fast(double a, double b)
 // per-thread sequential over a contiguous chunk, then a scan of the chunk
 // totals by warp shuffles (within each warp, then over the warp totals) --
 // few FP64 instructions per thread (GB300 issues FP64 at a low rate).
-template <int ADAPT_NT>
-__device__ void block_inclusive_scan(double *v, int n, double *part /* >= 32 */)
+static __device__ void block_inclusive_scan(double *v, int n, double *part /* >= 32 */)
 {
-    constexpr int NW = ADAPT_NT / 32;
+    const int NT = (int)blockDim.x, NW = NT >> 5;
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    const int per = (n + ADAPT_NT - 1) / ADAPT_NT;
+    const int per = (n + NT - 1) / NT;
     const int b = t * per, e = min(n, b + per);
     double s = 0.0;
     for (int i = b; i < e; i++) {
@@ -89,13 +88,12 @@ __device__ void block_inclusive_scan(double *v, int n, double *part /* >= 32 */)
 }
 
 // Sum of v[0..n) in a fixed order; result broadcast to all threads.
-template <int ADAPT_NT>
-__device__ double block_sum(const double *v, int n, double *part /* >= 33 */)
+static __device__ double block_sum(const double *v, int n, double *part /* >= 33 */)
 {
-    constexpr int NW = ADAPT_NT / 32;
+    const int NT = (int)blockDim.x, NW = NT >> 5;
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     double s = 0.0;
-    for (int i = t; i < n; i += ADAPT_NT) s = __dadd_rn(s, v[i]);
+    for (int i = t; i < n; i += NT) s = __dadd_rn(s, v[i]);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, off));
     if (lane == 0) part[w] = s;
@@ -112,12 +110,12 @@ __device__ double block_sum(const double *v, int n, double *part /* >= 33 */)
     return r;
 }
 
-// FP32 block reductions (max, sum) over the first RED_NT threads; f = shared
+// FP32 block reductions (max, sum) over the first red_nt threads; f = shared
 // scratch of >= 33 floats.  Result broadcast to all threads.
-template <int RED_NT, bool MAX>
-__device__ float block_reduce_f(float v, float *f)
+template <bool MAX>
+__device__ float block_reduce_f(float v, float *f, int red_nt)
 {
-    constexpr int NW = RED_NT / 32;
+    const int NW = red_nt >> 5;
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
@@ -148,14 +146,14 @@ __device__ float block_reduce_f(float v, float *f)
 // (or within 1e-5 of 1) is formed and damped in FP64, so tiny weights keep
 // the reference's ((1 - v) / -ln v)^alpha.  The cumulative sums and the new
 // nodes (regrid) stay FP64.
-template <int ADAPT_NT, int SUM_NT>
+template <int SUM_NT>
 __device__ void adapt_weights_fast(const AdaptArgs &a, int d, int K, double *avg, double *tmp, double *part)
 {
-    const int t = threadIdx.x;
+    const int t = threadIdx.x, NT = (int)blockDim.x;
     float *af = reinterpret_cast<float *>(tmp);   // [K] averages
     float *sf = af + K;                           // [K] smoothed (tmp holds 2K floats)
     float *pf = reinterpret_cast<float *>(part);
-    for (int i = t; i < K; i += ADAPT_NT) {
+    for (int i = t; i < K; i += NT) {
         const unsigned long long c = a.n_f[d * a.ldi + i];
         af[i] = c ? (float)div_fast(a.sum_f[d * a.ldi + i], (double)c) : 0.f;
         if (a.zero_hist) {
@@ -165,7 +163,7 @@ __device__ void adapt_weights_fast(const AdaptArgs &a, int d, int K, double *avg
     }
     __syncthreads();
     float mx = 0.f;
-    for (int i = t; i < K; i += ADAPT_NT) {
+    for (int i = t; i < K; i += NT) {
         float v;
         if (i == 0) v = fmaf(7.f, af[0], af[1]);
         else if (i == K - 1) v = fmaf(7.f, af[K - 1], af[K - 2]);
@@ -174,15 +172,16 @@ __device__ void adapt_weights_fast(const AdaptArgs &a, int d, int K, double *avg
         sf[i] = v;
         mx = fmaxf(mx, v);
     }
-    mx = block_reduce_f<ADAPT_NT, true>(mx, pf);
+    mx = block_reduce_f<true>(mx, pf, NT);
     const float rmx = mx > 0.f ? 1.f / mx : 0.f;   // sum of values scaled by the max: no overflow
     float sp = 0.f;
-    if (t < SUM_NT)
-        for (int i = t; i < K; i += SUM_NT) sp += sf[i] * rmx;
-    sp = block_reduce_f<SUM_NT, false>(sp, pf);
+    const int sum_nt = SUM_NT > 0 ? SUM_NT : NT;
+    if (t < sum_nt)
+        for (int i = t; i < K; i += sum_nt) sp += sf[i] * rmx;
+    sp = block_reduce_f<false>(sp, pf, sum_nt);
     const float rs = sp > 0.f ? 1.f / sp : 0.f;
     const float alf = (float)a.alpha;
-    for (int i = t; i < K; i += ADAPT_NT) {
+    for (int i = t; i < K; i += NT) {
         const float vf = sf[i] * rmx * rs;
         double v;
         if (sp > 0.f && vf >= 1.17549435e-38f && vf < 0.99999f) {
@@ -204,19 +203,19 @@ __device__ void adapt_weights_fast(const AdaptArgs &a, int d, int K, double *avg
 // memory, max_old + 1 and max_old doubles) the axis' old nodes and
 // increments are staged there first, so new_grid / new_inc may be the grid
 // itself (adapt in place).
-template <int ADAPT_NT, int SUM_NT = ADAPT_NT>
+template <int SUM_NT = 0>
 __device__ void adapt_axis(const AdaptArgs &a, int d, double *avg, double *tmp, double *part,
                            double *gs = nullptr, double *is = nullptr)
 {
     const int K = a.old_ninc[d];
     const int Kn = a.new_ninc[d];
-    const int t = threadIdx.x;
+    const int t = threadIdx.x, NT = (int)blockDim.x;
     const double alpha = a.alpha;
     if (alpha > 0 && K > 1 && a.fast && a.sum_f != nullptr) {
-        adapt_weights_fast<ADAPT_NT, SUM_NT>(a, d, K, avg, tmp, part);
+        adapt_weights_fast<SUM_NT>(a, d, K, avg, tmp, part);
     } else if (alpha != 0 && K > 1) {
         if (a.sum_f != nullptr) {
-            for (int i = t; i < K; i += ADAPT_NT) {
+            for (int i = t; i < K; i += NT) {
                 const unsigned long long c = a.n_f[d * a.ldi + i];
                 if (a.fast) {
                     avg[i] = c ? div_fast(a.sum_f[d * a.ldi + i], (double)c) : 0.0;
@@ -233,7 +232,7 @@ __device__ void adapt_axis(const AdaptArgs &a, int d, double *avg, double *tmp, 
         }
         if (alpha > 0) {
             // smoothing, pyx:548-553
-            for (int i = t; i < K; i += ADAPT_NT) {
+            for (int i = t; i < K; i += NT) {
                 double v;
                 if (i == 0) v = __dadd_rn(__dmul_rn(7., avg[0]), avg[1]);
                 else if (i == K - 1) v = __dadd_rn(__dmul_rn(7., avg[K - 1]), avg[K - 2]);
@@ -241,10 +240,10 @@ __device__ void adapt_axis(const AdaptArgs &a, int d, double *avg, double *tmp, 
                 tmp[i] = __dmul_rn(fabs(v), 0.125);   // == v / 8 exactly
             }
             __syncthreads();
-            double s = block_sum<ADAPT_NT>(tmp, K, part);
+            double s = block_sum(tmp, K, part);
             // normalise + damp, pyx:554-562
             const double rs = (s > 0) ? 1.0 / s : 0.0;
-            for (int i = t; i < K; i += ADAPT_NT) {
+            for (int i = t; i < K; i += NT) {
                 double v;
                 if (a.fast) {
                     v = (s > 0) ? tmp[i] * rs + VG_TINY : VG_TINY;
@@ -263,7 +262,7 @@ __device__ void adapt_axis(const AdaptArgs &a, int d, double *avg, double *tmp, 
     double *P = tmp;
     const double *gd = a.grid + d * a.ldg;
     const double *id = a.inc + d * a.ldi;
-    for (int i = t; i < K; i += ADAPT_NT) {
+    for (int i = t; i < K; i += NT) {
         P[i] = avg[i];
         if (gs != nullptr) {
             gs[i] = gd[i];
@@ -276,11 +275,11 @@ __device__ void adapt_axis(const AdaptArgs &a, int d, double *avg, double *tmp, 
         gd = gs;
         id = is;
     }
-    block_inclusive_scan<ADAPT_NT>(P, K, part);
+    block_inclusive_scan(P, K, part);
     const double total = P[K - 1];
     const double f_ninc = a.fast ? div_fast(total, (double)Kn) : __ddiv_rn(total, (double)Kn);
     double *ng = a.new_grid + d * a.ldg_new;
-    for (int i = t; i <= Kn; i += ADAPT_NT) {
+    for (int i = t; i <= Kn; i += NT) {
         double v;
         if (i == 0) v = gd[0];
         else if (i == Kn) v = gd[K];
@@ -304,7 +303,7 @@ __device__ void adapt_axis(const AdaptArgs &a, int d, double *avg, double *tmp, 
     }
     __syncthreads();
     double *ni = a.new_inc + d * a.ldi_new;
-    for (int i = t; i < Kn; i += ADAPT_NT) ni[i] = __dsub_rn(ng[i + 1], ng[i]);
+    for (int i = t; i < Kn; i += NT) ni[i] = __dsub_rn(ng[i + 1], ng[i]);
     __syncthreads();
 }
 

@@ -51,10 +51,7 @@ size_t smem_budget(int minb)
 
 size_t range_smem(int ntb, int dim, int maxK, int tab_len, int train, size_t budget, int *table, int *copies)
 {
-    if (ntb == 256) return vg::range_fit<256>(dim, maxK, tab_len, train, 1, budget, table, copies).total;
-    if (ntb == 512) return vg::range_fit<512>(dim, maxK, tab_len, train, 1, budget, table, copies).total;
-    if (ntb == 768) return vg::range_fit<768>(dim, maxK, tab_len, train, 1, budget, table, copies).total;
-    return vg::range_fit<1024>(dim, maxK, tab_len, train, 1, budget, table, copies).total;
+    return vg::range_fit(ntb, dim, maxK, tab_len, train, 1, budget, table, copies).total;
 }
 
 int bucket_of(int dim) { return dim <= 4 ? 0 : (dim <= 8 ? 1 : 2); }

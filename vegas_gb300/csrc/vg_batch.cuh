@@ -75,12 +75,15 @@ __device__ __forceinline__ bool group_barrier(unsigned int *ctr, unsigned int ta
 constexpr int APER = 4;          // hypercubes per thread and pass of the allocation
 constexpr int F64_S = 2;         // samples per thread of the FP64 tiles
 
+// Chunks of 128 samples in a unit: one where a CTA has the integral to itself
+// (its warps then stay together in the sample order), four in a group of CTAs.
+__device__ __forceinline__ int deal_chunks(int G) { return G > 1 ? 4 : 1; }
+
 // Allocation of one iteration by one CTA: neval_h, offsets, tile heads,
 // totals in the integral's stats (the three allocation kernels' work).
-template <int NTB>
-static __device__ __noinline__ void cta_alloc(const IterArgs &a, int64_t *scan /* NTB/32 */)
+static __device__ __noinline__ void cta_alloc(const IterArgs &a, int64_t *scan /* one per warp */)
 {
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, NTB = (int)blockDim.x;
     build_tablef(a, tid, NTB);   // the FP32 grid table of this iteration
     vg_stats *st = a.stats;
     const double sum_sigf = st->sum_sigf;
@@ -110,7 +113,7 @@ static __device__ __noinline__ void cta_alloc(const IterArgs &a, int64_t *scan /
             s += n;
         }
         int64_t total;
-        int64_t off = run + block_excl_scan<NTB>(s, scan, &total);
+        int64_t off = run + block_excl_scan(s, scan, &total);
 #pragma unroll
         for (int k = 0; k < APER; k++) {
             const int64_t h = base + (int64_t)tid * APER + k;
@@ -124,7 +127,7 @@ static __device__ __noinline__ void cta_alloc(const IterArgs &a, int64_t *scan /
         }
         run += total;
     }
-    mxn = block_max<NTB>(mxn, scan);
+    mxn = block_max(mxn, scan);
     if (tid == 0) {
         const int64_t N = run;
         int64_t ntiles = (N + BASE_TILE - 1) / BASE_TILE;
@@ -152,13 +155,12 @@ static __device__ __noinline__ void cta_alloc(const IterArgs &a, int64_t *scan /
 // CTAs plus the Chan et al. merge of every hypercube cut by the ends of the
 // warps' ranges (the finalize kernels' work); sum_sigf and the constant-integrand
 // reset (pyx:2209-2215).
-template <int NTB>
 static __device__ __noinline__ void cta_finalize(const IterArgs &a, int ngroup, int *flag)
 {
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, NTB = (int)blockDim.x;
     vg_stats *st = a.stats;
     float s6[6];
-    finalize_ranges<NTB>(a, ngroup, (int64_t)ngroup * (NTB / 32 / GROUP), ngroup > 1, s6);
+    finalize_ranges(a, ngroup, (int64_t)ngroup * (NTB / 32 / GROUP), deal_chunks(ngroup), s6);
     if (tid == 0) {
         st->mean = vg_ff_value(s6[0], s6[1]);
         st->var = vg_ff_value(s6[2], s6[3]);
@@ -258,17 +260,16 @@ static __device__ __noinline__ void cta_finalize_f64(const IterArgs &a, int ngro
 
 // End of iteration: adapt the map (one axis after another), copy the new
 // grid back, clear the training histogram (vg_end_iteration's work).
-template <int NTB>
 static __device__ __noinline__ void cta_adapt(const BatchJob &J, const IterArgs &a, unsigned char *smem)
 {
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, NTB = (int)blockDim.x;
     const vgadapt::AdaptArgs &ad = J.ad;
     double *avg = (double *)smem;
     double *tmp = avg + ad.max_old;
     double *part = tmp + ad.max_old;
     for (int i = tid; i < ad.max_old; i += NTB) avg[i] = 1.0;
     __syncthreads();
-    for (int d = 0; d < ad.dim; d++) vgadapt::adapt_axis<NTB, 256>(ad, d, avg, tmp, part);
+    for (int d = 0; d < ad.dim; d++) vgadapt::adapt_axis<256>(ad, d, avg, tmp, part);
     __syncthreads();
     for (int d = 0; d < ad.dim; d++) {
         const int K = ad.old_ninc[d];
@@ -311,18 +312,48 @@ static __device__ __noinline__ void cta_ravg(const BatchJob &J, int nitn, int nw
     J.res[3] = (double)(cnt > 0 ? cnt - 1 : 0);
 }
 
+// The fused body of one integral, compiled for its dimension.
+template <int KIND, int DIM, int F>
+static __device__ __noinline__ void cta_range(const IterArgs &a, const VgParams &prm, unsigned char *smem, int rank,
+                                              int G)
+{
+    range_body<MODE_FUSED, KIND, DIM, F>(a, prm, smem, rank, G, deal_chunks(G));
+}
+
+template <int KIND, int DIMB>
+__device__ __forceinline__ void range_dispatch(const IterArgs &a, const VgParams &prm, unsigned char *smem, int rank,
+                                               int G)
+{
+    constexpr int ET = RF_EXACT | RF_TABLE;
+    if (a.wide || (a.train && !a.hist_smem) || (DIMB <= 8 && !a.table_smem)) return cta_range<KIND, DIMB, RF_GENERAL>(a, prm, smem, rank, G);
+    if constexpr (DIMB == 4) {
+        if (a.dim == 4) cta_range<KIND, 4, ET>(a, prm, smem, rank, G);
+        else if (a.dim == 3) cta_range<KIND, 3, ET>(a, prm, smem, rank, G);
+        else if (a.dim == 2) cta_range<KIND, 2, ET>(a, prm, smem, rank, G);
+        else cta_range<KIND, 1, ET>(a, prm, smem, rank, G);
+    } else if constexpr (DIMB == 8) {
+        if (a.dim == 8) cta_range<KIND, 8, ET>(a, prm, smem, rank, G);
+        else if (a.dim == 7) cta_range<KIND, 7, ET>(a, prm, smem, rank, G);
+        else if (a.dim == 6) cta_range<KIND, 6, ET>(a, prm, smem, rank, G);
+        else cta_range<KIND, 5, ET>(a, prm, smem, rank, G);
+    } else {
+        if (a.table_smem) cta_range<KIND, DIMB, RF_TABLE>(a, prm, smem, rank, G);
+        else cta_range<KIND, DIMB, 0>(a, prm, smem, rank, G);
+    }
+}
+
 // The persistent kernel of one dimension bucket (every integral it takes has
 // dim <= DIMB): sampling, map and evaluation in T (float; double in the
-// FP64 parity configuration), NTB threads per CTA and MINB CTAs per SM (the
-// occupancy the autotuner picks per bucket).
+// FP64 parity configuration), at most MAXT threads per CTA (the number of
+// threads and of CTAs per SM is picked by the autotuner per bucket).
 //
 // Queue mode (group <= 1): each CTA takes whole integrals from the queue.
 // Group mode (group = G >= 2, cooperative launch): CTA c works on integral
 // order[c / G] as rank c % G; rank 0 allocates, finalizes and adapts, all G
 // ranks share the tiles (rank r takes tiles r, r + G, ...), with two group
 // barriers per iteration.
-template <typename T, int KIND, int DIMB, int NTB, int MINB>
-__global__ void __launch_bounds__(NTB, MINB) batch_kernel(const BatchJob *__restrict__ jobs,
+template <typename T, int KIND, int DIMB, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1) batch_kernel(const BatchJob *__restrict__ jobs,
                                                    const VgParams *__restrict__ params,
                                                    const int *__restrict__ order, int njobs, int nitn,
                                                    int nwarm, uint32_t itn0, unsigned int *queue,
@@ -330,10 +361,10 @@ __global__ void __launch_bounds__(NTB, MINB) batch_kernel(const BatchJob *__rest
 {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ IterArgs sa;
-    __shared__ int64_t scan[NTB / 32];
-    __shared__ VgKSum red[NTB / 32];
+    __shared__ int64_t scan[MAXT / 32];
+    __shared__ VgKSum red[MAXT / 32];
     __shared__ int s_q, s_flag;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, NTB = (int)blockDim.x;
     const int G = group > 1 ? group : 1;
     const int rank = G > 1 ? (int)(blockIdx.x % G) : 0;
     bool first = true;
@@ -368,27 +399,25 @@ __global__ void __launch_bounds__(NTB, MINB) batch_kernel(const BatchJob *__rest
         for (int it = 0; it < nitn && ok; it++) {
             if (tid == 0) sa.itn = itn0 + (uint32_t)it;
             __syncthreads();
-            if (rank == 0) cta_alloc<NTB>(sa, scan);
+            if (rank == 0) cta_alloc(sa, scan);
             if (G > 1 && !(ok = group_barrier(J.sync, (unsigned)G * ++rounds, sa.wait_iters))) break;
             if (sa.stats->ntiles > 0) {
                 if constexpr (sizeof(T) == 8)
-                    tile_body<MODE_FUSED, KIND, DIMB, F64_S, NTB>(sa, params[j], smem, rank, G, rank);
-                else if (G > 1)
-                    range_body<MODE_FUSED, KIND, DIMB, NTB, true>(sa, params[j], smem, rank, G);
+                    tile_body<MODE_FUSED, KIND, DIMB, F64_S, MAXT>(sa, params[j], smem, rank, G, rank);
                 else
-                    range_body<MODE_FUSED, KIND, DIMB, NTB, false>(sa, params[j], smem, 0, 1);
+                    range_dispatch<KIND, DIMB>(sa, params[j], smem, rank, G);
             }
             __syncthreads();
             if (G > 1 && !(ok = group_barrier(J.sync, (unsigned)G * ++rounds, sa.wait_iters))) break;
             if (rank == 0) {
                 if constexpr (sizeof(T) == 8) cta_finalize_f64(sa, G, red, &s_flag);
-                else cta_finalize<NTB>(sa, G, &s_flag);
+                else cta_finalize(sa, G, &s_flag);
                 if (tid == 0) {
                     J.out[3 * it] = sa.stats->mean;
                     J.out[3 * it + 1] = sa.stats->var;
                     J.out[3 * it + 2] = (double)sa.stats->neval;
                 }
-                if (J.adapt) cta_adapt<NTB>(J, sa, smem);
+                if (J.adapt) cta_adapt(J, sa, smem);
             }
             __syncthreads();
         }
@@ -404,29 +433,29 @@ __global__ void __launch_bounds__(NTB, MINB) batch_kernel(const BatchJob *__rest
 
 // Launch (queue mode, or cooperative for co-resident groups) and occupancy
 // of one instantiation; the bucket files dispatch to these.
-template <typename T, int KIND, int DIMB, int NTB, int MINB>
-int launch_one(const BatchJob *jobs, const VgParams *prm, const int *order, int njobs, int nitn, int nwarm,
+template <typename T, int KIND, int DIMB, int MAXT>
+int launch_one(int ntb, const BatchJob *jobs, const VgParams *prm, const int *order, int njobs, int nitn, int nwarm,
                uint32_t itn0, unsigned int *queue, size_t smem, int grid, int group, int *status, cudaStream_t st)
 {
-    auto k = batch_kernel<T, KIND, DIMB, NTB, MINB>;
+    auto k = batch_kernel<T, KIND, DIMB, MAXT>;
     if (group > 1) {
         void *args[] = {(void *)&jobs, (void *)&prm, (void *)&order, (void *)&njobs, (void *)&nitn, (void *)&nwarm,
                         (void *)&itn0, (void *)&queue, (void *)&group, (void *)&status};
-        VG_CUDA_CHECK(cudaLaunchCooperativeKernel((const void *)k, dim3((unsigned)grid), dim3(NTB), args, smem, st));
+        VG_CUDA_CHECK(cudaLaunchCooperativeKernel((const void *)k, dim3((unsigned)grid), dim3(ntb), args, smem, st));
         return VG_OK;
     }
-    k<<<grid, NTB, smem, st>>>(jobs, prm, order, njobs, nitn, nwarm, itn0, queue, group, status);
+    k<<<grid, ntb, smem, st>>>(jobs, prm, order, njobs, nitn, nwarm, itn0, queue, group, status);
     VG_LAUNCH_CHECK();
     return VG_OK;
 }
 
 // sets the kernel's shared-memory attribute (outside any stream capture)
-template <typename T, int KIND, int DIMB, int NTB, int MINB>
-int occupancy_one(size_t smem, int *per_sm)
+template <typename T, int KIND, int DIMB, int MAXT>
+int occupancy_one(int ntb, size_t smem, int *per_sm)
 {
-    auto k = batch_kernel<T, KIND, DIMB, NTB, MINB>;
-    VG_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    VG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k, NTB, smem));
+    auto k = batch_kernel<T, KIND, DIMB, MAXT>;
+    VG_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    VG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k, ntb, smem));
     return VG_OK;
 }
 
@@ -445,7 +474,7 @@ constexpr int F64_DIMB = 8;
 constexpr BucketConfig BUCKET_CONFIGS[NBUCKET][NCONFIG] = {
     {{1024, 1}, {512, 2}, {256, 4}},   // dim <= 4
     {{512, 2}, {1024, 1}, {768, 1}},   // dim <= 8
-    {{768, 1}, {512, 1}, {1024, 1}},   // dim <= 16
+    {{768, 1}, {512, 1}, {256, 2}},    // dim <= 16
 };
 
 // One bucket's launch and occupancy for configuration cfg (instantiated by
@@ -456,30 +485,15 @@ int bucket_launch(int cfg, const BatchJob *jobs, const VgParams *prm, const int 
                   cudaStream_t st)
 {
     constexpr int b = DIMB == 4 ? 0 : (DIMB == 8 ? 1 : 2);
-    constexpr BucketConfig c0 = BUCKET_CONFIGS[b][0], c1 = BUCKET_CONFIGS[b][1], c2 = BUCKET_CONFIGS[b][2];
-    switch (cfg) {
-    case 0:
-        return launch_one<float, KIND, DIMB, c0.ntb, c0.minb>(jobs, prm, order, njobs, nitn, nwarm, itn0, queue, smem, grid,
-                                                     group, status, st);
-    case 1:
-        return launch_one<float, KIND, DIMB, c1.ntb, c1.minb>(jobs, prm, order, njobs, nitn, nwarm, itn0, queue, smem, grid,
-                                                     group, status, st);
-    default:
-        return launch_one<float, KIND, DIMB, c2.ntb, c2.minb>(jobs, prm, order, njobs, nitn, nwarm, itn0, queue, smem, grid,
-                                                     group, status, st);
-    }
+    return launch_one<float, KIND, DIMB, range_threads(DIMB)>(BUCKET_CONFIGS[b][cfg].ntb, jobs, prm, order, njobs, nitn,
+                                                              nwarm, itn0, queue, smem, grid, group, status, st);
 }
 
 template <int KIND, int DIMB>
 int bucket_occupancy(int cfg, size_t smem, int *per_sm)
 {
     constexpr int b = DIMB == 4 ? 0 : (DIMB == 8 ? 1 : 2);
-    constexpr BucketConfig c0 = BUCKET_CONFIGS[b][0], c1 = BUCKET_CONFIGS[b][1], c2 = BUCKET_CONFIGS[b][2];
-    switch (cfg) {
-    case 0: return occupancy_one<float, KIND, DIMB, c0.ntb, c0.minb>(smem, per_sm);
-    case 1: return occupancy_one<float, KIND, DIMB, c1.ntb, c1.minb>(smem, per_sm);
-    default: return occupancy_one<float, KIND, DIMB, c2.ntb, c2.minb>(smem, per_sm);
-    }
+    return occupancy_one<float, KIND, DIMB, range_threads(DIMB)>(BUCKET_CONFIGS[b][cfg].ntb, smem, per_sm);
 }
 
 // The entry points of each bucket's translation unit.

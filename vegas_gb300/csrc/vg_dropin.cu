@@ -13,10 +13,7 @@ int launch_points(IterArgs &a, int f64, cudaStream_t st)
         if (a.dim <= 8) return launch_tile<MODE_POINTS, 0, 8, 1>(a, nullptr, st);
         return launch_tile<MODE_POINTS, 0, 64, 1>(a, nullptr, st);
     }
-    if (a.dim <= 4) return launch_range<MODE_POINTS, 0, 4>(a, nullptr, 0, st);
-    if (a.dim <= 8) return launch_range<MODE_POINTS, 0, 8>(a, nullptr, 0, st);
-    if (a.dim <= 16) return launch_range<MODE_POINTS, 0, 16>(a, nullptr, 0, st);
-    return launch_range<MODE_POINTS, 0, 64>(a, nullptr, 0, st);
+    return launch_range<MODE_POINTS, 0>(a, nullptr, 0, st);
 }
 
 int launch_reduce(IterArgs &a, int f64, cudaStream_t st)
@@ -25,10 +22,7 @@ int launch_reduce(IterArgs &a, int f64, cudaStream_t st)
         if (a.dim <= 8) return launch_tile<MODE_REDUCE, 0, 8, 2>(a, nullptr, st);
         return launch_tile<MODE_REDUCE, 0, 64, 1>(a, nullptr, st);
     }
-    if (a.dim <= 4) return launch_range<MODE_REDUCE, 0, 4>(a, nullptr, 0, st);
-    if (a.dim <= 8) return launch_range<MODE_REDUCE, 0, 8>(a, nullptr, 0, st);
-    if (a.dim <= 16) return launch_range<MODE_REDUCE, 0, 16>(a, nullptr, 0, st);
-    return launch_range<MODE_REDUCE, 0, 64>(a, nullptr, 0, st);
+    return launch_range<MODE_REDUCE, 0>(a, nullptr, 0, st);
 }
 
 int launch_reduce_kept(IterArgs &a, int f64, cudaStream_t st)
@@ -37,10 +31,7 @@ int launch_reduce_kept(IterArgs &a, int f64, cudaStream_t st)
         if (a.dim <= 8) return launch_tile<MODE_REDUCE_KEPT, 0, 8, 2>(a, nullptr, st);
         return launch_tile<MODE_REDUCE_KEPT, 0, 64, 1>(a, nullptr, st);
     }
-    if (a.dim <= 4) return launch_range<MODE_REDUCE_KEPT, 0, 4>(a, nullptr, 0, st);
-    if (a.dim <= 8) return launch_range<MODE_REDUCE_KEPT, 0, 8>(a, nullptr, 0, st);
-    if (a.dim <= 16) return launch_range<MODE_REDUCE_KEPT, 0, 16>(a, nullptr, 0, st);
-    return launch_range<MODE_REDUCE_KEPT, 0, 64>(a, nullptr, 0, st);
+    return launch_range<MODE_REDUCE_KEPT, 0>(a, nullptr, 0, st);
 }
 
 }  // namespace vg

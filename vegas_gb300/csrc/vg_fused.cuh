@@ -20,21 +20,16 @@ int launch_fused_kind(IterArgs &a, const VgParams &P, int tab_len, int f64, cuda
         if (a.dim <= 8) return launch_tile<MODE_FUSED, KIND, 8, 2>(a, &P, st);
         return launch_tile<MODE_FUSED, KIND, 64, 1>(a, &P, st);
     }
-    if (KIND == VG_F_RIDGE && g_eval_split == 2) {
-        int rc;
-        if (a.dim <= 4) rc = launch_range<MODE_EVAL, KIND, 4>(a, &P, tab_len, st);
-        else if (a.dim <= 8) rc = launch_range<MODE_EVAL, KIND, 8>(a, &P, tab_len, st);
-        else if (a.dim <= 16) rc = launch_range<MODE_EVAL, KIND, 16>(a, &P, tab_len, st);
-        else rc = launch_range<MODE_EVAL, KIND, 64>(a, &P, tab_len, st);
+    if constexpr (KIND == VG_F_RIDGE) {
+      if (g_eval_split == 2) {
+        int rc = launch_range<MODE_EVAL, KIND>(a, &P, tab_len, st);
         if (rc) return rc;
         a.f_in = a.f_eval;
         a.f_f64 = 0;
         return launch_reduce(a, 0, st);
+      }
     }
-    if (a.dim <= 4) return launch_range<MODE_FUSED, KIND, 4>(a, &P, tab_len, st);
-    if (a.dim <= 8) return launch_range<MODE_FUSED, KIND, 8>(a, &P, tab_len, st);
-    if (a.dim <= 16) return launch_range<MODE_FUSED, KIND, 16>(a, &P, tab_len, st);
-    return launch_range<MODE_FUSED, KIND, 64>(a, &P, tab_len, st);
+    return launch_range<MODE_FUSED, KIND>(a, &P, tab_len, st);
 }
 
 int launch_fused_gauss(IterArgs &a, const VgParams &P, int tab_len, int f64, cudaStream_t st);

@@ -125,8 +125,8 @@ __global__ void __launch_bounds__(ALLOC_NT) alloc_kernel(IterArgs a, int64_t nbl
             if (h0 + k < a.H) a.neval_h[h0 + k] = (int32_t)loc[k];
     }
     int64_t tot;
-    int64_t run = block_excl_scan<ALLOC_NT>(sum, wtot, &tot);
-    const int64_t bm = block_max<ALLOC_NT>(m, wtot);
+    int64_t run = block_excl_scan(sum, wtot, &tot);
+    const int64_t bm = block_max(m, wtot);
     // warp 0: publish the block total, then look back 32 predecessors at a
     // time (each lane waits for one published word; the nearest inclusive
     // prefix ends the walk)
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(FIN32_NT) finalize32_kernel(const __grid_const
 {
     __shared__ int s_reset;
     float s6[6];
-    finalize_ranges<FIN32_NT>(a, a.ncta, a.ngroups, false, s6);
+    finalize_ranges(a, a.ncta, a.ngroups, 0, s6);
     finalize_store(a, vg_ff_value(s6[0], s6[1]), vg_ff_value(s6[2], s6[3]), vg_ff_value(s6[4], s6[5]), &s_reset);
 }
 
@@ -420,7 +420,7 @@ WorkLayout layout(const vg_integrator *it, int64_t ncap)
     const int64_t tiles = (ncap + 255) / 256 + 1;
     L.part_cap = L.ntiles_cap < MAX_PARTS ? L.ntiles_cap : (int64_t)MAX_PARTS;
     if (L.part_cap < 1024) L.part_cap = 1024;   // the batched launch's groups of CTAs, whatever the integral's size
-    const int64_t units = L.ntiles_cap / DEAL_CHUNKS + 2;
+    const int64_t units = L.ntiles_cap + 1;
     L.rec_cap = f64 ? tiles : (units > L.part_cap ? units : L.part_cap);
     const int64_t fin = L.rec_cap > L.part_cap ? L.rec_cap : L.part_cap;
     L.recs = o;    o = align256(o + (f64 ? sizeof(TileRec) : sizeof(RangeRec)) * 2 * L.rec_cap);
@@ -471,6 +471,7 @@ int fill_args(IterArgs &a, const vg_integrator *it, uint32_t itn, const double *
     a.H = it->nhcube;
     a.wide |= it->nhcube > 0x7fffffff;
     a.ncap = neval_cap(it);
+    a.wide |= a.ncap > 0x7fffffff - 4096;
     WorkLayout L = layout(it, a.ncap);
     if (it->work_bytes < L.total)
         return vg_fail(VG_ERR_VALUE, "workspace too small: %zu < %zu", it->work_bytes, L.total);

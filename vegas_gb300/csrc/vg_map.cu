@@ -124,9 +124,9 @@ __global__ void __launch_bounds__(ADAPT_NT) adapt_kernel(AdaptArgs a)
     for (int i = threadIdx.x; i < a.max_old; i += ADAPT_NT) avg[i] = 1.0;
     __syncthreads();
     if (a.sequential) {
-        for (int d = 0; d < a.dim; d++) vgadapt::adapt_axis<ADAPT_NT>(a, d, avg, tmp, part, gs, is);
+        for (int d = 0; d < a.dim; d++) vgadapt::adapt_axis(a, d, avg, tmp, part, gs, is);
     } else {
-        vgadapt::adapt_axis<ADAPT_NT>(a, blockIdx.x, avg, tmp, part, gs, is);
+        vgadapt::adapt_axis(a, blockIdx.x, avg, tmp, part, gs, is);
     }
 }
 

@@ -49,8 +49,8 @@ struct RangePlan {
     size_t table, hsum, hcnt, itab, red, recs, warps, total;
 };
 
-template <int NTB>
-__host__ __device__ inline RangePlan range_plan(int dim, int maxK, int table_smem, int hist_copies, int tab_len)
+__host__ __device__ inline RangePlan range_plan(int ntb, int dim, int maxK, int table_smem, int hist_copies,
+                                                int tab_len)
 {
     RangePlan p;
     size_t o = 0;
@@ -63,11 +63,11 @@ __host__ __device__ inline RangePlan range_plan(int dim, int maxK, int table_sme
     p.itab = o;
     o = (o + sizeof(float) * (tab_len + 4) + 15) & ~(size_t)15;
     p.red = o;
-    o = (o + sizeof(float) * 6 * (NTB / 32) + 15) & ~(size_t)15;
+    o = (o + sizeof(float) * 6 * (ntb / 32) + 15) & ~(size_t)15;
     p.recs = o;
-    o += sizeof(RangeRec) * 2 * (NTB / 32);
+    o += sizeof(RangeRec) * 2 * (ntb / 32);
     p.warps = o;
-    o += sizeof(WarpBuf) * (NTB / 32);
+    o += sizeof(WarpBuf) * (ntb / 32);
     p.total = o;
     return p;
 }
@@ -79,12 +79,11 @@ __host__ __device__ inline RangePlan range_plan(int dim, int maxK, int table_sme
 // samples of dim 4).
 constexpr int GROUP = 8;
 // Records of an iteration of N samples: one pair per group that has any chunk,
-// or, where units of DEAL_CHUNKS chunks are dealt to the CTAs, per unit.
-constexpr int DEAL_CHUNKS = 4;
-__host__ __device__ __forceinline__ int64_t record_count(int64_t N, int64_t ngroups, bool deal)
+// or, where units of `deal` chunks are dealt to the warps (deal > 0), per unit.
+__host__ __device__ __forceinline__ int64_t record_count(int64_t N, int64_t ngroups, int deal)
 {
     const int64_t c = (N + CHUNK - 1) / CHUNK;
-    return deal ? (c + DEAL_CHUNKS - 1) / DEAL_CHUNKS : (c < ngroups ? c : ngroups);
+    return deal ? (c + deal - 1) / deal : (c < ngroups ? c : ngroups);
 }
 
 // Sums of d = x - c and d^2 in float-float (TwoDiff and TwoProd, error-free).
@@ -153,22 +152,12 @@ static __device__ __noinline__ int wide_digit(int64_t &h, int nstrat)
     return y0;
 }
 
-// A piece of a hypercube cut by the end of a range: its sum and its squared
-// deviations about its own mean, for the finalize's merge.
-static __device__ __noinline__ void put_record(RangeRec *slot, int64_t h, int n, float c, DQ v, int spans)
+// adapt_to_errors: a hypercube's |variance| trains the map at its last sample.
+static __device__ __noinline__ void train_last(const IterArgs &a, int64_t h, double v)
 {
-    const float fn = (float)n;
-    float sh, sl;
-    piece_sum(fn, c, v, sh, sl);
-    if (v.qh == 0.f) {
-        v.qh = guard_q(fn, sh);
-    } else {
-        float d2h, d2l, th, tl;
-        ff_sqr(v.dh, v.dl, d2h, d2l);
-        ff_div_f(d2h, d2l, fn, th, tl);
-        ff_add_pair(v.qh, v.ql, -th, -tl);
-    }
-    *slot = RangeRec{h, n, spans, sh, sl, v.qh, v.ql};
+    unsigned short b[VG_MAX_DIM];
+    last_sample_bins<float>(a, h, b);
+    train_hcube(a, b, v);
 }
 
 // Running sums of the hypercubes a lane finishes.
@@ -218,9 +207,7 @@ __device__ __forceinline__ void finish_hcube(const IterArgs &a, int64_t h, int n
             ff_from_double(r.z, rh, rl);
             ff_add_pair(s.sh, s.sl, rh, rl);
         } else {
-            unsigned short b[VG_MAX_DIM];
-            last_sample_bins<float>(a, h, b);
-            train_hcube(a, b, r.z);
+            train_last(a, h, r.z);
         }
         return;
     }
@@ -240,11 +227,7 @@ __device__ __forceinline__ void finish_hcube(const IterArgs &a, int64_t h, int n
         a.sigf[h] = (double)sg;
         vg_ff_add(s.sh, s.sl, sg);
     }
-    if (a.train_hc) {   // adapt_to_errors: train at the hypercube's last sample
-        unsigned short b[VG_MAX_DIM];
-        last_sample_bins<float>(a, h, b);
-        train_hcube(a, b, fabs(vg_ff_value(vh, vl)));
-    }
+    if (a.train_hc) train_last(a, h, fabs(vg_ff_value(vh, vl)));
 }
 
 // A piece of a hypercube cut by the ends of ranges: samples, sum, squared
@@ -252,6 +235,28 @@ __device__ __forceinline__ void finish_hcube(const IterArgs &a, int64_t h, int n
 // parallel-variance update: Q = Q1 + Q2 + (m2 - m1)^2 n1 n2 / (n1 + n2).
 struct Piece {
     float n, sh, sl, qh, ql;
+    __device__ __forceinline__ void from(const RangeRec &r)
+    {
+        n = (float)(r.n < 0 ? -r.n : r.n);
+        sh = r.dh;
+        sl = r.dl;
+        qh = r.qh;
+        ql = r.ql;
+        if (r.c != r.c) return;
+        piece_sum(n, r.c, DQ{r.dh, r.dl, r.qh, r.ql}, sh, sl);
+        if (qh == 0.f) {
+            qh = guard_q(n, sh);
+        } else {
+            float d2h, d2l, th, tl;
+            ff_sqr(r.dh, r.dl, d2h, d2l);
+            ff_div_f(d2h, d2l, n, th, tl);
+            ff_add_pair(qh, ql, -th, -tl);
+        }
+    }
+    __device__ __forceinline__ RangeRec record(int64_t h, bool spans) const
+    {
+        return RangeRec{h, spans ? -(int)n : (int)n, __int_as_float(0x7fffffff), sh, sl, qh, ql};
+    }
     __device__ __forceinline__ void put_first(const Piece &p)   // p comes before this one
     {
         if (!(p.n > 0.f)) return;
@@ -296,11 +301,7 @@ static __device__ __noinline__ void finish_cut(const IterArgs &a, int64_t h, con
         vh = (float)v;
         vl = (float)(v - (double)vh);
     }
-    if (a.train_hc) {   // adapt_to_errors: train at the hypercube's last sample
-        unsigned short b[VG_MAX_DIM];
-        last_sample_bins<float>(a, h, b);
-        train_hcube(a, b, fabs(vg_ff_value(vh, vl)));
-    }
+    if (a.train_hc) train_last(a, h, fabs(vg_ff_value(vh, vl)));
     ff_add_pair(s6[0], s6[1], p.sh, p.sl);
     ff_add_pair(s6[2], s6[3], vh, vl);
     if (a.adaptive) {
@@ -328,24 +329,49 @@ __device__ __forceinline__ bool scan_pieces(Piece &cur, bool started)
 }
 
 // ------------------------------------------------------------------ kernel
+template <bool WIDE>
+struct IndexType {
+    typedef int type;
+};
+template <>
+struct IndexType<true> {
+    typedef int64_t type;
+};
+
+// What a body is compiled for.  A sample's code reads few of the run-time
+// choices below again and again for each axis; compiled in, they take a third
+// of the instructions away (2^20 samples of the 8-d mixture: 37 -> 25 million
+// warp instructions).
+constexpr int RF_EXACT = 1;   // dim == DIMB
+constexpr int RF_TABLE = 2;   // the grid table is in shared memory (else: read through L1)
+constexpr int RF_GENERAL = 4; // injected uniforms, 2^31 hypercubes or samples, 2^24 strata on an axis, the table
+                              // and the histogram in either place
+
 // The work of CTA `rank` of `nranks` on one integral's iteration; its partial
-// sums go to a.parts[rank].  DEAL (the batched launch's groups of CTAs): units
-// of 512 samples are dealt to the CTAs in turn.  Which samples share a CTA's
-// FP32 histogram decides how its sums are rounded, and on the lattice integrals
-// (a few samples carry a bin) adapting amplifies that a thousandfold: the units
-// keep the results of the launches before this kernel to the atomics' noise.
-template <int MODE, int KIND, int DIMB, int NTB, bool DEAL>
+// sums go to a.parts[rank].  deal > 0 (the batched launch): units of `deal`
+// chunks are dealt to the CTAs and their warps in turn.  Which samples share a
+// CTA's FP32 histogram, and in what order they come, decides how its sums are
+// rounded; where a few samples carry a bin (the lattice integrals, Lorentzians
+// in 9 dimensions) adapting from iteration to iteration amplifies that a
+// thousandfold.  Dealt units add in the order of the samples as a CTA walking
+// tile by tile does, so results stay those of such a launch to the atomics'
+// noise.
+template <int MODE, int KIND, int DIMB, int F>
 __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &prm, unsigned char *smem, int rank,
-                                           int nranks)
+                                           int nranks, int deal)
 {
     constexpr bool NEED_RED = (MODE == MODE_REDUCE || MODE == MODE_FUSED || MODE == MODE_REDUCE_KEPT);
     constexpr bool NEED_MAP = MODE != MODE_REDUCE_KEPT;
     constexpr bool NEED_X = MODE == MODE_POINTS || MODE == MODE_FUSED || MODE == MODE_EVAL;
-    constexpr int NW = NTB / 32;
-    const int dim = a.dim;
+    constexpr bool GENERAL = F & RF_GENERAL;
+    typedef typename IndexType<GENERAL>::type Idx;   // samples and hypercubes
+    const int NTB = (int)blockDim.x, NW = NTB >> 5;
+    const int dim = (F & RF_EXACT) ? DIMB : a.dim;
+    const bool table_smem = NEED_MAP && (GENERAL ? a.table_smem != 0 : bool(F & RF_TABLE));
+    const bool wide = GENERAL && a.wide;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int W = a.maxK + 1;
-    const RangePlan sp = range_plan<NTB>(dim, a.maxK, a.table_smem, a.hist_smem, a.tab_len);
+    const RangePlan sp = range_plan(NTB, dim, a.maxK, table_smem, a.hist_smem, a.tab_len);
     float2 *table = reinterpret_cast<float2 *>(smem + sp.table);
     float *hsum = reinterpret_cast<float *>(smem + sp.hsum);
     unsigned int *hcnt = reinterpret_cast<unsigned int *>(smem + sp.hcnt);
@@ -359,7 +385,7 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
     const int64_t N = a.stats->neval;
 
     // ---- per-CTA setup: grid table, histogram, integrand constants
-    if (NEED_MAP && a.table_smem)
+    if (NEED_MAP && table_smem)
         for (int i = tid; i < dim * W; i += NTB) table[i] = a.tablef[i];
     const int hist = dim * W;   // the last bin of an axis takes what is not counted
     if (NEED_RED && a.train && a.hist_smem) {
@@ -379,30 +405,37 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
     int nan_local = 0;
     LaneSums sums = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 
-    const int64_t nchunk = (N + CHUNK - 1) / CHUNK;
-    const int64_t nrec = record_count(N, (int64_t)nranks * (NW / GROUP), DEAL);
-    const int64_t seg = rank + (int64_t)nranks * (warp / GROUP);   // the group's range
-    int64_t seg0 = 0, nsc = 0;                                     // its chunks
-    if (!DEAL && seg < nrec) {
-        seg0 = nchunk * seg / nrec;
-        nsc = nchunk * (seg + 1) / nrec - seg0;
+    const unsigned int nchunk = (unsigned int)((N + CHUNK - 1) / CHUNK);
+    const unsigned int nrec = (unsigned int)record_count(N, (int64_t)nranks * (NW / GROUP), deal);
+    const unsigned int seg = rank + nranks * (warp / GROUP);   // the group's range
+    unsigned int seg0 = 0, nsc = 0;                            // its chunks
+    if (!deal && seg < nrec) {
+        const unsigned int q = nchunk / nrec, m = nchunk - q * nrec;
+        seg0 = seg * q + min(seg, m);
+        nsc = q + (seg < m);
     }
     // ranges of the group's warps, or units
-    const int64_t nu = DEAL ? nrec : (nsc < GROUP ? nsc : (int64_t)GROUP);
-    for (int64_t u = DEAL ? rank + (int64_t)nranks * warp : warp % GROUP; u < nu;
-         u += DEAL ? (int64_t)nranks * NW : (int64_t)GROUP) {
-        RangeRec *rec = DEAL ? a.rrecs + 2 * u : s_rec + 2 * warp;
-        const int64_t c0 = DEAL ? u * DEAL_CHUNKS : seg0 + nsc * u / nu;
-        const int64_t c1 = DEAL ? c0 + DEAL_CHUNKS : seg0 + nsc * (u + 1) / nu;
-        const int64_t s0 = c0 * CHUNK, s1 = c1 * CHUNK < N ? c1 * CHUNK : N;
-        int64_t h = a.tile_h0[c0];
-        bool cut0 = NEED_RED && a.offsets[h] < s0;   // the hypercube started before the range
-        const bool cut_first = cut0;
+    const unsigned int nu = deal ? nrec : min(nsc, (unsigned int)GROUP);
+    const unsigned int ustep = deal ? nranks * NW : GROUP;
+    Idx h_ahead = -1;   // dealt units: the next one's first hypercube, loaded a unit ahead
+    for (unsigned int u = deal ? rank + nranks * warp : warp % GROUP; u < nu; u += ustep) {
+        RangeRec *rec = deal ? a.rrecs + 2 * (size_t)u : s_rec + 2 * warp;
+        unsigned int c0 = u * deal, c1 = c0 + deal;
+        if (!deal) {
+            const unsigned int q = nsc / nu, m = nsc - q * nu;
+            c0 = seg0 + u * q + min(u, m);
+            c1 = c0 + q + (u < m);
+        }
+        const Idx s0 = (Idx)c0 * CHUNK, s1 = c1 < nchunk ? (Idx)c1 * CHUNK : (Idx)N;
+        Idx h = h_ahead >= 0 ? h_ahead : (Idx)a.tile_h0[c0];
+        if (deal && u + ustep < nu) h_ahead = (Idx)a.tile_h0[(u + ustep) * deal];
+        bool cut0 = false, cut_first = false;   // the hypercube started before the range
         bool open = false;
+        int n_open = 0;                         // samples of the open hypercube
         float c_open = 0.f;
         DQ v_open;
         v_open.zero();
-        for (int64_t b = s0; b < s1; b += CHUNK) {
+        for (Idx b = s0; b < s1; b += CHUNK) {
             const int len = (int)(s1 - b < CHUNK ? s1 - b : CHUNK);
             // ---- the hypercubes of the chunk
             int nw = 0;
@@ -411,9 +444,9 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
             for (int q = 0; q < 3; q++) {
                 const int k = 32 * q + lane;
                 // below 2^31 where it is used: a hypercube has at most that many samples
-                const int64_t d64 = (h + k <= a.H ? a.offsets[h + k] : N) - b;
-                const int rel = d64 > 0x7fffffff ? 0x7fffffff : (int)d64;
-                const bool in = h + k < a.H && rel < len;
+                const Idx dif = (Idx)(h + k <= (Idx)a.H ? a.offsets[h + k] : N) - b;
+                const int rel = GENERAL && dif > (Idx)0x7fffffff ? 0x7fffffff : (int)dif;
+                const bool in = h + k < (Idx)a.H && rel < len;
                 if (k < WCAP) wb.off[k] = rel;
                 if (k > 0 && in && rel >= 0) atomicOr(&wb.mask[rel >> 5], 1u << (rel & 31));
                 const unsigned int m = __ballot_sync(0xffffffffu, in);
@@ -438,10 +471,10 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
                 before += __popc(m);
                 float wf = 0.f;
                 if (li < len) {
-                    const int64_t ig = b + li;
+                    const Idx ig = b + li;
                     float jac = 1.f;
                     float x[DIMB];
-                    unsigned int bins[(DIMB + 1) / 2];   // training bins, 16 bits each (ninc: none)
+                    unsigned int bins[(DIMB + 3) / 4 * 2];   // training bins, 16 bits each (ninc: none)
                     if (NEED_MAP) {
                         unsigned int hh = (unsigned int)(h + cur);
                         int64_t hl = h + cur;
@@ -449,25 +482,24 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
                         for (int g = 0; 4 * g < DIMB; g++) {
                             if (4 * g >= dim) break;
                             float u[4];
-                            if (a.u != nullptr) {
+                            if (GENERAL && a.u != nullptr) {
 #pragma unroll
                                 for (int q = 0; q < 4; q++)
-                                    u[q] = 4 * g + q < dim ? (float)a.u[ig * dim + 4 * g + q] : 0.5f;
+                                    u[q] = 4 * g + q < dim ? (float)a.u[(size_t)ig * dim + 4 * g + q] : 0.5f;
                             } else {
                                 VgUniform<float>::group(a.seed, a.stream, a.itn, (uint64_t)ig, g, u);
                             }
 #pragma unroll
                             for (int q = 0; q < 4; q++) {
                                 const int d = 4 * g + q;
-                                if (d >= DIMB) continue;
                                 if (d >= dim) {
-                                    x[d] = 0.f;
+                                    if (d < DIMB) x[d] = 0.f;
                                     if (!(d & 1)) bins[d >> 1] = 0u;
                                     continue;
                                 }
                                 const AxisArgs &ax = a.ax[d];
                                 int y0;
-                                if (!a.wide) {
+                                if (!wide) {
                                     const unsigned int qh = __umulhi(hh << 1, ax.dmul) >> ax.dshift;
                                     y0 = (int)(hh - qh * (unsigned int)ax.nstrat);
                                     hh = qh;
@@ -480,22 +512,22 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
                                 // y <= 1 (below 2^24 strata the product y0 + u = nstrat times 1 / nstrat
                                 // rounds to 1 at most), so iy <= ninc, and at y = 1 the table's last entry
                                 // has x and dy = 0
-                                const float2 e = a.table_smem ? table[d * W + iy] : __ldg(a.tablef + d * W + iy);
+                                const float2 e = table_smem ? table[d * W + iy] : __ldg(a.tablef + d * W + iy);
                                 float dy = yn - yfl;
-                                if (a.wide && iy >= ax.ninc) dy = 0.f;
+                                if (wide && iy >= ax.ninc) dy = 0.f;
                                 if (NEED_X) x[d] = fmaf(e.y, dy, e.x);
                                 jac *= e.y * ax.Kf;
                                 // the training bin; y = 0 and y = 1 are not counted (pyx:460)
                                 const unsigned int bin = yn > 0.f ? (unsigned int)iy : (unsigned int)ax.ninc;
                                 if (d & 1) bins[d >> 1] |= bin << 16;
                                 else bins[d >> 1] = bin;
-                                if (MODE == MODE_POINTS && a.y_out) ((float *)a.y_out)[ig * dim + d] = yd;
+                                if (MODE == MODE_POINTS && a.y_out) ((float *)a.y_out)[(size_t)ig * dim + d] = yd;
                             }
                         }
                     } else {
                         jac = __ldg((const float *)a.keep_jac + ig);
                         if (a.train) {
-                            const uint2 *src = reinterpret_cast<const uint2 *>(a.keep_bins + ig * a.keep_bstride);
+                            const uint2 *src = reinterpret_cast<const uint2 *>(a.keep_bins + (size_t)ig * a.keep_bstride);
 #pragma unroll
                             for (int g = 0; 4 * g < DIMB; g++) {
                                 if (4 * g >= dim) break;
@@ -508,8 +540,8 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
                     // weight, pyx:1748-1749: jac *= dv_y / neval_hcube
                     const float wg = jac * win_w[cur];
                     if (MODE == MODE_POINTS) {
-                        float *xo = (float *)a.x_out + ig * dim;
-                        if (DIMB >= 4 && a.x_vec) {   // dim a multiple of 4, 16-byte aligned rows
+                        float *xo = (float *)a.x_out + (size_t)ig * dim;
+                        if (DIMB % 4 == 0 && a.x_vec) {   // dim a multiple of 4, 16-byte aligned rows
 #pragma unroll
                             for (int g = 0; 4 * g < DIMB; g++)
                                 if (4 * g < dim)
@@ -524,7 +556,7 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
                         if (a.hc_out) a.hc_out[ig] = h + cur;
                         if (a.keep_jac) {
                             ((float *)a.keep_jac)[ig] = jac;
-                            uint2 *dst = reinterpret_cast<uint2 *>(a.keep_bins + ig * a.keep_bstride);
+                            uint2 *dst = reinterpret_cast<uint2 *>(a.keep_bins + (size_t)ig * a.keep_bstride);
 #pragma unroll
                             for (int g = 0; 4 * g < DIMB; g++)
                                 if (4 * g < dim) dst[g] = make_uint2(bins[2 * g], bins[2 * g + 1]);
@@ -547,7 +579,7 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
                                 for (int d = 0; d < DIMB; d++) {
                                     if (d >= dim) break;
                                     const unsigned int bin = (d & 1) ? bins[d >> 1] >> 16 : bins[d >> 1] & 0xffffu;
-                                    if (a.hist_smem) {
+                                    if (!GENERAL || a.hist_smem) {
                                         atomicAdd(my_hsum + d * W + bin, fd);
                                         atomicAdd(hcnt + d * W + bin, 1u);
                                     } else if (bin < (unsigned int)a.ax[d].ninc) {
@@ -562,6 +594,7 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
                 if (NEED_RED) wb.wf[li] = wf;
             }
             __syncwarp();
+            if (b == s0) cut_first = cut0 = wb.off[0] < 0;
             const bool ended = wb.off[nw] == len;   // the chunk's last hypercube ends with it
             const int nfin = ended ? nw : nw - 1;
             if (NEED_RED) {
@@ -629,7 +662,7 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
                     const int o = wb.off[k], oe = wb.off[k + 1];
                     const float ck = o < 0 ? c_open : wb.wf[o];
                     if (k == 0 && cut0)
-                        put_record(rec, h, (int)(b + oe - s0), ck, q, 0);
+                        rec[0] = RangeRec{h, (int)(b + oe - s0), ck, q.dh, q.dl, q.qh, q.ql};
                     else
                         finish_hcube(a, h + k, oe - o, ck, q, o < 0 ? nullptr : wb.wf + o, beta_half_f, sums);
                 }
@@ -637,15 +670,17 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
                 v_open = v_next;
                 c_open = c_next;
                 open = !ended;
+                n_open = len - wb.off[nw - 1];
             }
             h += nfin;
             __syncwarp();
         }
         if (NEED_RED && lane == 0) {   // records of the hypercubes cut by the range
             const bool spans = open && cut0;
-            if (spans) put_record(rec, h, (int)(s1 - s0), c_open, v_open, 1);
+            const DQ &v = v_open;
+            if (spans) rec[0] = RangeRec{h, -(int)(s1 - s0), c_open, v.dh, v.dl, v.qh, v.ql};
             else if (!cut_first) rec[0].h = -1;
-            if (open && !spans) put_record(rec + 1, h, (int)(s1 - a.offsets[h]), c_open, v_open, 0);
+            if (open && !spans) rec[1] = RangeRec{h, n_open, c_open, v.dh, v.dl, v.qh, v.ql};
             else rec[1].h = -1;
         }
     }
@@ -654,38 +689,40 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
     if (NEED_RED) {
         if (nan_local) atomicExch((int *)&a.stats->nan_seen, 1);
         float r6[6] = {sums.mh, sums.ml, sums.vh, sums.vl, sums.sh, sums.sl};
-        if (!DEAL) {
+        if (!deal) {
             __syncthreads();
             if (warp % GROUP == 0 && nu > 0) {   // lane l joins the pieces of the l-th warp's range with those before it
                 RangeRec H, T;
                 H.h = T.h = -1;
-                if (lane < nu) {
+                if (lane < (int)nu) {
                     H = s_rec[2 * (warp + lane)];
                     T = s_rec[2 * (warp + lane) + 1];
                 }
                 Piece cur = {0.f, 0.f, 0.f, 0.f, 0.f}, end = cur;
-                if (H.h >= 0) (H.spans ? cur : end) = Piece{(float)H.n, H.sh, H.sl, H.qh, H.ql};
-                if (T.h >= 0) cur = Piece{(float)T.n, T.sh, T.sl, T.qh, T.ql};
-                const bool inside = scan_pieces(cur, !(H.h >= 0 && H.spans));
+                const bool h_spans = H.h >= 0 && H.n < 0, h_ends = H.h >= 0 && H.n > 0;
+                if (h_spans) cur.from(H);
+                if (h_ends) end.from(H);
+                if (T.h >= 0) cur.from(T);
+                const bool inside = scan_pieces(cur, !h_spans);
                 const Piece prev = cur.up(1);
                 const bool prev_inside = __shfl_up_sync(0xffffffffu, (int)inside, 1) && lane > 0;
-                if (H.h >= 0 && !H.spans) {   // a hypercube begun earlier ends in this lane's range
+                if (h_ends) {   // a hypercube begun earlier ends in this lane's range
                     if (lane > 0) end.put_first(prev);
                     if (prev_inside) finish_cut(a, H.h, end, r6);
-                    else a.rrecs[2 * seg] = RangeRec{H.h, (int)end.n, 0, end.sh, end.sl, end.qh, end.ql};
+                    else a.rrecs[2 * (size_t)seg] = end.record(H.h, false);
                 }
-                const unsigned int wrote = __ballot_sync(0xffffffffu, H.h >= 0 && !H.spans && !prev_inside);
-                if (lane == nu - 1) {   // what is open at the end of the CTA's range
-                    const bool spans = H.h >= 0 && H.spans && !inside;
-                    const RangeRec o = {T.h >= 0 ? T.h : H.h, (int)cur.n, spans ? 1 : 0, cur.sh, cur.sl, cur.qh, cur.ql};
-                    if (spans) a.rrecs[2 * seg] = o;
-                    else if (!wrote) a.rrecs[2 * seg].h = -1;
-                    if (!spans && (T.h >= 0 || (H.h >= 0 && H.spans))) a.rrecs[2 * seg + 1] = o;
-                    else a.rrecs[2 * seg + 1].h = -1;
+                const unsigned int wrote = __ballot_sync(0xffffffffu, h_ends && !prev_inside);
+                if (lane == (int)nu - 1) {   // what is open at the end of the CTA's range
+                    const bool spans = h_spans && !inside;
+                    const RangeRec o = cur.record(T.h >= 0 ? T.h : H.h, spans);
+                    if (spans) a.rrecs[2 * (size_t)seg] = o;
+                    else if (!wrote) a.rrecs[2 * (size_t)seg].h = -1;
+                    if (!spans && (T.h >= 0 || h_spans)) a.rrecs[2 * (size_t)seg + 1] = o;
+                    else a.rrecs[2 * (size_t)seg + 1].h = -1;
                 }
             }
         }
-        ff_block_reduce6<NTB>(r6, red);   // a fixed order; its barriers also end the histogram
+        ff_block_reduce6(r6, red);   // a fixed order; its barriers also end the histogram
         if (tid == 0) {
             TilePart p;
             p.mean = VgKSum{ff_pack(r6[0], r6[1]), 0.0};
@@ -709,14 +746,6 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
     }
 }
 
-template <int MODE, int KIND, int DIMB, int NTB>
-__global__ void __launch_bounds__(NTB, 1) range_kernel(const __grid_constant__ IterArgs a,
-                                                       const __grid_constant__ VgParams prm)
-{
-    extern __shared__ __align__(16) unsigned char smem[];
-    range_body<MODE, KIND, DIMB, NTB, false>(a, prm, smem, blockIdx.x, gridDim.x);
-}
-
 // ---------------------------------------------------------------- finalize
 // The iteration's sums by one CTA: the partial sums of the ncta reduction CTAs
 // (ngroups groups of warps) and the hypercubes cut by the ends of their ranges (or of the dealt units).
@@ -724,14 +753,13 @@ __global__ void __launch_bounds__(NTB, 1) range_kernel(const __grid_constant__ I
 // the other; a segmented scan joins those of a hypercube that goes on through
 // several threads' records, so the time follows the logarithm of its length.
 // Sums in a fixed order; valid in thread 0.
-template <int NTB>
-__device__ __forceinline__ void finalize_ranges(const IterArgs &a, int ncta, int64_t ngroups, bool deal,
+__device__ __forceinline__ void finalize_ranges(const IterArgs &a, int ncta, int64_t ngroups, int deal,
                                                 float (&s6)[6])
 {
-    constexpr int NW = NTB / 32;
-    __shared__ Piece s_last[NW];
-    __shared__ int s_head[NW];
-    __shared__ float s_red[6 * NW];
+    __shared__ Piece s_last[32];
+    __shared__ int s_head[32];
+    __shared__ float s_red[6 * 32];
+    const int NTB = (int)blockDim.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const vg_stats *st = a.stats;
     const int64_t R = st->ntiles ? record_count(st->neval, ngroups, deal) : 0;
@@ -756,10 +784,11 @@ __device__ __forceinline__ void finalize_ranges(const IterArgs &a, int ncta, int
     for (int64_t t = t0; t < t1; t++) {
         const RangeRec H = a.rrecs[2 * t], T = a.rrecs[2 * t + 1];
         if (H.h >= 0) {
-            Piece p = {(float)H.n, H.sh, H.sl, H.qh, H.ql};
+            Piece p;
+            p.from(H);
             p.put_first(cur);
             cur = p;
-            if (!H.spans) {
+            if (H.n > 0) {
                 if (started) {
                     finish_cut(a, H.h, cur, s6);
                 } else {
@@ -773,7 +802,7 @@ __device__ __forceinline__ void finalize_ranges(const IterArgs &a, int ncta, int
             started = true;   // nothing comes in from before
         }
         if (T.h >= 0) {
-            cur = Piece{(float)T.n, T.sh, T.sl, T.qh, T.ql};
+            cur.from(T);
             started = true;
         }
     }
@@ -796,31 +825,35 @@ __device__ __forceinline__ void finalize_ranges(const IterArgs &a, int ncta, int
         first.put_first(prev);
         finish_cut(a, hfirst, first, s6);
     }
-    ff_block_reduce6<NTB>(s6, s_red);
+    ff_block_reduce6(s6, s_red);
 }
 
+// ---------------------------------------------------------------- launcher
 // Threads per CTA (one CTA per SM) by dimension: as many as the registers of
 // one sample's coordinates leave.
-template <int DIMB>
-constexpr int range_threads()
+__host__ __device__ constexpr int range_threads(int dimb) { return dimb <= 8 ? 1024 : (dimb <= 16 ? 768 : 256); }
+
+template <int MODE, int KIND, int DIMB, int F>
+__global__ void __launch_bounds__(range_threads(DIMB), 1)
+range_kernel(const __grid_constant__ IterArgs a, const __grid_constant__ VgParams prm)
 {
-    return DIMB <= 8 ? 1024 : (DIMB <= 16 ? 768 : 256);
+    extern __shared__ __align__(16) unsigned char smem[];
+    range_body<MODE, KIND, DIMB, F>(a, prm, smem, blockIdx.x, gridDim.x, 0);
 }
 
 // Shared memory of a CTA: the histogram comes first (its copies spread the
 // lanes' colliding float adds, which are compare-and-swap loops: 53 cycles
 // per warp-wide add on 50 bins, 15 on 1000), then the grid table, then up to 8
 // copies of the histogram.
-template <int NTB>
-inline RangePlan range_fit(int dim, int maxK, int tab_len, int train, int want_table, size_t budget, int *table_smem,
-                           int *hist_copies)
+inline RangePlan range_fit(int ntb, int dim, int maxK, int tab_len, int train, int want_table, size_t budget,
+                           int *table_smem, int *hist_copies)
 {
     int hc = train ? 1 : 0, tb = want_table ? 1 : 0;
-    RangePlan p = range_plan<NTB>(dim, maxK, tb, hc, tab_len);
-    if (p.total > budget && tb) p = range_plan<NTB>(dim, maxK, tb = 0, hc, tab_len);
-    if (p.total > budget && hc) p = range_plan<NTB>(dim, maxK, tb, hc = 0, tab_len);
+    RangePlan p = range_plan(ntb, dim, maxK, tb, hc, tab_len);
+    if (p.total > budget && tb) p = range_plan(ntb, dim, maxK, tb = 0, hc, tab_len);
+    if (p.total > budget && hc) p = range_plan(ntb, dim, maxK, tb, hc = 0, tab_len);
     while (hc > 0 && hc < 8) {
-        const RangePlan q = range_plan<NTB>(dim, maxK, tb, 2 * hc, tab_len);
+        const RangePlan q = range_plan(ntb, dim, maxK, tb, 2 * hc, tab_len);
         if (q.total > budget) break;
         hc *= 2;
         p = q;
@@ -830,18 +863,18 @@ inline RangePlan range_fit(int dim, int maxK, int tab_len, int train, int want_t
     return p;
 }
 
-template <int MODE, int KIND, int DIMB>
-int launch_range(IterArgs &a, const VgParams *prm, int tab_len, cudaStream_t st)
+constexpr size_t RANGE_SMEM = 220 * 1024;
+
+template <int MODE, int KIND, int DIMB, int F>
+int launch_range_as(IterArgs &a, const VgParams *prm, size_t smem, cudaStream_t st)
 {
-    constexpr int NTB = range_threads<DIMB>();
-    constexpr int NEED_RED = (MODE == MODE_REDUCE || MODE == MODE_FUSED || MODE == MODE_REDUCE_KEPT);
-    a.tab_len = tab_len;
-    const int train = NEED_RED && a.train && g_tile_hist != 0;
-    const int table = MODE != MODE_REDUCE_KEPT && g_tile_table != 0;
-    const RangePlan p = range_fit<NTB>(a.dim, a.maxK, tab_len, train, table, 220 * 1024, &a.table_smem, &a.hist_smem);
-    if (p.total > 220 * 1024) return vg_fail(VG_ERR_UNSUPPORTED, "shared memory plan too large");
-    auto kern = range_kernel<MODE, KIND, DIMB, NTB>;
-    VG_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.total));
+    constexpr int NTB = range_threads(DIMB);
+    auto kern = range_kernel<MODE, KIND, DIMB, F>;
+    static bool attr = false;   // once per kernel: always the largest
+    if (!attr) {
+        VG_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RANGE_SMEM));
+        attr = true;
+    }
     // one CTA per SM, fewer where there are fewer chunks
     int64_t grid = vg_num_sms();
     const int64_t chunks = (a.ncap + CHUNK - 1) / CHUNK;
@@ -850,9 +883,47 @@ int launch_range(IterArgs &a, const VgParams *prm, int tab_len, cudaStream_t st)
     a.ncta = (int)grid;
     a.ngroups = grid * (NTB / 32 / GROUP);
     static const VgParams empty = {};
-    kern<<<(unsigned)grid, NTB, p.total, st>>>(a, prm ? *prm : empty);
+    kern<<<(unsigned)grid, NTB, smem, st>>>(a, prm ? *prm : empty);
     VG_LAUNCH_CHECK();
     return VG_OK;
+}
+
+// The body for this iteration: by exact dimension to 8, where most of the work
+// of low-dimensional integrals is per axis; above that by the run-time one.
+template <int MODE, int KIND>
+int launch_range(IterArgs &a, const VgParams *prm, int tab_len, cudaStream_t st)
+{
+    constexpr bool NEED_RED = (MODE == MODE_REDUCE || MODE == MODE_FUSED || MODE == MODE_REDUCE_KEPT);
+    constexpr bool NEED_MAP = MODE != MODE_REDUCE_KEPT;
+    constexpr int T = RF_TABLE, ET = RF_EXACT | RF_TABLE, G = RF_GENERAL;
+    a.tab_len = tab_len;
+    const int train = NEED_RED && a.train && g_tile_hist != 0;
+    const RangePlan p = range_fit(range_threads(a.dim), a.dim, a.maxK, tab_len, train, NEED_MAP && g_tile_table != 0,
+                                  RANGE_SMEM, &a.table_smem, &a.hist_smem);
+    if (p.total > RANGE_SMEM) return vg_fail(VG_ERR_UNSUPPORTED, "shared memory plan too large");
+    if ((!NEED_MAP || a.u == nullptr) && !a.wide && (!NEED_RED || !a.train || a.hist_smem)) {
+        if (!NEED_MAP || a.table_smem) {
+            switch (a.dim) {
+            case 1: return launch_range_as<MODE, KIND, 1, ET>(a, prm, p.total, st);
+            case 2: return launch_range_as<MODE, KIND, 2, ET>(a, prm, p.total, st);
+            case 3: return launch_range_as<MODE, KIND, 3, ET>(a, prm, p.total, st);
+            case 4: return launch_range_as<MODE, KIND, 4, ET>(a, prm, p.total, st);
+            case 5: return launch_range_as<MODE, KIND, 5, ET>(a, prm, p.total, st);
+            case 6: return launch_range_as<MODE, KIND, 6, ET>(a, prm, p.total, st);
+            case 7: return launch_range_as<MODE, KIND, 7, ET>(a, prm, p.total, st);
+            case 8: return launch_range_as<MODE, KIND, 8, ET>(a, prm, p.total, st);
+            }
+            if (a.dim <= 16) return launch_range_as<MODE, KIND, 16, T>(a, prm, p.total, st);
+        }
+        if constexpr (NEED_MAP)
+            if (a.dim > 8 && a.dim <= 16) return launch_range_as<MODE, KIND, 16, 0>(a, prm, p.total, st);
+    }
+    // (64 takes every dimension: the reduction of kept samples has little per axis)
+    if constexpr (NEED_MAP) {
+        if (a.dim <= 8) return launch_range_as<MODE, KIND, 8, G>(a, prm, p.total, st);
+        if (a.dim <= 16) return launch_range_as<MODE, KIND, 16, G>(a, prm, p.total, st);
+    }
+    return launch_range_as<MODE, KIND, 64, G>(a, prm, p.total, st);
 }
 
 }  // namespace vg

@@ -51,12 +51,13 @@ struct TileRec {
     int32_t pad;
 };
 
-// FP32: the same of a hypercube cut by the end of a range (n samples,
-// their sum and their squared deviations about their mean in float-float).
+// FP32: a piece of a hypercube cut by the end of a range: n samples (-n where it
+// also continues past the range), the sums D of wf - c and Q of their squares in
+// float-float; with c = NaN, D is the sum of wf and Q that about the mean.
 struct __align__(16) RangeRec {
-    int64_t h;
-    int32_t n, spans;
-    float sh, sl, qh, ql;
+    int64_t h;       // hypercube, -1 if the slot is empty
+    int32_t n;
+    float c, dh, dl, qh, ql;
 };
 
 struct TilePart {
@@ -101,7 +102,7 @@ struct IterArgs {
     TilePart *parts;
     int64_t ntiles_cap;       // in BASE_TILE units
     AxisArgs ax[VG_MAX_DIM];  // FP32: what a sample needs of each axis
-    int wide;                 // FP32: 2^31 hypercubes or more, or 2^24 strata on an axis
+    int wide;                 // FP32: 2^31 hypercubes or samples or more, or 2^24 strata on an axis
     int x_vec;                // MODE_POINTS: rows of x are 16-byte aligned multiples of 16 bytes
     int64_t neval;
     double neval_frac;
@@ -165,10 +166,9 @@ __host__ __device__ inline SmemPlan smem_plan(int dim, int maxK, int Ttile, int 
 
 // Block-wide exclusive prefix sum of one int64 per thread (warp shuffles,
 // then a scan of the warp totals); *total = the block's sum.
-template <int NTB>
-__device__ __forceinline__ int64_t block_excl_scan(int64_t v, int64_t *wtot /* NTB/32 */, int64_t *total)
+__device__ __forceinline__ int64_t block_excl_scan(int64_t v, int64_t *wtot /* one per warp */, int64_t *total)
 {
-    constexpr int NW = NTB / 32;
+    const int NW = (int)blockDim.x >> 5;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int64_t x = v;
 #pragma unroll
@@ -194,10 +194,9 @@ __device__ __forceinline__ int64_t block_excl_scan(int64_t v, int64_t *wtot /* N
     return r;
 }
 
-template <int NTB>
-__device__ __forceinline__ int64_t block_max(int64_t v, int64_t *wtot /* NTB/32 */)
+__device__ __forceinline__ int64_t block_max(int64_t v, int64_t *wtot /* one per warp */)
 {
-    constexpr int NW = NTB / 32;
+    const int NW = (int)blockDim.x >> 5;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
@@ -296,10 +295,9 @@ __device__ __forceinline__ void ff_unpack(double d, float &h, float &l)
 }
 
 // Block-wide float-float reduction of six floats (three float-float values)
-// in a fixed order; the result is valid in thread 0.  scratch: 6 * NTB/32
-// floats of shared memory.
-template <int NTB>
-__device__ __forceinline__ void ff_block_reduce6(float (&r6)[6], float *scratch)
+// in a fixed order; the result is valid in thread 0.  scratch: 6 floats per
+// warp of shared memory.
+__device__ __forceinline__ void ff_warp_reduce6(float (&r6)[6])
 {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
@@ -309,27 +307,23 @@ __device__ __forceinline__ void ff_block_reduce6(float (&r6)[6], float *scratch)
 #pragma unroll
         for (int i = 0; i < 6; i += 2) ff_add_pair(r6[i], r6[i + 1], o6[i], o6[i + 1]);
     }
-    if (NTB > 32) {
-        const int tid = threadIdx.x;
-        if ((tid & 31) == 0) {
+}
+
+__device__ __forceinline__ void ff_block_reduce6(float (&r6)[6], float *scratch)
+{
+    const int tid = threadIdx.x;
+    ff_warp_reduce6(r6);
+    if ((tid & 31) == 0) {
 #pragma unroll
-            for (int i = 0; i < 6; i++) scratch[(tid >> 5) * 6 + i] = r6[i];
-        }
-        __syncthreads();
-        if (tid < 32) {
-#pragma unroll
-            for (int i = 0; i < 6; i++) r6[i] = tid < NTB / 32 ? scratch[tid * 6 + i] : 0.f;
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                float o6[6];
-#pragma unroll
-                for (int i = 0; i < 6; i++) o6[i] = __shfl_down_sync(0xffffffffu, r6[i], off);
-#pragma unroll
-                for (int i = 0; i < 6; i += 2) ff_add_pair(r6[i], r6[i + 1], o6[i], o6[i + 1]);
-            }
-        }
-        __syncthreads();
+        for (int i = 0; i < 6; i++) scratch[(tid >> 5) * 6 + i] = r6[i];
     }
+    __syncthreads();
+    if (tid < 32) {
+#pragma unroll
+        for (int i = 0; i < 6; i++) r6[i] = tid < (int)blockDim.x >> 5 ? scratch[tid * 6 + i] : 0.f;
+        ff_warp_reduce6(r6);
+    }
+    __syncthreads();
 }
 
 // (h, l) = (ah, al) * b in float-float (the head's product error by fma).
