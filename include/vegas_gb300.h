@@ -230,14 +230,18 @@ int vg_end_iteration(const vg_integrator *it, void *stream);
 /*
  * One full iteration for a built-in integrand (pyx:2086-2217: allocation,
  * the fused batch loop, the iteration sums, the map adapt) in one call:
- * vg_allocate + vg_fused_iteration + vg_end_iteration, with the adapt on a
- * forked stream concurrently with the finalize when adapt_to_errors is off
- * (the adapt needs only the tile kernel's training histogram); joined back
- * into `stream` before returning.  Call it once outside any stream capture
- * before capturing it (the first call on a device creates the forked stream).
+ * vg_allocate + vg_fused_iteration + vg_end_iteration, the finalize and the
+ * adapt in one kernel when adapt_to_errors is off (the adapt needs only the
+ * training histogram).
  */
 int vg_iterate(const vg_integrator *it, uint32_t itn, int kind, const double *params, int nparams,
                void *stream);
+
+/* vg_iterate, whose last kernel also writes the iteration's record to rec:
+ * memory that the device can write (pinned host memory, read after the stream
+ * or an event on it was waited for), or NULL. */
+int vg_iterate_record(const vg_integrator *it, uint32_t itn, int kind, const double *params, int nparams,
+                      vg_stats *rec, void *stream);
 
 /*
  * One vegas+ iteration (allocation, fused evaluation + reduction, adapt) for

@@ -4,6 +4,8 @@
 // The adapt kernel runs it with 1024 threads per axis, the batched kernel with
 // the threads of its CTA.
 #pragma once
+#include <cooperative_groups.h>
+
 #include "vg_common.cuh"
 
 namespace vgadapt {
@@ -139,6 +141,25 @@ __device__ float block_reduce_f(float v, float *f, int red_nt)
     return r;
 }
 
+// FP32 mode: the normalised, damped weight of a smoothed average sf; rmx the
+// reciprocal of the largest one, sp the sum of all times rmx.
+__device__ __forceinline__ double damped_weight_fast(float sf, float rmx, float sp, double alpha)
+{
+    const float rs = sp > 0.f ? 1.f / sp : 0.f;
+    const float vf = sf * rmx * rs;
+    double v;
+    if (sp > 0.f && vf >= 1.17549435e-38f && vf < 0.99999f) {
+        const float one_m = 1.f - vf;
+        const float lnv = one_m < 0.25f ? log1pf(-one_m) : vg_lg2_approx(vf) * 0.69314718f;
+        const float q = one_m / (-lnv);
+        v = (double)vg_ex2_approx((float)alpha * vg_lg2_approx(q));
+    } else {
+        v = sp > 0.f ? (double)sf * (double)rmx * (double)rs + VG_TINY : VG_TINY;
+        if (v > 0 && v <= 0.99999999) v = damp_fast(v, alpha);
+    }
+    return v;
+}
+
 // FP32 mode, alpha > 0 with training data: the weights of one axis (average,
 // 3-tap smoothing, normalisation, damping; pyx:539-562) in FP32 on the MUFU,
 // written to avg[] as doubles.  The FP32 sum is formed by SUM_NT threads, so that
@@ -179,21 +200,8 @@ __device__ void adapt_weights_fast(const AdaptArgs &a, int d, int K, double *avg
     if (t < sum_nt)
         for (int i = t; i < K; i += sum_nt) sp += sf[i] * rmx;
     sp = block_reduce_f<false>(sp, pf, sum_nt);
-    const float rs = sp > 0.f ? 1.f / sp : 0.f;
-    const float alf = (float)a.alpha;
     for (int i = t; i < K; i += NT) {
-        const float vf = sf[i] * rmx * rs;
-        double v;
-        if (sp > 0.f && vf >= 1.17549435e-38f && vf < 0.99999f) {
-            const float one_m = 1.f - vf;
-            const float lnv = one_m < 0.25f ? log1pf(-one_m) : vg_lg2_approx(vf) * 0.69314718f;
-            const float q = one_m / (-lnv);
-            v = (double)vg_ex2_approx(alf * vg_lg2_approx(q));
-        } else {
-            v = sp > 0.f ? (double)sf[i] * (double)rmx * (double)rs + VG_TINY : VG_TINY;
-            if (v > 0 && v <= 0.99999999) v = damp_fast(v, a.alpha);
-        }
-        avg[i] = v;
+        avg[i] = damped_weight_fast(sf[i], rmx, sp, a.alpha);
     }
     __syncthreads();
 }
@@ -307,5 +315,155 @@ __device__ void adapt_axis(const AdaptArgs &a, int d, double *avg, double *tmp, 
     __syncthreads();
 }
 
+// ----------------------------------------------------------- cluster form
+// The same for one axis by a cluster of CLUSTER CTAs of CLUSTER_NT threads, in
+// place: thread t of CTA c has increment and node i = c * CLUSTER_NT + t, and
+// cluster memory holds what the others need.  For alpha > 0 with training data
+// and at most CLUSTER * CLUSTER_NT - 1 increments.  The sums are formed in the
+// order of adapt_axis with 1024 threads, so the results are the same bits.
+constexpr int CLUSTER = 8, CLUSTER_NT = 128;
+constexpr int CLUSTER_MAX = CLUSTER * CLUSTER_NT - 1;
+
+struct ClusterSmem {
+    double P[CLUSTER * CLUSTER_NT];         // cumulative weights of the whole axis
+    double gs[CLUSTER * CLUSTER_NT], is[CLUSTER * CLUSTER_NT];   // its old nodes and increments
+    double avg[CLUSTER_NT];                 // this CTA's weights
+    double node[CLUSTER_NT];                // its new nodes
+    double near[CLUSTER_NT + 2];            // its averages and the neighbours'
+    double wtot[CLUSTER_NT / 32], wsum[CLUSTER_NT / 32];
+    float wmax[CLUSTER_NT / 32], wsumf[CLUSTER_NT / 32];
+};
+
+static __device__ __forceinline__ void adapt_axis_cluster(const AdaptArgs &a, int d)
+{
+    namespace cg = cooperative_groups;
+    __shared__ ClusterSmem s;
+    constexpr int NW = CLUSTER_NT / 32;
+    cg::cluster_group cl = cg::this_cluster();
+    const int c = (int)cl.block_rank(), t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int i = c * CLUSTER_NT + t, gw = c * NW + w;
+    const int K = a.old_ninc[d];
+    double *gd = a.new_grid + d * a.ldg;   // the grid itself
+    double *id = a.new_inc + d * a.ldi;
+    double *sum_f = const_cast<double *>(a.sum_f) + d * a.ldi;
+    unsigned long long *n_f = const_cast<unsigned long long *>(a.n_f) + d * a.ldi;
+    for (int j = t; j <= K; j += CLUSTER_NT) {
+        s.gs[j] = gd[j];
+        if (j < K) s.is[j] = id[j];
+    }
+    auto average = [&](int j) -> double {   // pyx:539-547
+        if (j < 0 || j >= K) return 0.0;
+        const unsigned long long n = n_f[j];
+        if (a.fast) return n ? (double)(float)div_fast(sum_f[j], (double)n) : 0.0;
+        return __ddiv_rn(sum_f[j], __dadd_rn((double)n, VG_TINY));
+    };
+    s.near[t + 1] = average(i);
+    if (t == 0) s.near[0] = average(i - 1);
+    if (t == CLUSTER_NT - 1) s.near[CLUSTER_NT + 1] = average(i + 1);
+    __syncthreads();
+    const double am = s.near[t], a0 = s.near[t + 1], ap = s.near[t + 2];
+    double v = 0.0;   // the weight
+    if (a.fast) {
+        // adapt_weights_fast: smoothing, normalisation and damping in FP32
+        float sf = 0.f;
+        if (i < K) {
+            if (i == 0) sf = fmaf(7.f, (float)a0, (float)ap);
+            else if (i == K - 1) sf = fmaf(7.f, (float)a0, (float)am);
+            else sf = fmaf(6.f, (float)a0, (float)am + (float)ap);
+            sf = fabsf(sf) * 0.125f;
+        }
+        float mx = sf;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+        if (lane == 0) s.wmax[w] = mx;
+        cl.sync();   // also: every CTA has read its averages and staged the axis
+        mx = cl.map_shared_rank(s.wmax, lane / NW)[lane % NW];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+        const float rmx = mx > 0.f ? 1.f / mx : 0.f;
+        float sp = 0.f;
+        if (i < K) sp += sf * rmx;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) sp = sp + __shfl_xor_sync(0xffffffffu, sp, off);
+        if (lane == 0) s.wsumf[w] = sp;
+        cl.sync();
+        sp = cl.map_shared_rank(s.wsumf, lane / NW)[lane % NW];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) sp = sp + __shfl_xor_sync(0xffffffffu, sp, off);
+        if (i < K) v = damped_weight_fast(sf, rmx, sp, a.alpha);
+    } else {
+        double sm = 0.0;
+        if (i < K) {
+            if (i == 0) sm = __dadd_rn(__dmul_rn(7., a0), ap);
+            else if (i == K - 1) sm = __dadd_rn(__dmul_rn(7., a0), am);
+            else sm = __dadd_rn(__dadd_rn(__dmul_rn(6., a0), am), ap);
+            sm = __dmul_rn(fabs(sm), 0.125);
+        }
+        double z = sm;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) z = __dadd_rn(z, __shfl_xor_sync(0xffffffffu, z, off));
+        if (lane == 0) s.wsum[w] = z;
+        cl.sync();   // also: every CTA has read its averages and staged the axis
+        z = cl.map_shared_rank(s.wsum, lane / NW)[lane % NW];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) z = __dadd_rn(z, __shfl_xor_sync(0xffffffffu, z, off));
+        if (i < K) {   // normalise + damp, pyx:554-562
+            v = (z > 0) ? __dadd_rn(__ddiv_rn(sm, z), VG_TINY) : VG_TINY;
+            if (v > 0 && v <= 0.99999999) v = pow(__ddiv_rn(-(1 - v), log(v)), a.alpha);
+        }
+    }
+    if (i < K) {
+        sum_f[i] = 0.0;
+        n_f[i] = 0ull;
+    }
+    // cumulative weights of the whole axis, into every CTA
+    s.avg[t] = v;
+    double x = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const double y = __shfl_up_sync(0xffffffffu, x, off);
+        if (lane >= off) x = __dadd_rn(x, y);
+    }
+    if (lane == 31) s.wtot[w] = x;
+    double ex = __shfl_up_sync(0xffffffffu, x, 1);
+    if (lane == 0) ex = 0.0;
+    cl.sync();
+    double z = cl.map_shared_rank(s.wtot, lane / NW)[lane % NW];
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const double y = __shfl_up_sync(0xffffffffu, z, off);
+        if (lane >= off) z = __dadd_rn(z, y);
+    }
+    const double before = __shfl_sync(0xffffffffu, z, gw > 0 ? gw - 1 : 0);
+    const double P = i > 0 ? __dadd_rn(v, gw > 0 ? __dadd_rn(before, ex) : ex) : v;
+    for (int r = 0; r < CLUSTER; r++) cl.map_shared_rank(s.P, r)[i] = P;
+    cl.sync();
+    // regrid, pyx:563-587
+    const double total = s.P[K - 1];
+    const double f_ninc = a.fast ? div_fast(total, (double)K) : __ddiv_rn(total, (double)K);
+    auto node = [&](int n) -> double {
+        if (n == 0) return s.gs[0];
+        if (n >= K) return s.gs[K];
+        const double target = __dmul_rn((double)n, f_ninc);
+        const long long tb = __double_as_longlong(target);
+        int lo = 0, hi = K - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (__double_as_longlong(s.P[mid]) < tb) lo = mid + 1;
+            else hi = mid;
+        }
+        const double acc = __dsub_rn(s.P[lo], target);
+        const double wgt = cl.map_shared_rank(s.avg, lo / CLUSTER_NT)[lo % CLUSTER_NT];
+        const double q = a.fast ? div_fast(acc, wgt) : __ddiv_rn(acc, wgt);
+        return __dsub_rn(s.gs[lo + 1], __dmul_rn(q, s.is[lo]));
+    };
+    const double mine = node(i);
+    s.node[t] = mine;
+    const double last = t == CLUSTER_NT - 1 ? node(i + 1) : 0.0;
+    __syncthreads();
+    if (i <= K) gd[i] = mine;
+    if (i < K) id[i] = __dsub_rn(t == CLUSTER_NT - 1 ? last : s.node[t + 1], mine);
+    cl.sync();   // no CTA ends while another reads its weights
+}
 
 }  // namespace vgadapt

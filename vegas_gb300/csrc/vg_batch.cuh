@@ -233,16 +233,15 @@ static __device__ __noinline__ void cta_finalize_f64(const IterArgs &a, int ngro
         cs = p.sigf;
     }
     for (int64_t t = tid; t < ntiles; t += NT) merge_cut_f64(a, t, ntiles, cm, cv, cs);
-    const VgKSum M = vg_block_ksum<NT>(cm, red);
-    const VgKSum V = vg_block_ksum<NT>(cv, red);
-    const VgKSum Sg = vg_block_ksum<NT>(cs, red);
+    VgKSum v3[3] = {cm, cv, cs};
+    vg_block_ksum3<NT>(v3, red);
     if (tid == 0) {
-        st->mean = M.value();
-        st->var = V.value();
+        st->mean = v3[0].value();
+        st->var = v3[1].value();
         st->sigf_reset = 0;
         *flag = 0;
         if (a.adaptive) {
-            const double ss = Sg.value();
+            const double ss = v3[2].value();
             if (ss > 0) {
                 st->sum_sigf = ss;
             } else {
@@ -362,7 +361,7 @@ __global__ void __launch_bounds__(MAXT, 1) batch_kernel(const BatchJob *__restri
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ IterArgs sa;
     __shared__ int64_t scan[MAXT / 32];
-    __shared__ VgKSum red[MAXT / 32];
+    __shared__ VgKSum red[3 * (MAXT / 32)];
     __shared__ int s_q, s_flag;
     const int tid = threadIdx.x, NTB = (int)blockDim.x;
     const int G = group > 1 ? group : 1;

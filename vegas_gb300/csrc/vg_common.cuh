@@ -218,6 +218,43 @@ __device__ __forceinline__ VgKSum vg_block_ksum(VgKSum v, VgKSum *smem /* NT/32 
     return v;
 }
 
+// The same of three sums at once: their FP64 chains (64 cycles per dependent
+// instruction) run side by side, one warp per sum across the warps.  smem: 3 per
+// warp; all threads get the results.
+template <int NT>
+__device__ __forceinline__ void vg_block_ksum3(VgKSum (&v)[3], VgKSum *smem /* 3 * NT/32, at least 3 */)
+{
+    static_assert(NT >= 96 || NT == 32, "one warp per sum");
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        VgKSum o[3];
+#pragma unroll
+        for (int i = 0; i < 3; i++) o[i] = vg_ksum_shfl_down(v[i], off);
+#pragma unroll
+        for (int i = 0; i < 3; i++) v[i].merge(o[i]);
+    }
+    __syncthreads();
+    if (lane == 0)
+#pragma unroll
+        for (int i = 0; i < 3; i++) smem[i * (NT / 32) + w] = v[i];
+    __syncthreads();
+    if (NT > 32) {
+        if (w < 3) {
+            VgKSum x = lane < NT / 32 ? smem[w * (NT / 32) + lane] : VgKSum{0.0, 0.0};
+#pragma unroll
+            for (int off = (NT / 32 > 16 ? 16 : NT / 32 > 8 ? 8 : NT / 32 > 4 ? 4 : 2); off > 0; off >>= 1)
+                x.merge(vg_ksum_shfl_down(x, off));
+            __syncwarp();
+            if (lane == 0) smem[w * (NT / 32)] = x;
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++) v[i] = smem[i * (NT / 32)];
+    __syncthreads();
+}
+
 // Float-float (double-single) accumulation: (h, l) += x with Knuth's
 // TwoSum (error-free in h, the rounding error carried in l).  The FP32 mode
 // accumulates a thread's few samples this way (about 2^-48 relative, close
@@ -249,6 +286,32 @@ __device__ __forceinline__ double vg_ff_value(float h, float l) { return (double
             return vg_fail(VG_ERR_CUDA, "kernel launch: %s (%s:%d)", cudaGetErrorString(_e), \
                            __FILE__, __LINE__);                                              \
     } while (0)
+
+// Launches of an iteration's chain overlap: a kernel launched with vg_launch_pdl
+// may be placed on the SMs while the one before it on the stream still runs,
+// and calls vg_pdl_wait() before it reads or writes anything that kernel does
+// (the wait is for its end and its writes).  vg_pdl_go() lets the next kernel of
+// the chain be placed; all of this grid's CTAs are running by then, so a CTA
+// waiting on an SM keeps none of them out.
+__device__ __forceinline__ void vg_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void vg_pdl_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+static inline cudaError_t vg_launch_pdl(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+                                        A &&...args)
+{
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kern, static_cast<A &&>(args)...);
+}
 
 static inline int vg_num_sms()
 {

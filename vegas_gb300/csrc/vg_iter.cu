@@ -26,7 +26,7 @@
 #include <math.h>
 #include <string.h>
 
-#include <mutex>
+#include <cooperative_groups.h>
 
 #include "vg_adapt.cuh"
 #include "vg_range.cuh"
@@ -71,7 +71,7 @@ __device__ __forceinline__ void st_release_u64(unsigned long long *p, unsigned l
     asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-__global__ void __launch_bounds__(ALLOC_NT) alloc_kernel(IterArgs a, int64_t nblk, int build_table)
+__global__ void __launch_bounds__(ALLOC_NT) alloc_kernel(const __grid_constant__ IterArgs a, int64_t nblk, int build_table)
 {
     __shared__ int64_t wtot[ALLOC_NT / 32];
     __shared__ double s_nsf;
@@ -80,6 +80,8 @@ __global__ void __launch_bounds__(ALLOC_NT) alloc_kernel(IterArgs a, int64_t nbl
     AllocSync *sy = reinterpret_cast<AllocSync *>(a.alloc_sync);
     unsigned long long *flags = reinterpret_cast<unsigned long long *>(a.bsum);
     const int t = threadIdx.x;
+    vg_pdl_wait();
+    vg_pdl_go();
     if (t == 0) {
         s_b = atomicAdd(&sy->ticket, 1u);
         s_epoch = *(volatile unsigned int *)&sy->epoch;
@@ -230,53 +232,18 @@ __global__ void tablef_kernel(IterArgs a)
 
 // ========================================================== finalize
 // FP64 mode.
-// Stage 1 (one thread per tile, FIN_TILES tiles per block): the tile's
+// Stage 1 (one thread per tile, FIN_NT tiles per block): the tile's
 // partial sums plus, for a tile whose last hypercube continues into later
 // tiles, the Chan et al. merge of that hypercube's partial records; a
 // fixed-order block reduction gives one partial per block.
 // Stage 2 (one block): those partials in block order -> iteration mean, var,
 // sum_sigf (compensated FP64), and the constant-integrand reset.
-constexpr int FIN_TILES = 32;   // one warp per finalize block: few FP64 lanes per value
-
-// Stage 2 body (one block): the stage-1 partials in block order -> the
-// iteration's mean, var, sum_sigf and the constant-integrand reset.
-__device__ __forceinline__ void finalize_totals(const IterArgs &a, int64_t nblk, VgKSum *red, int *reset)
-{
-    VgKSum cm = {0.0, 0.0}, cv = {0.0, 0.0}, cs = {0.0, 0.0};
-    for (int64_t b = threadIdx.x; b < nblk; b += FIN_TILES) {
-        const TilePart p = a.part2[b];
-        cm.merge(p.mean);
-        cv.merge(p.var);
-        cs.merge(p.sigf);
-    }
-    const VgKSum M = vg_block_ksum<FIN_TILES>(cm, red);
-    const VgKSum V = vg_block_ksum<FIN_TILES>(cv, red);
-    const VgKSum Sg = vg_block_ksum<FIN_TILES>(cs, red);
-    if (threadIdx.x == 0) {
-        vg_stats *s = a.stats;
-        s->mean = M.value();
-        s->var = V.value();
-        *reset = 0;
-        s->sigf_reset = 0;
-        if (a.adaptive) {
-            const double ss = Sg.value();
-            if (ss > 0) {
-                s->sum_sigf = ss;
-            } else {   // integrand looks constant: even distribution (pyx:2212-2215)
-                s->sum_sigf = (double)a.H;
-                s->sigf_reset = 1;
-                *reset = 1;
-            }
-        }
-    }
-    __syncthreads();
-    if (*reset)
-        for (int64_t h = threadIdx.x; h < a.H; h += FIN_TILES) a.sigf[h] = 1.0;
-}
+constexpr int FIN_NT = 128;      // threads per finalize block, one tile each (the tail kernel's CTAs)
 
 // The iteration's results from the stats fields (mean, var, sum_sigf) and
 // the constant-integrand reset (pyx:2209-2215); thread 0 has the sums.
-__device__ __forceinline__ void finalize_store(const IterArgs &a, double mean, double var, double ss, int *reset)
+__device__ __forceinline__ void finalize_store(const IterArgs &a, double mean, double var, double ss, int *reset,
+                                               vg_stats *rec)
 {
     if (threadIdx.x == 0) {
         vg_stats *st = a.stats;
@@ -293,6 +260,7 @@ __device__ __forceinline__ void finalize_store(const IterArgs &a, double mean, d
                 *reset = 1;
             }
         }
+        if (rec != nullptr) *rec = *st;   // the caller's copy (pinned host memory)
     }
     __syncthreads();
     if (*reset)
@@ -301,30 +269,37 @@ __device__ __forceinline__ void finalize_store(const IterArgs &a, double mean, d
 
 // FP32 mode: one CTA.
 constexpr int FIN32_NT = 256;
-__global__ void __launch_bounds__(FIN32_NT) finalize32_kernel(const __grid_constant__ IterArgs a)
+__device__ __forceinline__ void finalize32(const IterArgs &a, vg_stats *rec)
 {
     __shared__ int s_reset;
     float s6[6];
     finalize_ranges(a, a.ncta, a.ngroups, 0, s6);
-    finalize_store(a, vg_ff_value(s6[0], s6[1]), vg_ff_value(s6[2], s6[3]), vg_ff_value(s6[4], s6[5]), &s_reset);
+    finalize_store(a, vg_ff_value(s6[0], s6[1]), vg_ff_value(s6[2], s6[3]), vg_ff_value(s6[4], s6[5]), &s_reset, rec);
+}
+
+__global__ void __launch_bounds__(FIN32_NT) finalize32_kernel(const __grid_constant__ IterArgs a, vg_stats *rec)
+{
+    vg_pdl_wait();
+    vg_pdl_go();
+    finalize32(a, rec);
 }
 
 // Stage 1, and stage 2 in the block that finishes last (a counter the
 // allocation resets; the partials are read back in block order, so the
-// result does not depend on which block that is).
-__global__ void __launch_bounds__(FIN_TILES) finalize1_kernel(IterArgs a)
+// result does not depend on which block that is).  Block `block` of `nblocks`.
+__device__ __forceinline__ void finalize64(const IterArgs &a, int block, int nblocks, vg_stats *rec)
 {
-    __shared__ VgKSum red[1];
+    __shared__ VgKSum red[3 * (FIN_NT / 32)];
     __shared__ int s_last, s_reset;
     const vg_stats *st = a.stats;
     const int64_t N = st->neval;
     const int64_t ntiles = st->ntiles ? (N + a.T - 1) / a.T : 0;
     const int64_t nwork = ntiles > a.ncta ? ntiles : a.ncta;
-    const int64_t nblk = (nwork + FIN_TILES - 1) / FIN_TILES;
-    if ((int64_t)blockIdx.x < nblk) {
+    const int64_t nblk = (nwork + FIN_NT - 1) / FIN_NT;
+    if (block < nblk) {
         const double beta_half = a.beta_half;
         VgKSum cm = {0.0, 0.0}, cv = {0.0, 0.0}, cs = {0.0, 0.0};
-        const int64_t t = (int64_t)blockIdx.x * FIN_TILES + threadIdx.x;
+        const int64_t t = (int64_t)block * FIN_NT + threadIdx.x;
         if (t < a.ncta && ntiles > 0) {   // partial sums of the reduction CTA t
             const TilePart p = a.parts[t];
             cm = p.mean;
@@ -362,26 +337,66 @@ __global__ void __launch_bounds__(FIN_TILES) finalize1_kernel(IterArgs a)
                 }
             }
         }
-        const VgKSum M = vg_block_ksum<FIN_TILES>(cm, red);
-        const VgKSum V = vg_block_ksum<FIN_TILES>(cv, red);
-        const VgKSum Sg = vg_block_ksum<FIN_TILES>(cs, red);
+        VgKSum v3[3] = {cm, cv, cs};
+        vg_block_ksum3<FIN_NT>(v3, red);
+        if (nblocks == 1) {   // nothing to wait for
+            finalize_store(a, v3[0].value(), v3[1].value(), v3[2].value(), &s_reset, rec);
+            return;
+        }
         if (threadIdx.x == 0) {
             TilePart p;
-            p.mean = M;
-            p.var = V;
-            p.sigf = Sg;
-            a.part2[blockIdx.x] = p;
+            p.mean = v3[0];
+            p.var = v3[1];
+            p.sigf = v3[2];
+            a.part2[block] = p;
         }
     }
     if (threadIdx.x == 0) {
         __threadfence();
-        s_last = (atomicAdd(a.fin_counter, 1u) == gridDim.x - 1);
+        s_last = (atomicAdd(a.fin_counter, 1u) == (unsigned int)nblocks - 1);
     }
     __syncthreads();
     if (!s_last) return;
     __threadfence();
     if (threadIdx.x == 0) *a.fin_counter = 0u;
-    finalize_totals(a, nblk, red, &s_reset);
+    VgKSum t3[3] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+    for (int64_t b = threadIdx.x; b < nblk; b += FIN_NT) {
+        const TilePart p = a.part2[b];
+        t3[0].merge(p.mean);
+        t3[1].merge(p.var);
+        t3[2].merge(p.sigf);
+    }
+    vg_block_ksum3<FIN_NT>(t3, red);
+    finalize_store(a, t3[0].value(), t3[1].value(), t3[2].value(), &s_reset, rec);
+}
+
+__global__ void __launch_bounds__(FIN_NT) finalize64_kernel(const __grid_constant__ IterArgs a, vg_stats *rec)
+{
+    vg_pdl_wait();
+    vg_pdl_go();
+    finalize64(a, blockIdx.x, gridDim.x, rec);
+}
+
+// The end of an iteration in one launch: the iteration's sums, and the map's
+// adapt, which needs only the training histogram.  A cluster of 8 CTAs per
+// axis adapts, 128 of the axis' increments each: the FP64 work per increment
+// (damping in FP64 mode; the cumulative sum, the search for each new node and
+// its interpolation in both) is spread over 8 SMs, whose FP64 pipes take 19
+// cycles per warp instruction; one CTA of 1024 threads per axis took 53 us
+// in FP64 and 18 us in FP32 at 1000 increments.  The clusters after them
+// finalize (FP32: one CTA; FP64: 128 tiles per CTA).
+__global__ void __cluster_dims__(vgadapt::CLUSTER, 1, 1) __launch_bounds__(FIN_NT)
+tail_kernel(const __grid_constant__ IterArgs a, const __grid_constant__ vgadapt::AdaptArgs ad, int f64, int nfin,
+            vg_stats *rec)
+{
+    vg_pdl_wait();
+    vg_pdl_go();
+    const int b = (int)blockIdx.x - ad.dim * vgadapt::CLUSTER;
+    if (b < 0) vgadapt::adapt_axis_cluster(ad, blockIdx.x / vgadapt::CLUSTER);
+    else if (b < nfin) {
+        if (f64) finalize64(a, b, nfin, rec);
+        else finalize32(a, rec);
+    }
 }
 
 // ================================================================ host
@@ -415,9 +430,10 @@ WorkLayout layout(const vg_integrator *it, int64_t ncap)
     L.bsum = o;    o = align256(o + sizeof(int64_t) * L.nblk);
     L.tile_h0 = o; o = align256(o + sizeof(int64_t) * (L.ntiles_cap + 1));
     L.counter = o; o = align256(o + 16 + sizeof(AllocSync));
-    // FP64: two records per tile of 256 or more samples; FP32: per CTA or dealt unit
+    // FP64: two records per tile of 256 or more samples (or 128); FP32: per group or dealt unit
     const int f64 = it->precision == VG_F64;
-    const int64_t tiles = (ncap + 255) / 256 + 1;
+    const int64_t small = L.ntiles_cap < 1024 ? L.ntiles_cap : 1024;   // tiles of 128 where there are few
+    const int64_t tiles = (ncap + 255) / 256 + 1 > small ? (ncap + 255) / 256 + 1 : small;
     L.part_cap = L.ntiles_cap < MAX_PARTS ? L.ntiles_cap : (int64_t)MAX_PARTS;
     if (L.part_cap < 1024) L.part_cap = 1024;   // the batched launch's groups of CTAs, whatever the integral's size
     const int64_t units = L.ntiles_cap + 1;
@@ -425,7 +441,7 @@ WorkLayout layout(const vg_integrator *it, int64_t ncap)
     const int64_t fin = L.rec_cap > L.part_cap ? L.rec_cap : L.part_cap;
     L.recs = o;    o = align256(o + (f64 ? sizeof(TileRec) : sizeof(RangeRec)) * 2 * L.rec_cap);
     L.parts = o;   o = align256(o + sizeof(TilePart) * L.part_cap);
-    L.part2 = o;   o = align256(o + sizeof(TilePart) * (fin / FIN_TILES + 2));
+    L.part2 = o;   o = align256(o + sizeof(TilePart) * (fin / FIN_NT + 2));
     L.feval = o;   o = align256(o + sizeof(float) * ncap);
     L.ncap = ncap;
     L.newgrid = o; o = align256(o + sizeof(double) * it->dim * it->ldg);
@@ -519,18 +535,18 @@ int fill_args(IterArgs &a, const vg_integrator *it, uint32_t itn, const double *
 }  // namespace
 
 namespace vg {
-int finalize_launch(IterArgs &a, cudaStream_t st, int fast)
+// CTAs of the FP64 finalize: the tiles of the launched kernel, bounded by the capacity.
+static int64_t finalize_blocks(const IterArgs &a)
 {
-    if (fast) {
-        finalize32_kernel<<<1, FIN32_NT, 0, st>>>(a);
-    } else {
-        // tiles of the launched kernel, bounded by the capacity
-        const int64_t tcap = (a.ncap + a.T - 1) / a.T;
-        const int64_t nwork = tcap > a.ncta ? tcap : a.ncta;
-        const int64_t nblk = (nwork + FIN_TILES - 1) / FIN_TILES;
-        finalize1_kernel<<<(unsigned)nblk, FIN_TILES, 0, st>>>(a);
-    }
-    VG_LAUNCH_CHECK();
+    const int64_t tcap = (a.ncap + a.T - 1) / a.T;
+    const int64_t nwork = tcap > a.ncta ? tcap : a.ncta;
+    return (nwork + FIN_NT - 1) / FIN_NT;
+}
+
+int finalize_launch(IterArgs &a, cudaStream_t st, int fast, vg_stats *rec)
+{
+    if (fast) VG_CUDA_CHECK(vg_launch_pdl(finalize32_kernel, 1, FIN32_NT, 0, st, a, rec));
+    else VG_CUDA_CHECK(vg_launch_pdl(finalize64_kernel, (unsigned)finalize_blocks(a), FIN_NT, 0, st, a, rec));
     return VG_OK;
 }
 
@@ -578,8 +594,7 @@ extern "C" int vg_allocate(const vg_integrator *it, void *stream)
     // grid has too few threads for it
     const int64_t ntab = (int64_t)a.dim * (a.maxK + 1);
     const int table_in_count = (it->precision == VG_F32) && ntab <= L.nblk * ALLOC_NT;
-    alloc_kernel<<<(unsigned)L.nblk, ALLOC_NT, 0, st>>>(a, L.nblk, table_in_count);
-    VG_LAUNCH_CHECK();
+    VG_CUDA_CHECK(vg_launch_pdl(alloc_kernel, (unsigned)L.nblk, ALLOC_NT, 0, st, a, L.nblk, table_in_count));
     if (it->precision == VG_F32 && !table_in_count) {
         tablef_kernel<<<(unsigned)((ntab + 255) / 256), 256, 0, st>>>(a);
         VG_LAUNCH_CHECK();
@@ -641,7 +656,7 @@ extern "C" int vg_reduce(const vg_integrator *it, uint32_t itn, const double *u,
     a.f_f64 = (f_dtype == VG_F64);
     cudaStream_t st = (cudaStream_t)stream;
     if ((rc = vg::launch_reduce(a, it->precision == VG_F64, st))) return rc;   // static tiles
-    return vg::finalize_launch(a, st, it->precision == VG_F32);
+    return vg::finalize_launch(a, st, it->precision == VG_F32, nullptr);
 }
 
 // An iteration record set to zero but for the carried sum_sigf.
@@ -737,7 +752,7 @@ extern "C" int vg_reduce_kept(const vg_integrator *it, uint32_t itn, const doubl
     a.f_f64 = (f_dtype == VG_F64);
     cudaStream_t st = (cudaStream_t)stream;
     if ((rc = vg::launch_reduce_kept(a, it->precision == VG_F64, st))) return rc;   // static tiles
-    return vg::finalize_launch(a, st, it->precision == VG_F32);
+    return vg::finalize_launch(a, st, it->precision == VG_F32, nullptr);
 }
 
 static unsigned long long *g_term_count = nullptr;
@@ -838,7 +853,7 @@ extern "C" int vg_fused_iteration(const vg_integrator *it, uint32_t itn, const d
     if ((rc = vg_build_params(kind, it->dim, params, nparams, &P, &tab_len))) return rc;
     cudaStream_t st = (cudaStream_t)stream;
     if ((rc = vg::launch_fused(a, kind, P, tab_len, it->precision == VG_F64, st))) return rc;
-    return vg::finalize_launch(a, st, it->precision == VG_F32);
+    return vg::finalize_launch(a, st, it->precision == VG_F32, nullptr);
 }
 
 // forward declaration: one full iteration (below)
@@ -849,6 +864,8 @@ int vg_adapt_launch(int dim, const int64_t *old_ninc, const int64_t *new_ninc, c
                     const uint64_t *n_f, double alpha, double *new_grid, double *new_inc,
                     int64_t ldg_new, int64_t ldi_new, cudaStream_t st, int fast, int zero_hist);
 int vg_adapt_in_place_ok(int max_old);
+int vg_adapt_cluster_args(vgadapt::AdaptArgs &a, int dim, const int64_t *ninc, double *grid, double *inc, int64_t ldg,
+                          int64_t ldi, double *sum_f, uint64_t *n_f, double alpha, int fast);
 
 extern "C" int vg_end_iteration(const vg_integrator *it, void *stream)
 {
@@ -884,45 +901,14 @@ extern "C" int vg_end_iteration(const vg_integrator *it, void *stream)
 }
 
 // One full vegas+ iteration = vg_allocate + vg_fused_iteration +
-// vg_end_iteration, enqueued by one call.  The map adapt needs only the
-// training histogram the tile kernel completed, so (unless adapt_to_errors,
-// whose finalize adds to that histogram) it runs on a forked stream while the
-// finalize merges the hypercubes cut by tile boundaries; both join back into
-// `stream` before the call returns.  The forked stream and events are created
-// on the first call on a device (outside any stream capture).
-namespace {
-struct IterAux {
-    cudaStream_t s;
-    cudaEvent_t fork, join;
-};
-std::mutex g_iter_aux_mutex;
-IterAux *g_iter_aux[VG_MAX_DEVICES];   // per device ordinal; created once, never replaced
-
-// The forked stream and events of the current device, created on the first
-// call on that device.
-int iter_aux(IterAux **out)
+// vg_end_iteration, enqueued by one call: allocation, tiles, and one kernel
+// that finalizes and adapts (adapt_to_errors, whose finalize adds to the
+// training histogram, and maps the cluster form does not take adapt after the
+// finalize).  rec: a copy of the iteration's record goes there.
+static int iterate(const vg_integrator *it, uint32_t itn, int kind, const double *params, int nparams, vg_stats *rec,
+                   cudaStream_t st)
 {
-    int dev = 0;
-    VG_CUDA_CHECK(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= VG_MAX_DEVICES) return vg_fail(VG_ERR_UNSUPPORTED, "device ordinal %d", dev);
-    std::lock_guard<std::mutex> lock(g_iter_aux_mutex);
-    if (g_iter_aux[dev] == nullptr) {
-        IterAux a;
-        VG_CUDA_CHECK(cudaStreamCreateWithFlags(&a.s, cudaStreamNonBlocking));
-        VG_CUDA_CHECK(cudaEventCreateWithFlags(&a.fork, cudaEventDisableTiming));
-        VG_CUDA_CHECK(cudaEventCreateWithFlags(&a.join, cudaEventDisableTiming));
-        g_iter_aux[dev] = new IterAux(a);
-    }
-    *out = g_iter_aux[dev];
-    return VG_OK;
-}
-}  // namespace
-
-extern "C" int vg_iterate(const vg_integrator *it, uint32_t itn, int kind, const double *params, int nparams,
-                          void *stream)
-{
-    VG_RANGE("vg_iterate");
-    int rc = vg_allocate(it, stream);
+    int rc = vg_allocate(it, st);
     if (rc) return rc;
     vg_clear_error();
     IterArgs a;
@@ -930,22 +916,35 @@ extern "C" int vg_iterate(const vg_integrator *it, uint32_t itn, int kind, const
     VgParams P;   // copied into the kernel arguments at launch
     int tab_len = 0;
     if ((rc = vg_build_params(kind, it->dim, params, nparams, &P, &tab_len))) return rc;
-    cudaStream_t st = (cudaStream_t)stream;
-    if ((rc = vg::launch_fused(a, kind, P, tab_len, it->precision == VG_F64, st))) return rc;
-    int64_t kmax = 0;
-    for (int d = 0; d < it->dim; d++) kmax = it->ninc[d] > kmax ? it->ninc[d] : kmax;
-    const int overlap = it->adapt && it->alpha > 0 && !it->adapt_to_errors && vg_adapt_in_place_ok((int)kmax);
-    if (!overlap) {
-        if ((rc = vg::finalize_launch(a, st, it->precision == VG_F32))) return rc;
-        return vg_end_iteration(it, stream);
+    const int f64 = it->precision == VG_F64;
+    if ((rc = vg::launch_fused(a, kind, P, tab_len, f64, st))) return rc;
+    vgadapt::AdaptArgs ad;
+    if (!(it->adapt && it->alpha > 0) || it->adapt_to_errors ||
+        !vg_adapt_cluster_args(ad, it->dim, it->ninc, it->grid, it->inc, it->ldg, it->ldi, it->sum_f, it->n_f, it->alpha,
+                               !f64)) {
+        if ((rc = vg::finalize_launch(a, st, !f64, rec))) return rc;
+        return vg_end_iteration(it, st);
     }
-    IterAux *aux = nullptr;
-    if ((rc = iter_aux(&aux))) return rc;
-    VG_CUDA_CHECK(cudaEventRecord(aux->fork, st));
-    VG_CUDA_CHECK(cudaStreamWaitEvent(aux->s, aux->fork, 0));
-    rc = vg_end_iteration(it, aux->s);
-    VG_CUDA_CHECK(cudaEventRecord(aux->join, aux->s));
-    if (rc == VG_OK) rc = vg::finalize_launch(a, st, it->precision == VG_F32);
-    VG_CUDA_CHECK(cudaStreamWaitEvent(st, aux->join, 0));
-    return rc;
+    const int nfin = f64 ? (int)finalize_blocks(a) : 1;
+    const int C = vgadapt::CLUSTER;
+    const unsigned grid = (unsigned)(C * (it->dim + (nfin + C - 1) / C));
+    // placed early, its CTAs would all wait on the few SMs that come free first
+    // and share their FP64 pipes there: an ordinary launch
+    tail_kernel<<<grid, FIN_NT, 0, st>>>(a, ad, f64, nfin, rec);
+    VG_LAUNCH_CHECK();
+    return VG_OK;
+}
+
+extern "C" int vg_iterate(const vg_integrator *it, uint32_t itn, int kind, const double *params, int nparams,
+                          void *stream)
+{
+    VG_RANGE("vg_iterate");
+    return iterate(it, itn, kind, params, nparams, nullptr, (cudaStream_t)stream);
+}
+
+extern "C" int vg_iterate_record(const vg_integrator *it, uint32_t itn, int kind, const double *params, int nparams,
+                                 vg_stats *rec, void *stream)
+{
+    VG_RANGE("vg_iterate_record");
+    return iterate(it, itn, kind, params, nparams, rec, (cudaStream_t)stream);
 }

@@ -329,6 +329,31 @@ extern "C" int vg_add_training_data(int dim, const int64_t *ninc, int64_t ldi, i
 // In place the kernel also stages the old nodes and increments (two more rows).
 int vg_adapt_in_place_ok(int max_old) { return 4 * (size_t)max_old + 1 <= 2 * VG_ADAPT_MAX_NINC; }
 
+// Arguments of the in-place adapt by clusters; 0 where that form does not take
+// the map (an axis with a single increment reuses the previous axis' weight,
+// pyx:533-564, and a CTA holds 128 increments).
+int vg_adapt_cluster_args(AdaptArgs &a, int dim, const int64_t *ninc, double *grid, double *inc, int64_t ldg,
+                          int64_t ldi, double *sum_f, uint64_t *n_f, double alpha, int fast)
+{
+    if (dim < 1 || dim > VG_MAX_DIM || sum_f == nullptr || !(alpha > 0)) return 0;
+    memset(&a, 0, sizeof(a));
+    a.dim = dim;
+    for (int d = 0; d < dim; d++) {
+        if (ninc[d] < 2 || ninc[d] > vgadapt::CLUSTER_MAX || ninc[d] + 1 > ldg || ninc[d] > ldi) return 0;
+        a.old_ninc[d] = a.new_ninc[d] = (int)ninc[d];
+    }
+    a.grid = a.new_grid = grid;
+    a.inc = a.new_inc = inc;
+    a.ldg = a.ldg_new = ldg;
+    a.ldi = a.ldi_new = ldi;
+    a.sum_f = sum_f;
+    a.n_f = (const unsigned long long *)n_f;
+    a.alpha = alpha;
+    a.fast = fast;
+    a.zero_hist = 1;
+    return 1;
+}
+
 // In place (new_grid == grid, new_inc == inc) needs the old ninc to equal
 // the new one and vg_adapt_in_place_ok(); zero_hist clears sum_f / n_f once
 // read.

@@ -329,6 +329,8 @@ __device__ __forceinline__ bool scan_pieces(Piece &cur, bool started)
 }
 
 // ------------------------------------------------------------------ kernel
+constexpr int RF_CHAIN = 8;   // a kernel of its own, launched with vg_launch_pdl
+
 template <bool WIDE>
 struct IndexType {
     typedef int type;
@@ -381,12 +383,8 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
     WarpBuf &wb = reinterpret_cast<WarpBuf *>(smem + sp.warps)[warp];
     float *win_w = reinterpret_cast<float *>(wb.res);
 
-    if (a.stats->ntiles == 0) return;   // allocation failed: nothing to do
-    const int64_t N = a.stats->neval;
-
-    // ---- per-CTA setup: grid table, histogram, integrand constants
-    if (NEED_MAP && table_smem)
-        for (int i = tid; i < dim * W; i += NTB) table[i] = a.tablef[i];
+    // ---- per-CTA setup: histogram, integrand constants; then, once the
+    // allocation is done, the grid table
     const int hist = dim * W;   // the last bin of an axis takes what is not counted
     if (NEED_RED && a.train && a.hist_smem) {
         for (int i = tid; i < hist * a.hist_smem; i += NTB) hsum[i] = 0.f;
@@ -397,6 +395,14 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
         kc = vg_prepare_f32<KIND>(prm, dim);
         vg_fill_table_f32<KIND>(prm, dim, itab, kc);
     }
+    if (F & RF_CHAIN) {
+        vg_pdl_wait();
+        vg_pdl_go();
+    }
+    if (a.stats->ntiles == 0) return;   // allocation failed: nothing to do
+    const int64_t N = a.stats->neval;
+    if (NEED_MAP && table_smem)
+        for (int i = tid; i < dim * W; i += NTB) table[i] = a.tablef[i];
     __syncthreads();
 
     const float dv_yf = (float)a.dv_y;
@@ -838,7 +844,7 @@ __global__ void __launch_bounds__(range_threads(DIMB), 1)
 range_kernel(const __grid_constant__ IterArgs a, const __grid_constant__ VgParams prm)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    range_body<MODE, KIND, DIMB, F>(a, prm, smem, blockIdx.x, gridDim.x, 0);
+    range_body<MODE, KIND, DIMB, F | RF_CHAIN>(a, prm, smem, blockIdx.x, gridDim.x, 0);
 }
 
 // Shared memory of a CTA: the histogram comes first (its copies spread the
@@ -883,8 +889,7 @@ int launch_range_as(IterArgs &a, const VgParams *prm, size_t smem, cudaStream_t 
     a.ncta = (int)grid;
     a.ngroups = grid * (NTB / 32 / GROUP);
     static const VgParams empty = {};
-    kern<<<(unsigned)grid, NTB, smem, st>>>(a, prm ? *prm : empty);
-    VG_LAUNCH_CHECK();
+    VG_CUDA_CHECK(vg_launch_pdl(kern, (unsigned)grid, NTB, smem, st, a, prm ? *prm : empty));
     return VG_OK;
 }
 

@@ -551,14 +551,13 @@ __device__ __forceinline__ void tile_body(const IterArgs &a, const VgParams &prm
     // a.parts[slot]; the sums restart from zero.
     auto emit_partial = [&](int64_t slot) {
         __syncthreads();
-        const VgKSum m = vg_block_ksum<NTB>(VgKSum{acc_m, 0.0}, red);
-        const VgKSum v = vg_block_ksum<NTB>(VgKSum{acc_v, 0.0}, red);
-        const VgKSum sg = vg_block_ksum<NTB>(VgKSum{acc_s, 0.0}, red);
+        VgKSum v3[3] = {{acc_m, 0.0}, {acc_v, 0.0}, {acc_s, 0.0}};
+        vg_block_ksum3<NTB>(v3, red);
         if (tid == 0) {
             TilePart p;
-            p.mean = m;
-            p.var = v;
-            p.sigf = sg;
+            p.mean = v3[0];
+            p.var = v3[1];
+            p.sigf = v3[2];
             a.parts[slot] = p;
         }
         acc_m = acc_v = acc_s = 0.0;
@@ -947,6 +946,8 @@ __global__ void __launch_bounds__(NTB, 1) tile_kernel(const __grid_constant__ It
                                                    const __grid_constant__ VgParams prm)
 {
     extern __shared__ __align__(16) unsigned char smem[];
+    vg_pdl_wait();
+    vg_pdl_go();
     tile_body<MODE, KIND, DIMB, S, NTB>(a, prm, smem, blockIdx.x, gridDim.x, blockIdx.x);
 }
 
@@ -994,18 +995,23 @@ int launch_tile_as(IterArgs &a, const VgParams *prm, cudaStream_t st, int stage)
     if (NEED_RED && grid > MAX_PARTS) grid = MAX_PARTS;
     a.ncta = (int)grid;
     static const VgParams empty = {};
-    kern<<<(unsigned)grid, NTB, p.total, st>>>(a, prm ? *prm : empty);
-    VG_LAUNCH_CHECK();
+    VG_CUDA_CHECK(vg_launch_pdl(kern, (unsigned)grid, NTB, p.total, st, a, prm ? *prm : empty));
     return VG_OK;
 }
 
 template <int MODE, int KIND, int DIMB, int S>
 int launch_tile(IterArgs &a, const VgParams *prm, cudaStream_t st)
 {
+    // Fewer large tiles than SMs: tiles of 128 samples instead, four times as
+    // many, so that the FP64 work (19 cycles per warp instruction and SM) spreads
+    // over more SMs; a CTA then has too few samples to stage the grid or a
+    // histogram for.  1e4 evaluations at dim 4: 75 us on 18 SMs before.
+    if (MODE != MODE_POINTS && (a.ncap + NT * S - 1) / (NT * S) < vg_num_sms())
+        return launch_tile_as<MODE, KIND, DIMB, 1, BASE_TILE>(a, prm, st, 0);
     return launch_tile_as<MODE, KIND, DIMB, S, NT>(a, prm, st, 1);
 }
 
-int finalize_launch(IterArgs &a, cudaStream_t st, int fast);
+int finalize_launch(IterArgs &a, cudaStream_t st, int fast, vg_stats *rec);
 int launch_reduce(IterArgs &a, int f64, cudaStream_t st);
 int launch_reduce_kept(IterArgs &a, int f64, cudaStream_t st);
 // IterArgs of one integral (pointers into its workspace) and its adapt scratch grid

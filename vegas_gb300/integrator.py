@@ -662,11 +662,10 @@ class Integrator(object):
     def _call_pipelined(self, fcn, result):
         """__call__ for a built-in integrand when no iteration needs a host
         decision (no rtol/atol stop, analyzer or save): every iteration --
-        allocation, fused evaluate+reduce, adapt, one ``vg_iterate`` call
-        that overlaps the adapt with the iteration sums -- is enqueued without
-        waiting, and each iteration's record is copied to pinned host memory
-        on the same stream; the records are read once after the last
-        iteration.  Same kernels and results as the iteration-by-iteration
+        allocation, fused evaluate+reduce, adapt, one ``vg_iterate_record``
+        call -- is enqueued without waiting, and its last kernel writes the
+        iteration's record to pinned host memory; the records are read once
+        after the last iteration.  Same kernels and results as the iteration-by-iteration
         loop, without a host round trip per iteration."""
         L = N.load()
         stream = N.stream_ptr(self.device)
@@ -676,14 +675,13 @@ class Integrator(object):
         params = N.dbl_array(p)
         nitn = int(self.nitn)
         host = self._records_host(nitn)
+        rec, sz = host.data_ptr(), ctypes.sizeof(N.VgStats)   # pinned: the device writes the records there
         for k in range(nitn):
             self._itn += 1
-            N.check(L.vg_iterate(ctypes.byref(it), self._itn & 0xffffffff, int(fcn.kind), params, len(p),
-                                 stream))
-            host[k].copy_(self._stats, non_blocking=True)
+            N.check(L.vg_iterate_record(ctypes.byref(it), self._itn & 0xffffffff, int(fcn.kind), params, len(p),
+                                        rec + k * sz, stream))
         torch.cuda.current_stream(self.device).synchronize()
         raw = host[:nitn].numpy().tobytes()
-        sz = ctypes.sizeof(N.VgStats)
         gs = []
         for k in range(nitn):
             st = N.VgStats.from_buffer_copy(raw, k * sz)
@@ -695,9 +693,9 @@ class Integrator(object):
 
     def _call_stepwise(self, fcn, result, save, saveall):
         """__call__ for a built-in integrand when iterations need a host
-        decision (rtol/atol stop, analyzer, save): one ``vg_iterate`` call
-        per iteration (the kernels of the pipelined path), its record copied
-        to pinned host memory and waited for on an event; sum_sigf stays on
+        decision (rtol/atol stop, analyzer, save): one ``vg_iterate_record``
+        call per iteration (the kernels of the pipelined path), its record
+        written to pinned host memory and waited for on an event; sum_sigf stays on
         the device between iterations.  The analyzer, save and stopping rule
         run after each iteration as in the reference (pyx:2086-2226)."""
         L = N.load()
@@ -713,9 +711,8 @@ class Integrator(object):
             if self.analyzer is not None:
                 self.analyzer.begin(itn, self)
             self._itn += 1
-            N.check(L.vg_iterate(ctypes.byref(it), self._itn & 0xffffffff, int(fcn.kind), params, len(p),
-                                 stream))
-            host[0].copy_(self._stats, non_blocking=True)
+            N.check(L.vg_iterate_record(ctypes.byref(it), self._itn & 0xffffffff, int(fcn.kind), params, len(p),
+                                        host.data_ptr(), stream))
             done.record(torch.cuda.current_stream(self.device))
             done.synchronize()
             st = N.VgStats.from_buffer_copy(host[0].numpy().tobytes()[:sz])
@@ -758,9 +755,8 @@ class Integrator(object):
         itn0 = self._itn
 
         def enqueue(k):
-            N.check(L.vg_iterate(ctypes.byref(it), (itn0 + k + 1) & 0xffffffff, int(fcn.kind), params, len(p),
-                                 stream))
-            host[k % 2].copy_(self._stats, non_blocking=True)
+            N.check(L.vg_iterate_record(ctypes.byref(it), (itn0 + k + 1) & 0xffffffff, int(fcn.kind), params, len(p),
+                                        host.data_ptr() + (k % 2) * sz, stream))
             done[k % 2].record(cur)
             g, i, s_ = bk[k % 2]
             g.copy_(grid, non_blocking=True)
