@@ -1419,6 +1419,299 @@ __global__ void __launch_bounds__(UNT, 1) flow_pass_umma_kernel(FlowGeom g, cons
     if (warp == 0) umma::tmem_dealloc(tmem, 512);
 }
 
+// ------------------------------------- two groups of warps, A operands in TMEM
+// The same pass with the CTA's 16 warps in two groups of 8, each on its own
+// 128-row sub-tiles: while one group waits for its MMAs or its barriers, the
+// other computes (one group of 16 warps in step issued 0.47 instructions per
+// cycle and scheduler).  A group's activations stay in TMEM as the A operands
+// of its MMAs (tcgen05.st), so no shared memory is needed for them and two groups
+// fit beside the weights at dim 16 too.  TMEM columns of a group: 144 for H1 W2^T
+// and, after the H2 epilogue has read it, the logits of one pair of coordinates;
+// 64 for H1 and then H2.  The pair's MMA is followed by the next pair's as soon as
+// the logits are in registers, so it runs under the splines.  A sub-tile stays with
+// its group through the layers; the groups share only the weights: the one
+// that finishes a layer's MMAs second starts the copy of the next layer's, under
+// the last splines.  Every wait is bounded; one that gives up sets a flag, after
+// which nothing waits any more and the loops run to their end.
+// The splines of 2^20 rows at dim 8: 1.60 ms with one group; see the launcher for
+// when this form is taken.
+constexpr int DUO_NT = 256;      // threads of a group
+constexpr int DUO_D = 0, DUO_A = 160, DUO_COLS = 256;   // TMEM columns of a group
+
+struct DuoPlan {
+    int ST, zst;
+    size_t oW2, oW3, oV, vgroup, oZ, oLD, total;
+};
+
+__host__ __device__ inline DuoPlan duo_plan(const FlowGeom &g, int ST)
+{
+    DuoPlan p;
+    p.ST = ST;
+    p.zst = g.dim | 1;
+    size_t o = 0;
+    p.oW2 = o; o += (size_t)FH * FH * 2;
+    p.oW3 = o; o += (size_t)g.NPmax * FH * 2;
+    // per group: W1 padded to 8 columns, b1, b2, b3 (8 coordinates of 2K + 1, padded)
+    p.oV = o;
+    p.vgroup = sizeof(float) * (FH * 8 + 2 * FH + 8 * bias_stride(g.K));
+    o += 2 * p.vgroup;
+    p.oZ = o;  o += sizeof(float) * (size_t)ST * FROWS * p.zst;
+    p.oLD = o; o += sizeof(float) * UNH * (size_t)ST * FROWS;
+    p.total = o + 1024;          // + alignment slack of the dynamic base
+    return p;
+}
+
+template <int K, int DIR>
+__global__ void __launch_bounds__(UNT, 1) flow_pass_duo_kernel(FlowGeom g, const float *__restrict__ theta,
+                                                              const __nv_bfloat16 *__restrict__ mirror, int64_t n,
+                                                              const float *__restrict__ zin, float *__restrict__ zout,
+                                                              float *__restrict__ logdet, float *__restrict__ zl, int ST)
+{
+    constexpr int NR = 2 * K + 1;
+    extern __shared__ uint8_t dsm[];
+    __shared__ uint64_t bars[4];   // 0 weights, 1-2 the groups' MMAs, 3 drain
+    __shared__ uint32_t tslot;
+    __shared__ volatile int abort_flag;
+    __shared__ int layers_done;    // by both groups together
+    __shared__ volatile int ncopies;   // of a layer's weights, begun
+    uint8_t *base = umma::align1024(dsm);
+    const DuoPlan pl = duo_plan(g, ST);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int grp = tid / DUO_NT, tg = tid % DUO_NT;
+    const int r = tg & (FROWS - 1), h = tg >> 7;   // row, and which of a pair of coordinates / half of the columns
+    const bool leader = tg == 0;
+    uint8_t *sW2 = base + pl.oW2, *sW3 = base + pl.oW3;
+    float *sW1 = (float *)(base + pl.oV + grp * pl.vgroup), *sb1 = sW1 + FH * 8, *sb2 = sb1 + FH, *sb3 = sb2 + FH;
+    float *sZ = (float *)(base + pl.oZ), *sLD = (float *)(base + pl.oLD);
+    const int dim = g.dim, zst = pl.zst, CH = g.CH;
+    const uint32_t bar_w = umma::smem_u32(&bars[0]), bar_m = umma::smem_u32(&bars[1 + grp]);
+    const uint32_t bar_d = umma::smem_u32(&bars[3]);
+    if (warp == 0) umma::tmem_alloc(umma::smem_u32(&tslot), 512);
+    if (tid == 0) {
+        for (int i = 0; i < 3; i++) umma::mbar_init(umma::smem_u32(&bars[i]), 1);
+        umma::mbar_init(bar_d, 2);
+        abort_flag = 0;
+        layers_done = 0;
+        ncopies = 0;
+    }
+    umma::fence_before_sync();
+    __syncthreads();
+    umma::fence_after_sync();
+    const uint32_t tmem = tslot + (uint32_t)(grp * DUO_COLS);
+    const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;
+    const uint32_t tD = tmem + DUO_D, tA = tmem + DUO_A;
+    const int64_t rows_per = (int64_t)ST * FROWS;
+    const int64_t nsuper = (n + rows_per - 1) / rows_per;
+    const int64_t nmine = (nsuper - blockIdx.x + gridDim.x - 1) / gridDim.x;
+    const int64_t nsteps = nmine * g.L;
+
+    auto layer_of = [&](int64_t step) { return DIR == 0 ? (int)(step % g.L) : g.L - 1 - (int)(step % g.L); };
+    auto copy_weights = [&](int64_t step) {   // one thread
+        const FlowLayer &y = g.ly[layer_of(step)];
+        const uint32_t b2 = (uint32_t)FH * FH * 2, b3 = (uint32_t)y.NP * FH * 2;
+        ncopies = ncopies + 1;
+        umma::mbar_expect_tx(bar_w, b2 + b3);
+        umma::bulk_g2s(umma::smem_u32(sW2), mirror + y.mU2, b2, bar_w);
+        for (uint32_t off = 0; off < b3; off += 32768u) {
+            const uint32_t sz = (b3 - off) < 32768u ? (b3 - off) : 32768u;
+            umma::bulk_g2s(umma::smem_u32(sW3) + off, (const uint8_t *)(mirror + y.mU3) + off, sz, bar_w);
+        }
+    };
+    auto wait = [&](uint32_t bar, uint32_t ph) {   // every warp; bounded
+        if (lane == 0 && !abort_flag && !umma::mbar_wait(bar, ph)) abort_flag = 1;
+        __syncwarp();
+    };
+    auto group_sync = [&]() { asm volatile("bar.sync %0, 256;" ::"r"(1 + grp) : "memory"); };
+    // Thread work and fences before the group's leader issues an MMA.
+    auto before_mma = [&]() {
+        umma::fence_before_sync();
+        group_sync();
+        if (leader) umma::fence_after_sync();
+    };
+    uint32_t ph_w = 0, ph_m = 0;
+    if (tid == 0 && nsteps > 0) copy_weights(0);
+    int64_t step = 0;
+    for (int64_t sup = blockIdx.x; sup < nsuper; sup += gridDim.x) {
+        const int64_t r0 = sup * rows_per;
+        const int nrows = (int)((n - r0) < rows_per ? (n - r0) : rows_per);
+        const int nsub = (nrows + FROWS - 1) / FROWS;
+        for (int s = grp; s < nsub; s += 2) {
+            for (int i = tg; i < FROWS * dim; i += DUO_NT) {
+                const int rr = s * FROWS + i / dim, d = i % dim;
+                sZ[rr * zst + d] = rr < nrows ? zin[(r0 + rr) * dim + d] : 0.5f;
+            }
+            for (int i = tg; i < FROWS * UNH; i += DUO_NT)
+                sLD[(size_t)(i / FROWS) * ST * FROWS + s * FROWS + i % FROWS] = 0.f;
+        }
+        for (int q = 0; q < g.L; q++, step++) {
+            const int l = layer_of(step);
+            const FlowLayer &y = g.ly[l];
+            const int dA = y.realA ? y.dA : 1;
+            for (int i = tg; i < FH * 8; i += DUO_NT) {   // W1 padded to 8 columns: [128][8]
+                const int c = i >> 3, a = i & 7;
+                sW1[i] = a < dA ? theta[y.oW1 + c * dA + a] : 0.f;
+            }
+            for (int i = tg; i < FH; i += DUO_NT) {
+                sb1[i] = theta[y.ob1 + i];
+                sb2[i] = theta[y.ob2 + i];
+            }
+            for (int i = tg; i < y.dB * NR; i += DUO_NT) sb3[(i / NR) * bias_stride(K) + i % NR] = theta[y.ob3 + i];
+            wait(bar_w, ph_w);
+            ph_w ^= 1;
+            group_sync();
+            const int npair = (y.dB + 1) / 2;
+            // the output layer of a pair of coordinates; leader only
+            auto issue_pair = [&](int p) {
+                const int N = 2 * p + 1 < y.dB ? 2 * CH : (CH + 15) / 16 * 16;
+                umma::gemm_ts_128xN(tD, tA, umma::smem_u32(sW3) + (uint32_t)(2 * p * CH) * 128u, N, FH, y.NP);
+                umma::mma_commit(bar_m);
+            };
+            auto done_with_weights = [&]() {   // leader, after the group's last MMA of the layer
+                __threadfence_block();
+                if (atomicAdd(&layers_done, 1) & 1) {   // the other group is done as well
+                    __threadfence_block();
+                    if (step + 1 < nsteps && !abort_flag) copy_weights(step + 1);
+                }
+            };
+            if (grp >= nsub && leader) done_with_weights();
+            for (int s = grp; s < nsub; s += 2) {
+                float *Zs = sZ + (size_t)s * FROWS * zst;
+                if (zl != nullptr)
+                    for (int i = tg; i < FROWS * dim; i += DUO_NT) {
+                        const int rr = i / dim, d = i % dim;
+                        const int64_t grow = r0 + (int64_t)s * FROWS + rr;
+                        if (grow < n) zl[((int64_t)l * n + grow) * dim + d] = Zs[rr * zst + d];
+                    }
+                {   // H1 = relu(W1 z_A + b1) in FP32 -> A operand
+                    float xa[8];
+#pragma unroll
+                    for (int a = 0; a < 8; a++) xa[a] = (a < dA && y.realA) ? Zs[r * zst + y.A[a]] : 0.f;
+                    const bool wide = dA > 4;
+#pragma unroll 1
+                    for (int c0 = 64 * h; c0 < 64 * h + 64; c0 += 32) {
+                        uint32_t pk[16];
+#pragma unroll
+                        for (int c = 0; c < 32; c += 2) {
+                            float v[2];
+#pragma unroll
+                            for (int e = 0; e < 2; e++) {
+                                const float4 w0 = *reinterpret_cast<const float4 *>(sW1 + (c0 + c + e) * 8);
+                                float acc = sb1[c0 + c + e];
+                                acc = fmaf(w0.x, xa[0], acc);
+                                acc = fmaf(w0.y, xa[1], acc);
+                                acc = fmaf(w0.z, xa[2], acc);
+                                acc = fmaf(w0.w, xa[3], acc);
+                                if (wide) {
+                                    const float4 w1 = *reinterpret_cast<const float4 *>(sW1 + (c0 + c + e) * 8 + 4);
+                                    acc = fmaf(w1.x, xa[4], acc);
+                                    acc = fmaf(w1.y, xa[5], acc);
+                                    acc = fmaf(w1.z, xa[6], acc);
+                                    acc = fmaf(w1.w, xa[7], acc);
+                                }
+                                v[e] = fmaxf(acc, 0.f);
+                            }
+                            pk[c >> 1] = pack_bf16(v[0], v[1]);
+                        }
+                        umma::tmem_st16(tA + lane_base + (uint32_t)(c0 >> 1), pk);
+                    }
+                    umma::tmem_wait_st();
+                }
+                before_mma();
+                if (leader) {
+                    umma::gemm_ts_128xN(tD, tA, umma::smem_u32(sW2), FH, FH, FH);
+                    umma::mma_commit(bar_m);
+                }
+                wait(bar_m, ph_m);
+                ph_m ^= 1;
+                umma::fence_after_sync();
+                // H2 = relu(. + b2) -> A operand (in place of H1)
+#pragma unroll 1
+                for (int c0 = 64 * h; c0 < 64 * h + 64; c0 += 32) {
+                    float v[32];
+                    umma::tmem_ld32(tD + lane_base + (uint32_t)c0, v);
+                    uint32_t pk[16];
+#pragma unroll
+                    for (int c = 0; c < 32; c += 4) {
+                        const float4 b = *reinterpret_cast<const float4 *>(sb2 + c0 + c);
+                        pk[c >> 1] = pack_bf16(fmaxf(v[c] + b.x, 0.f), fmaxf(v[c + 1] + b.y, 0.f));
+                        pk[(c >> 1) + 1] = pack_bf16(fmaxf(v[c + 2] + b.z, 0.f), fmaxf(v[c + 3] + b.w, 0.f));
+                    }
+                    umma::tmem_st16(tA + lane_base + (uint32_t)(c0 >> 1), pk);
+                }
+                umma::tmem_wait_st();
+                before_mma();
+                if (leader) issue_pair(0);
+#pragma unroll 1
+                for (int p = 0; p < npair; p++) {
+                    wait(bar_m, ph_m);
+                    ph_m ^= 1;
+                    umma::fence_after_sync();
+                    if (p + 1 == npair && s + 2 >= nsub && leader) done_with_weights();
+                    const int j = 2 * p + h;   // this thread's coordinate
+                    float o[NR];
+                    if (j < y.dB) {
+                        const uint32_t col = tD + lane_base + (uint32_t)(h * CH);
+                        float v[32];
+                        umma::tmem_ld32(col, v);
+#pragma unroll
+                        for (int i = 0; i < 32; i++) o[i] = v[i];
+                        if (NR > 32) {
+                            umma::tmem_ld32(col + 32u, v);
+#pragma unroll
+                            for (int i = 0; i < 32; i++)
+                                if (32 + i < NR) o[32 + i] = v[i];
+                        }
+                        if (NR > 64) o[64] = umma::tmem_ld1(col + 64u);
+                    }
+                    if (p + 1 < npair) {   // the next pair's logits replace these
+                        before_mma();
+                        if (leader) issue_pair(p + 1);
+                    }
+                    if (j < y.dB) {
+                        add_bias<K>(o, sb3 + j * bias_stride(K));
+                        const int cz = y.B[j];
+                        const float xin = Zs[r * zst + cz];
+                        float lp;
+                        const float xo = spline_reg<K, DIR>(o, xin, lp);
+                        Zs[r * zst + cz] = fminf(fmaxf(xo, 0.f), 1.f);
+                        sLD[(size_t)(j & (UNH - 1)) * ST * FROWS + s * FROWS + r] += lp;
+                    }
+                }
+            }
+            group_sync();   // the layer's output, and its vectors are free
+        }
+        for (int s = grp; s < nsub; s += 2) {
+            for (int i = tg; i < FROWS * dim; i += DUO_NT) {
+                const int rr = s * FROWS + i / dim, d = i % dim;
+                if (rr < nrows) zout[(r0 + rr) * dim + d] = sZ[rr * zst + d];
+            }
+            for (int i = tg; i < FROWS; i += DUO_NT) {
+                const int rr = s * FROWS + i;
+                float ld = 0.f;
+#pragma unroll
+                for (int q = 0; q < UNH; q++) ld += sLD[(size_t)q * ST * FROWS + rr];
+                if (rr < nrows) logdet[r0 + rr] = ld;
+            }
+        }
+        group_sync();
+    }
+    // drain: every MMA issued has completed before TMEM is freed (and after a
+    // wait that gave up, the weights in flight have arrived)
+    if (leader) umma::mma_commit(bar_d);
+    if (tid == 0) {
+        if (!umma::mbar_wait(bar_d, 0)) abort_flag = 1;
+    }
+    umma::fence_before_sync();
+    __syncthreads();
+    if (tid == 0 && abort_flag) {
+        umma::mbar_wait(bar_w, (uint32_t)(ncopies - 1) & 1u);
+        atomicExch(&g_flow_status, VG_ERR_TIMEOUT);
+    }
+    umma::fence_after_sync();
+    __syncthreads();
+    if (warp == 0) umma::tmem_dealloc(tslot, 512);
+}
+
 // ------------------------------------------------ tcgen05 training backward
 // Makes the compiler treat the values of o[] as redefined here (no
 // instruction is emitted), so that sums of them are recomputed in the next
@@ -2365,6 +2658,52 @@ extern "C" int vg_flow_refresh(const vg_flow *fl, void *stream)
     return VG_OK;
 }
 
+// The two-group form where every CTA has two sub-tiles or more; below that one
+// group of 16 warps on a CTA's only sub-tile has the shorter way through a layer.
+// Returns 1 when it launched.
+template <int K>
+static int flow_pass_duo_k(const FlowGeom &g, const vg_flow *fl, int dir, int64_t n, const float *zin, float *zout,
+                           float *logdet, float *zl, cudaStream_t st, int *rc)
+{
+    const int64_t nsub = (n + FROWS - 1) / FROWS, G = vg_num_sms();
+    if (nsub <= G) return 0;
+    const void *k = dir == 0 ? (const void *)flow_pass_duo_kernel<K, 0> : (const void *)flow_pass_duo_kernel<K, 1>;
+    size_t stat = 0;
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, k) == cudaSuccess) stat = fa.sharedSizeBytes;
+    else (void)cudaGetLastError();
+    const size_t limit = VG_FLOW_SMEM_MAX > stat ? VG_FLOW_SMEM_MAX - stat : 0;
+    if (duo_plan(g, 2).total > limit) return 0;
+    // sub-tiles per super-tile: an even number; the fewest steps of a group over
+    // all of a CTA's super-tiles, then the fewest super-tiles (copies of the weights)
+    int ST = 2;
+    int64_t best = 0;
+    for (int t = 2; t <= UST_MAX && duo_plan(g, t).total <= limit; t += 2) {
+        const int64_t nsup = (nsub + t - 1) / t, rounds = (nsup + G - 1) / G;
+        const int64_t cost = rounds * (t / 2) * 8 + rounds;
+        if (best == 0 || cost < best) {
+            best = cost;
+            ST = t;
+        }
+    }
+    const DuoPlan pl = duo_plan(g, ST);
+    const size_t smem = pl.total < 120 * 1024 ? 120 * 1024 : pl.total;   // one CTA per SM (TMEM: 512 columns)
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    const int64_t nsup = (nsub + ST - 1) / ST;
+    const unsigned grid = (unsigned)(nsup < G ? nsup : G);
+    const __nv_bfloat16 *mirror = (const __nv_bfloat16 *)fl->mirror;
+    if (dir == 0)
+        flow_pass_duo_kernel<K, 0><<<grid, UNT, smem, st>>>(g, fl->theta, mirror, n, zin, zout, logdet, zl, ST);
+    else
+        flow_pass_duo_kernel<K, 1><<<grid, UNT, smem, st>>>(g, fl->theta, mirror, n, zin, zout, logdet, zl, ST);
+    cudaError_t e = cudaGetLastError();
+    *rc = e == cudaSuccess ? VG_OK : vg_fail(VG_ERR_CUDA, "flow pass launch: %s", cudaGetErrorString(e));
+    return 1;
+}
+
 // tcgen05 inference pass when the configuration fits it (K in {16, 32},
 // at most 8 conditioning coordinates per layer, shared memory); returns 1
 // when it launched, 0 when the caller should use the mma.sync pass.
@@ -2423,6 +2762,9 @@ static int flow_pass(const vg_flow *fl, int dir, int64_t n, const float *zin, fl
     if (n <= 0) return VG_OK;
     if (!g_flow_force_legacy && g.dAmax <= 8 && g.dBmax <= 8) {
         int used = 0;
+        if (g.K == 32) used = flow_pass_duo_k<32>(g, fl, dir, n, zin, zout, logdet, zl, st, &rc);
+        else if (g.K == 16) used = flow_pass_duo_k<16>(g, fl, dir, n, zin, zout, logdet, zl, st, &rc);
+        if (used) return rc;
         if (g.K == 32) used = flow_pass_umma_k<32>(g, fl, dir, n, zin, zout, logdet, zl, st, &rc);
         else if (g.K == 16) used = flow_pass_umma_k<16>(g, fl, dir, n, zin, zout, logdet, zl, st, &rc);
         if (used) return rc;

@@ -102,6 +102,16 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
+// the same with A in TMEM: bf16, lane = row, two consecutive k per 32-bit column
+__device__ __forceinline__ void mma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate)
+{
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate));
+}
+
 // arrive on the mbarrier once every MMA issued so far by this thread completed
 __device__ __forceinline__ void mma_commit(uint32_t bar)
 {
@@ -120,6 +130,17 @@ __device__ __forceinline__ void gemm_128xN(uint32_t tmem_d, uint32_t a_saddr, ui
         const uint32_t boff = (uint32_t)((k >> 6) * rowsB * 128 + ((k & 63) << 1));
         mma_bf16(tmem_d, sdesc_sw128(a_saddr + aoff), sdesc_sw128(b_saddr + boff), idesc,
                  (k > 0 || accumulate) ? 1u : 0u);
+    }
+}
+
+// The same with A in TMEM (Kt/2 columns at tmem_a).
+__device__ __forceinline__ void gemm_ts_128xN(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_saddr, int N, int Kt,
+                                              int rowsB)
+{
+    const uint32_t idesc = idesc_bf16(128, N);
+    for (int k = 0; k < Kt; k += 16) {
+        const uint32_t boff = (uint32_t)((k >> 6) * rowsB * 128 + ((k & 63) << 1));
+        mma_bf16_ts(tmem_d, tmem_a + (uint32_t)(k >> 1), sdesc_sw128(b_saddr + boff), idesc, k > 0 ? 1u : 0u);
     }
 }
 
@@ -181,6 +202,18 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32])
 #pragma unroll
     for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
+
+// registers -> TMEM: 32 lanes x 32 bit, 16 consecutive columns, and the wait
+// for this thread's stores
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16])
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ float tmem_ld1(uint32_t taddr)
 {
