@@ -889,6 +889,45 @@ __global__ void flow_adam_kernel(int64_t np, float *__restrict__ theta, const fl
     }
 }
 
+// Two FP32 values in a register pair and the packed operations on them (each
+// lane rounds as the scalar one): half the instructions where the splines are
+// bound by their issue.
+__device__ __forceinline__ uint64_t f2_pack(float a, float b)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2_unpack(uint64_t v, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c)
+{
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+// relu of a pair of bf16 (a NaN becomes 0, as fmaxf makes it)
+__device__ __forceinline__ uint32_t relu_bf16x2(uint32_t v)
+{
+    uint32_t r;
+    asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(0u));
+    return r;
+}
+
 // ------------------------------------------------- tcgen05 inference pass
 // Spline of one coordinate with its 2K+1 logits in registers (compile-time
 // K, fully unrolled).  DIR 0: CDF at x; DIR 1: inverse CDF at x.  Returns
@@ -902,41 +941,53 @@ __device__ __forceinline__ float spline_reg(float (&o)[2 * K + 1], float x, floa
     static_assert(K % 8 == 0, "K must be a multiple of 8");
     constexpr int NB = K / 8;
     constexpr float c1 = 1.f - K * EPS_W;
-    float m4[4], v4[4];
+    float mx = o[0], mv = o[K], mx2 = o[1], mv2 = o[K + 1];   // two chains each
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-        m4[q] = o[q];
-        v4[q] = o[K + q];
+    for (int k = 2; k < K; k += 4) {
+        mx = max3(mx, o[k], o[k + 1]);
+        if (k + 2 < K) mx2 = max3(mx2, o[k + 2], o[k + 3]);
     }
 #pragma unroll
-    for (int k = 4; k < K; k++) m4[k & 3] = fmaxf(m4[k & 3], o[k]);
-#pragma unroll
-    for (int k = 4; k <= K; k++) v4[k & 3] = fmaxf(v4[k & 3], o[K + k]);
-    const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-    const float mv = fmaxf(fmaxf(v4[0], v4[1]), fmaxf(v4[2], v4[3]));
+    for (int k = 2; k < K; k += 4) {
+        mv = max3(mv, o[K + k], o[K + k + 1]);
+        if (k + 2 < K) mv2 = max3(mv2, o[K + k + 2], o[K + k + 3]);
+    }
+    mx = fmaxf(mx, mx2);
+    mv = max3(mv, mv2, o[2 * K]);
     // exponentials as 2^(v log2 e - max log2 e): one FMA and the MUFU each;
     // the vertex heights are stored halved (exponent - 1), which absorbs the
     // trapezoid's 1/2 in the segment areas (the partial-bin formulas at the
     // end restore the factor 2)
     constexpr float L2E = 1.4426950408889634f;
     const float mxl = mx * L2E, mvl = fmaf(mv, L2E, 1.f);
+    const uint64_t l2 = f2_pack(L2E, L2E);
+    const uint64_t nx2 = f2_pack(-mxl, -mxl), nv2 = f2_pack(-mvl, -mvl);
     // width exponentials, summed per block of 8 bins (NB independent chains)
     float sB[NB];
 #pragma unroll
     for (int b = 0; b < NB; b++) sB[b] = 0.f;
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-        o[k] = vg_ex2_approx(fmaf(o[k], L2E, -mxl));
+    for (int k = 0; k < K; k += 2) {
+        f2_unpack(f2_fma(f2_pack(o[k], o[k + 1]), l2, nx2), o[k], o[k + 1]);
+        o[k] = vg_ex2_approx(o[k]);
+        o[k + 1] = vg_ex2_approx(o[k + 1]);
         sB[k >> 3] += o[k];
+        sB[k >> 3] += o[k + 1];
     }
     float stot = 0.f;
 #pragma unroll
     for (int b = 0; b < NB; b++) stot += sB[b];
     const float cw = __fdividef(c1, stot);
+    const uint64_t cw2 = f2_pack(cw, cw), ep2 = f2_pack(EPS_W, EPS_W);
 #pragma unroll
-    for (int k = 0; k < K; k++) o[k] = fmaf(cw, o[k], EPS_W);   // bin widths
+    for (int k = 0; k < K; k += 2) f2_unpack(f2_fma(cw2, f2_pack(o[k], o[k + 1]), ep2), o[k], o[k + 1]);   // bin widths
 #pragma unroll
-    for (int k = 0; k <= K; k++) o[K + k] = vg_ex2_approx(fmaf(o[K + k], L2E, -mvl));   // vertex heights / 2
+    for (int k = 0; k < K; k += 2) {   // vertex heights / 2
+        f2_unpack(f2_fma(f2_pack(o[K + k], o[K + k + 1]), l2, nv2), o[K + k], o[K + k + 1]);
+        o[K + k] = vg_ex2_approx(o[K + k]);
+        o[K + k + 1] = vg_ex2_approx(o[K + k + 1]);
+    }
+    o[2 * K] = vg_ex2_approx(fmaf(o[2 * K], L2E, -mvl));
     // per block: width EB = cw sum(exp) + 8 EPS_W, area PB = sum (u_k + u_k+1) W_k
     float EB[NB], PB[NB];
 #pragma unroll
@@ -982,22 +1033,32 @@ __device__ __forceinline__ float spline_reg(float (&o)[2 * K + 1], float x, floa
 #pragma unroll
         for (int b = 1; b < NB; b++) usel[q] = bsel == b ? o[K + 8 * b + q] : usel[q];
     }
-    float Wb = 0.f, ub = 0.f, ub1 = 0.f, Eb = 0.f, Pb = 0.f;
-    bool f = false;
+    // the block's bins: their starts, then a binary descent over these (the
+    // first bin that ends above t, the last one where none does)
+    float Eq[8], Pq[8];
 #pragma unroll
     for (int q = 0; q < 8; q++) {
         const float wq = wsel[q], sq = (usel[q] + usel[q + 1]) * wq;
-        // the last bin of the block takes t when no earlier bin did
-        const bool here = !f && (q == 7 || (DIR == 0 ? (t < E + wq) : (t < P + sq)));
-        Wb = here ? wq : Wb;
-        ub = here ? usel[q] : ub;
-        ub1 = here ? usel[q + 1] : ub1;
-        Eb = here ? E : Eb;
-        Pb = here ? P : Pb;
-        f = f || here;
+        Eq[q] = E;
+        Pq[q] = P;
         E += wq;
         P += sq;
     }
+#pragma unroll
+    for (int n = 4; n > 0; n >>= 1) {
+        const bool up = DIR == 0 ? t >= Eq[n] : t >= Pq[n];
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (q < n) {
+                wsel[q] = up ? wsel[n + q] : wsel[q];
+                Eq[q] = up ? Eq[n + q] : Eq[q];
+                Pq[q] = up ? Pq[n + q] : Pq[q];
+            }
+#pragma unroll
+        for (int q = 0; q <= 4; q++)
+            if (q <= n) usel[q] = up ? usel[n + q] : usel[q];
+    }
+    const float Wb = wsel[0], ub = usel[0], ub1 = usel[1], Eb = Eq[0], Pb = Pq[0];
     // ub, ub1 are half the vertex heights: the area of the first al of the
     // bin is Wb (al 2 ub + al^2 (ub1 - ub)), the pdf 2 ((1 - al) ub + al ub1) / Z
     float al, xo;
@@ -1029,10 +1090,14 @@ __device__ __forceinline__ void add_bias(float (&o)[2 * K + 1], const float *bb)
 #pragma unroll
     for (int q = 0; q < NR; q += 4) {
         const float4 b = *reinterpret_cast<const float4 *>(bb + q);
-        o[q] += b.x;
-        if (q + 1 < NR) o[q + 1] += b.y;
-        if (q + 2 < NR) o[q + 2] += b.z;
-        if (q + 3 < NR) o[q + 3] += b.w;
+        if (q + 3 < NR) {
+            f2_unpack(f2_add(f2_pack(o[q], o[q + 1]), f2_pack(b.x, b.y)), o[q], o[q + 1]);
+            f2_unpack(f2_add(f2_pack(o[q + 2], o[q + 3]), f2_pack(b.z, b.w)), o[q + 2], o[q + 3]);
+        } else {
+            o[q] += b.x;
+            if (q + 1 < NR) o[q + 1] += b.y;
+            if (q + 2 < NR) o[q + 2] += b.z;
+        }
     }
 }
 
@@ -1547,8 +1612,8 @@ __global__ void __launch_bounds__(UNT, 1) flow_pass_duo_kernel(FlowGeom g, const
             const int l = layer_of(step);
             const FlowLayer &y = g.ly[l];
             const int dA = y.realA ? y.dA : 1;
-            for (int i = tg; i < FH * 8; i += DUO_NT) {   // W1 padded to 8 columns: [128][8]
-                const int c = i >> 3, a = i & 7;
+            for (int i = tg; i < FH * 8; i += DUO_NT) {   // W1 transposed, padded to 8 inputs: [8][128]
+                const int c = i & (FH - 1), a = i / FH;
                 sW1[i] = a < dA ? theta[y.oW1 + c * dA + a] : 0.f;
             }
             for (int i = tg; i < FH; i += DUO_NT) {
@@ -1583,34 +1648,32 @@ __global__ void __launch_bounds__(UNT, 1) flow_pass_duo_kernel(FlowGeom g, const
                         if (grow < n) zl[((int64_t)l * n + grow) * dim + d] = Zs[rr * zst + d];
                     }
                 {   // H1 = relu(W1 z_A + b1) in FP32 -> A operand
-                    float xa[8];
+                    uint64_t xa[8];   // each input twice
 #pragma unroll
-                    for (int a = 0; a < 8; a++) xa[a] = (a < dA && y.realA) ? Zs[r * zst + y.A[a]] : 0.f;
-                    const bool wide = dA > 4;
+                    for (int a = 0; a < 8; a++) {
+                        const float v = (a < dA && y.realA) ? Zs[r * zst + y.A[a]] : 0.f;
+                        xa[a] = f2_pack(v, v);
+                    }
+                    const int na = dA > 4 ? 8 : 4;
 #pragma unroll 1
                     for (int c0 = 64 * h; c0 < 64 * h + 64; c0 += 32) {
                         uint32_t pk[16];
 #pragma unroll
-                        for (int c = 0; c < 32; c += 2) {
-                            float v[2];
+                        for (int c = 0; c < 32; c += 4) {
+                            const float4 b = *reinterpret_cast<const float4 *>(sb1 + c0 + c);
+                            uint64_t lo = f2_pack(b.x, b.y), hi = f2_pack(b.z, b.w);
 #pragma unroll
-                            for (int e = 0; e < 2; e++) {
-                                const float4 w0 = *reinterpret_cast<const float4 *>(sW1 + (c0 + c + e) * 8);
-                                float acc = sb1[c0 + c + e];
-                                acc = fmaf(w0.x, xa[0], acc);
-                                acc = fmaf(w0.y, xa[1], acc);
-                                acc = fmaf(w0.z, xa[2], acc);
-                                acc = fmaf(w0.w, xa[3], acc);
-                                if (wide) {
-                                    const float4 w1 = *reinterpret_cast<const float4 *>(sW1 + (c0 + c + e) * 8 + 4);
-                                    acc = fmaf(w1.x, xa[4], acc);
-                                    acc = fmaf(w1.y, xa[5], acc);
-                                    acc = fmaf(w1.z, xa[6], acc);
-                                    acc = fmaf(w1.w, xa[7], acc);
-                                }
-                                v[e] = fmaxf(acc, 0.f);
+                            for (int a = 0; a < 8; a++) {
+                                if (a >= 4 && a >= na) break;
+                                const float4 w = *reinterpret_cast<const float4 *>(sW1 + a * FH + c0 + c);
+                                lo = f2_fma(f2_pack(w.x, w.y), xa[a], lo);
+                                hi = f2_fma(f2_pack(w.z, w.w), xa[a], hi);
                             }
-                            pk[c >> 1] = pack_bf16(v[0], v[1]);
+                            float v0, v1;
+                            f2_unpack(lo, v0, v1);
+                            pk[c >> 1] = relu_bf16x2(pack_bf16(v0, v1));
+                            f2_unpack(hi, v0, v1);
+                            pk[(c >> 1) + 1] = relu_bf16x2(pack_bf16(v0, v1));
                         }
                         umma::tmem_st16(tA + lane_base + (uint32_t)(c0 >> 1), pk);
                     }
@@ -1633,8 +1696,11 @@ __global__ void __launch_bounds__(UNT, 1) flow_pass_duo_kernel(FlowGeom g, const
 #pragma unroll
                     for (int c = 0; c < 32; c += 4) {
                         const float4 b = *reinterpret_cast<const float4 *>(sb2 + c0 + c);
-                        pk[c >> 1] = pack_bf16(fmaxf(v[c] + b.x, 0.f), fmaxf(v[c + 1] + b.y, 0.f));
-                        pk[(c >> 1) + 1] = pack_bf16(fmaxf(v[c + 2] + b.z, 0.f), fmaxf(v[c + 3] + b.w, 0.f));
+                        float v0, v1;
+                        f2_unpack(f2_add(f2_pack(v[c], v[c + 1]), f2_pack(b.x, b.y)), v0, v1);
+                        pk[c >> 1] = relu_bf16x2(pack_bf16(v0, v1));
+                        f2_unpack(f2_add(f2_pack(v[c + 2], v[c + 3]), f2_pack(b.z, b.w)), v0, v1);
+                        pk[(c >> 1) + 1] = relu_bf16x2(pack_bf16(v0, v1));
                     }
                     umma::tmem_st16(tA + lane_base + (uint32_t)(c0 >> 1), pk);
                 }
