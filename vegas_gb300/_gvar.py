@@ -36,6 +36,9 @@ class GVar(object):
 
     @property
     def var(self):
+        if len(self._der) == 1:   # one iteration's estimate
+            (c,) = self._der.values()
+            return float(c * c)
         return float(sum(c * c for c in self._der.values()))
 
     @property
@@ -137,6 +140,8 @@ def fmt(mean, sdev):
 
 def gvar(mean, unc):
     """gvar(mean, sdev) -> GVar; gvar(mean_array, cov_matrix) -> correlated array."""
+    if type(mean) is float and type(unc) is float:
+        return GVar(mean, {next(_counter): unc})
     mean_a = np.asarray(mean, float)
     unc_a = np.asarray(unc, float)
     if mean_a.shape == ():

@@ -242,11 +242,15 @@ def ptr(t):
 
 def stream_ptr(device=None):
     import torch
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    if device is None or device.type != 'cuda' or device.index is None:
+        return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    # the raw handle without a Stream object: 0.3 us instead of 3
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(device.index))
 
 
 def i64_array(vals):
-    return (ctypes.c_int64 * len(vals))(*[int(v) for v in vals])
+    return (ctypes.c_int64 * len(vals))(*(vals.tolist() if getattr(vals, 'dtype', None) == 'int64'
+                                          else [int(v) for v in vals]))
 
 
 def dbl_array(vals):

@@ -93,9 +93,9 @@ class AdaptiveMap(object):
         return self._inc
 
     def region(self, d=-1):
-        g = self.grid
+        g = self.grid   # one copy for all directions
         if d < 0:
-            return [self.region(k) for k in range(self.dim)]
+            return [(g[k, 0], g[k, self._ninc[k]]) for k in range(self.dim)]
         return (g[d, 0], g[d, self._ninc[d]])
 
     def extract_grid(self):

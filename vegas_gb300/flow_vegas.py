@@ -165,11 +165,13 @@ class FlowIntegrator(object):
         stream = N.stream_ptr(self.device)
         it, ncap = s._struct()
         s._allocate(it)
-        n = int(s._read_stats().neval)
+        s._begin_read_stats()
         s._itn += 1
         itn_word = s._itn & 0xffffffff
-        # the iteration's device buffers are kept and reused (no allocator traffic per iteration)
+        # the iteration's device buffers are kept and reused (no allocator traffic per iteration);
+        # its points are drawn while the host reads their number
         yv, _, wgt, hc = s._points(it, ncap, itn_word, None, want_hc=train, bufs=self._bufs)
+        n = int(s._end_read_stats().neval)
         yv = yv[:n]
         yp, ld = self.flow.sample(yv, z=self._buf('yp', ncap, self.dim)[:n], ld=self._buf('ld', ncap)[:n])
         x = self._buf('xm', ncap, self.dim)[:n]

@@ -86,6 +86,7 @@ class Integrator(object):
         self._itn = 0
         self._work = None
         self._stats = None
+        self._stats_event = None
         self._sigf = None
         self.sum_sigf = HUGE
         self.nhcube = 1
@@ -129,7 +130,10 @@ class Integrator(object):
             lim = np.array(map, dtype=float)
             if lim.ndim < 2 or lim.shape[-1] != 2:
                 raise ValueError('integration limits must be [[xl, xu], ...]')
-            self.map = AdaptiveMap(lim.reshape(-1, 2), device=self.device)
+            lim = lim.reshape(-1, 2)
+            self.map = AdaptiveMap(lim, device=self.device)
+            self.xsample = 0.5 * (lim[:, 0] + lim[:, 1])   # of the limits, not of a copy from the device
+            return
         self.xsample = np.array([0.5 * (a + b) for a, b in self.map.region()])
 
     @property
@@ -235,8 +239,8 @@ class Integrator(object):
         if (3 * dim + 3) * workspace + (0 if self.minimize_mem else self.nhcube) > self.max_mem:
             raise MemoryError('work arrays larger than max_mem; reduce min_neval_batch or '
                               'max_neval_hcube (or increase max_mem)')
-        geometry = (tuple(int(v) for v in np.asarray(self.nstrat).reshape(-1)), self.nhcube,
-                    tuple(int(v) for v in np.asarray(self.map.ninc).reshape(-1)), self.neval,
+        geometry = (tuple(np.asarray(self.nstrat).reshape(-1).tolist()), self.nhcube,
+                    tuple(self.map._ninc.tolist()), self.neval,
                     self.neval_frac, self.min_neval_hcube, self.max_neval_hcube, self.precision)
         if geometry != getattr(self, '_geometry', None):
             # a new workspace (zeroed: the allocation keeps its ticket and
@@ -251,9 +255,9 @@ class Integrator(object):
         it.dim = self.dim
         it.precision = N.VG_F64 if self.precision == 'fp64' else N.VG_F32
         it.nhcube = self.nhcube
-        for d in range(self.dim):
-            it.nstrat[d] = int(self.nstrat[d])
-            it.ninc[d] = int(self.map._ninc[d])
+        dim = it.dim
+        it.nstrat[:dim] = [int(v) for v in np.asarray(self.nstrat)[:dim].tolist()]
+        it.ninc[:dim] = self.map._ninc.tolist()
         g, inc = self.map.grid_tensor, self.map.inc_tensor
         it.grid = g.data_ptr()
         it.inc = inc.data_ptr()
@@ -297,6 +301,20 @@ class Integrator(object):
     def _read_stats(self):
         b = self._stats.cpu().numpy().tobytes()
         return N.VgStats.from_buffer_copy(b)
+
+    def _begin_read_stats(self):
+        """Copies the device record to pinned host memory behind what is
+        enqueued so far; _end_read_stats waits for that copy alone, so work
+        enqueued in between runs on while the host reads the record."""
+        host = self._records_host(1)
+        host[0].copy_(self._stats, non_blocking=True)
+        if self._stats_event is None:
+            self._stats_event = torch.cuda.Event()
+        self._stats_event.record(torch.cuda.current_stream(self.device))
+
+    def _end_read_stats(self):
+        self._stats_event.synchronize()
+        return N.VgStats.from_buffer_copy(self._rec_host[0].numpy())
 
     def _allocate(self, it):
         self._put_sum_sigf()
@@ -506,6 +524,13 @@ class Integrator(object):
 
     def _reduce_array(self, it, f, fdt, w):
         """Mean and (co)variance of every component of an array integrand."""
+        s = int(f.shape[1])
+        host = self._enqueue_array(it, f, fdt, w).cpu().numpy()
+        return host[:s], host[s:].reshape(s, s)
+
+    def _enqueue_array(self, it, f, fdt, w):
+        """Mean and (co)variance of every component of an array integrand:
+        a device tensor of s + s * s values, enqueued without a wait."""
         L = N.load()
         s = int(f.shape[1])
         corr = 1 if self.correlate_integrals else 0
@@ -515,8 +540,17 @@ class Integrator(object):
         mean, var = out[:s], out[s:]
         N.check(L.vg_reduce_array(ctypes.byref(it), N.ptr(f), fdt, s, corr, N.ptr(w), N.ptr(mean),
                                   N.ptr(var), N.ptr(work), need, N.stream_ptr(self.device)))
-        host = out.cpu().numpy()   # one copy and one wait for both
-        return host[:s], host[s:].reshape(s, s)
+        return out
+
+    def _kept_points(self, it, ncap, itn_word, u, fshape):
+        """The points of an iteration for a batch integrand.  The sampler keeps
+        each sample's Jacobian and training bins, so the reduction streams
+        them instead of regenerating the samples; the weights are written only
+        while an array-valued integrand may need them."""
+        keep = self._keep_buffer(it, ncap)
+        x, yv, w, _ = self._points(it, ncap, itn_word, u, want_y=self.uses_jac,
+                                   want_w=fshape is None or bool(fshape), keep=keep)
+        return x, yv, w, keep
 
     def __call__(self, fcn, save=None, saveall=None, **kargs):
         """Integrate ``fcn``; returns an :class:`RAvg` (pyx:1912-2230)."""
@@ -552,23 +586,21 @@ class Integrator(object):
                 N.check(L.vg_fused_iteration(ctypes.byref(it), itn_word, None, int(fcn.kind),
                                              N.dbl_array(p), len(p), stream))
             else:
-                st = self._read_stats()
-                n = int(st.neval)
+                self._begin_read_stats()
+                if kind != 'builtin' and self.ran_array_generator is None:
+                    # the points of this iteration need nothing from the
+                    # host: they are drawn while it reads their number
+                    x, yv, w, keep = self._kept_points(it, ncap, itn_word, None, fshape)
+                n = int(self._end_read_stats().neval)
                 if self.ran_array_generator is not None:
                     u = self._draw_u(n)
+                    if kind != 'builtin':
+                        x, yv, w, keep = self._kept_points(it, ncap, itn_word, u, fshape)
                 if kind == 'builtin':
                     p = fcn.params(self.dim)
                     N.check(L.vg_fused_iteration(ctypes.byref(it), itn_word, N.ptr(u),
                                                  int(fcn.kind), N.dbl_array(p), len(p), stream))
                 else:
-                    # the sampler keeps each sample's Jacobian and training
-                    # bins, so the reduction streams them instead of
-                    # regenerating the samples; the weights are written only
-                    # while an array-valued integrand may need them
-                    keep = self._keep_buffer(it, ncap)
-                    want_w = fshape is None or bool(fshape)
-                    x, yv, w, _ = self._points(it, ncap, itn_word, u, want_y=self.uses_jac, want_w=want_w,
-                                               keep=keep)
                     jac = self.map.jac1d(yv[:n]) if self.uses_jac else None
                     f = None
                     nb = self._eval_batch_size()
@@ -599,16 +631,22 @@ class Integrator(object):
                     N.check(L.vg_reduce_kept(ctypes.byref(it), itn_word, N.ptr(u), N.ptr(f0), fdt, N.ptr(keep),
                                              keep.numel(), stream))
                     if f.dim() > 1:
-                        arr = self._reduce_array(it, f, fdt, w)
+                        arr = self._enqueue_array(it, f, fdt, w)
             # adapt the map on the device before reading the iteration record
             N.check(L.vg_end_iteration(ctypes.byref(it), stream))
-            st = self._read_stats()
+            if arr is not None:   # the record and the array's values on one wait
+                self._begin_read_stats()
+                arr = arr.cpu().numpy()
+                st = self._end_read_stats()
+            else:
+                st = self._read_stats()
             self._take_record(st)
             if arr is not None:
                 # array- or dictionary-valued integrand: RAvgArray of the
                 # integrand's shape / RAvgDict of its keys
                 # (VegasIntegrand.format_result, pyx:3127-3147)
-                mean_a, var_a = arr
+                s_f = int(f.shape[1])
+                mean_a, var_a = arr[:s_f], arr[s_f:].reshape(s_f, s_f)
                 if self.correlate_integrals:
                     g = gv.gvar(mean_a, var_a)
                 else:
@@ -676,18 +714,30 @@ class Integrator(object):
         nitn = int(self.nitn)
         host = self._records_host(nitn)
         rec, sz = host.data_ptr(), ctypes.sizeof(N.VgStats)   # pinned: the device writes the records there
-        for k in range(nitn):
-            self._itn += 1
-            N.check(L.vg_iterate_record(ctypes.byref(it), self._itn & 0xffffffff, int(fcn.kind), params, len(p),
-                                        rec + k * sz, stream))
-        torch.cuda.current_stream(self.device).synchronize()
-        raw = host[:nitn].numpy().tobytes()
+        cur = torch.cuda.current_stream(self.device)
         gs = []
-        for k in range(nitn):
-            st = N.VgStats.from_buffer_copy(raw, k * sz)
-            self._take_record(st)
-            gs.append(gv.gvar(st.mean, st.var ** 0.5))
-            result.sum_neval += self.last_neval
+
+        def take(k0, k1):
+            for k in range(k0, k1):
+                st = N.VgStats.from_address(rec + k * sz)
+                self._take_record(st)
+                gs.append(gv.gvar(st.mean, st.var ** 0.5))
+                result.sum_neval += self.last_neval
+
+        try:
+            for k in range(nitn):
+                self._itn += 1
+                if k > 0 and k == nitn - 1:
+                    before_last = torch.cuda.Event()
+                    before_last.record(cur)
+                N.check(L.vg_iterate_record(ctypes.byref(it), self._itn & 0xffffffff, int(fcn.kind), params, len(p),
+                                            rec + k * sz, stream))
+            if nitn > 1:   # the records before the last are read while it runs
+                before_last.synchronize()
+                take(0, nitn - 1)
+        finally:
+            cur.synchronize()
+        take(max(nitn - 1, 0), nitn)
         result.add_many(gs)
         return result
 
@@ -851,8 +901,8 @@ def strata(dim, mode, neval, neval_given, nstrat, neval_frac=0.75, beta=0.75,
                             float(neval_frac), float(beta), int(adapt_to_errors),
                             int(uniform_nstrat), float(max_mem), int(minimize_mem),
                             int(maxinc_axis), ns_out, ninc_out, ctypes.byref(mnh)))
-    return dict(neval=int(neval.value), nstrat=np.array(list(ns_out), np.int64),
-                ninc=np.array(list(ninc_out), np.int64), min_neval_hcube=int(mnh.value))
+    return dict(neval=int(neval.value), nstrat=np.array(ns_out, np.int64),
+                ninc=np.array(ninc_out, np.int64), min_neval_hcube=int(mnh.value))
 
 
 def _save(dest, obj):
