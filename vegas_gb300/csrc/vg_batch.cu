@@ -290,12 +290,28 @@ extern "C" int vg_batch_launch(const void *table, int njobs, int kind, int nitn,
         VG_CUDA_CHECK(cudaMemsetAsync(sync, 0, sizeof(unsigned int) * (size_t)njobs, st));
     }
     VG_CUDA_CHECK(cudaMemsetAsync(queue, 0, sizeof(unsigned int) * NBUCKET, st));
-    // fork: the first bucket (largest dimension first) runs on the caller's
-    // stream, the others on their own streams after it was enqueued
+    // fork: the first bucket runs on the caller's stream, the others on their
+    // own streams after it was enqueued.  Their CTAs start as SMs become free,
+    // so the bucket with the fewest integrals per CTA goes first (it ends with
+    // its longest integral, beside which little of its own is left to run) and
+    // the one with the most last, to fill up behind the others.  1024 integrals
+    // of dim 3 to 9, 285 + 591 + 148 of them in the buckets: 18.8 ms in the
+    // order of the dimensions (16, 8, 4), 14.4 so.
+    int turn[NBUCKET] = {2, 1, 0};   // ties: the larger dimension first
+    auto fewer = [&](int x, int y) {
+        if (seg[2 * x + 1] <= 0 || seg[2 * y + 1] <= 0) return seg[2 * x + 1] <= 0 && seg[2 * y + 1] > 0;
+        return (int64_t)seg[2 * x + 1] * grid[y] < (int64_t)seg[2 * y + 1] * grid[x];
+    };
+    for (int i = 1; i < NBUCKET; i++)
+        for (int k = i; k > 0 && fewer(turn[k], turn[k - 1]); k--) {
+            const int b = turn[k];
+            turn[k] = turn[k - 1];
+            turn[k - 1] = b;
+        }
     if (npresent > 1) VG_CUDA_CHECK(cudaEventRecord(aux->fork, st));
     int first = 1;
     int joined[NBUCKET] = {0, 0, 0};
-    for (int b = NBUCKET - 1; b >= 0; b--) {
+    for (int b : turn) {
         const int n = seg[2 * b + 1];
         if (n <= 0) continue;
         cudaStream_t sb = st;
