@@ -47,14 +47,32 @@ __device__ __forceinline__ double div_fast(double a, double b)
     return a * r;
 }
 
+// The threads that work on one axis: a whole CTA, or a set of GROUP_NT of its
+// threads with a barrier of their own, so that a CTA adapts several axes at once.
+struct WholeCta {
+    __device__ __forceinline__ int t() const { return threadIdx.x; }
+    __device__ __forceinline__ int n() const { return blockDim.x; }
+    __device__ __forceinline__ void sync() const { __syncthreads(); }
+};
+constexpr int GROUP_NT = 256;
+struct PartOfCta {
+    __device__ __forceinline__ int t() const { return threadIdx.x % GROUP_NT; }
+    __device__ __forceinline__ int n() const { return GROUP_NT; }
+    __device__ __forceinline__ void sync() const
+    {
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / GROUP_NT), "n"(GROUP_NT) : "memory");
+    }
+};
+
 // Block-wide inclusive prefix sum of v[0..n) in place (FP64, fixed order):
 // per-thread sequential over a contiguous chunk, then a scan of the chunk
 // totals by warp shuffles (within each warp, then over the warp totals) --
 // few FP64 instructions per thread (GB300 issues FP64 at a low rate).
-static __device__ void block_inclusive_scan(double *v, int n, double *part /* >= 32 */)
+template <typename CTA>
+static __device__ void block_inclusive_scan(const CTA cta, double *v, int n, double *part /* >= 32 */)
 {
-    const int NT = (int)blockDim.x, NW = NT >> 5;
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int NT = cta.n(), NW = NT >> 5;
+    const int t = cta.t(), lane = t & 31, w = t >> 5;
     const int per = (n + NT - 1) / NT;
     const int b = t * per, e = min(n, b + per);
     double s = 0.0;
@@ -69,7 +87,7 @@ static __device__ void block_inclusive_scan(double *v, int n, double *part /* >=
         if (lane >= off) x = __dadd_rn(x, y);
     }
     if (lane == 31) part[w] = x;
-    __syncthreads();
+    cta.sync();
     if (w == 0) {
         double z = lane < NW ? part[lane] : 0.0;
 #pragma unroll
@@ -79,53 +97,54 @@ static __device__ void block_inclusive_scan(double *v, int n, double *part /* >=
         }
         if (lane < NW) part[lane] = z;
     }
-    __syncthreads();
+    cta.sync();
     double ex = __shfl_up_sync(0xffffffffu, x, 1);   // exclusive prefix within the warp
     if (lane == 0) ex = 0.0;
     if (t > 0) {
         const double carry = (w > 0) ? __dadd_rn(part[w - 1], ex) : ex;
         for (int i = b; i < e; i++) v[i] = __dadd_rn(v[i], carry);
     }
-    __syncthreads();
+    cta.sync();
 }
 
 // Sum of v[0..n) in a fixed order; result broadcast to all threads.
-static __device__ double block_sum(const double *v, int n, double *part /* >= 33 */)
+template <typename CTA>
+static __device__ double block_sum(const CTA cta, const double *v, int n, double *part /* >= 33 */)
 {
-    const int NT = (int)blockDim.x, NW = NT >> 5;
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int NT = cta.n(), NW = NT >> 5;
+    const int t = cta.t(), lane = t & 31, w = t >> 5;
     double s = 0.0;
     for (int i = t; i < n; i += NT) s = __dadd_rn(s, v[i]);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, off));
     if (lane == 0) part[w] = s;
-    __syncthreads();
+    cta.sync();
     if (w == 0) {
         double z = lane < NW ? part[lane] : 0.0;
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) z = __dadd_rn(z, __shfl_xor_sync(0xffffffffu, z, off));
         if (lane == 0) part[32] = z;
     }
-    __syncthreads();
+    cta.sync();
     const double r = part[32];
-    __syncthreads();
+    cta.sync();
     return r;
 }
 
 // FP32 block reductions (max, sum) over the first red_nt threads; f = shared
 // scratch of >= 33 floats.  Result broadcast to all threads.
-template <bool MAX>
-__device__ float block_reduce_f(float v, float *f, int red_nt)
+template <bool MAX, typename CTA>
+__device__ float block_reduce_f(const CTA cta, float v, float *f, int red_nt)
 {
     const int NW = red_nt >> 5;
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int t = cta.t(), lane = t & 31, w = t >> 5;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
         const float o = __shfl_xor_sync(0xffffffffu, v, off);
         v = MAX ? fmaxf(v, o) : v + o;
     }
     if (lane == 0 && w < NW) f[w] = v;
-    __syncthreads();
+    cta.sync();
     if (w == 0) {
         float z = lane < NW ? f[lane] : 0.f;
 #pragma unroll
@@ -135,9 +154,9 @@ __device__ float block_reduce_f(float v, float *f, int red_nt)
         }
         if (lane == 0) f[32] = z;
     }
-    __syncthreads();
+    cta.sync();
     const float r = f[32];
-    __syncthreads();
+    cta.sync();
     return r;
 }
 
@@ -167,10 +186,11 @@ __device__ __forceinline__ double damped_weight_fast(float sf, float rmx, float 
 // (or within 1e-5 of 1) is formed and damped in FP64, so tiny weights keep
 // the reference's ((1 - v) / -ln v)^alpha.  The cumulative sums and the new
 // nodes (regrid) stay FP64.
-template <int SUM_NT>
-__device__ void adapt_weights_fast(const AdaptArgs &a, int d, int K, double *avg, double *tmp, double *part)
+template <int SUM_NT, typename CTA>
+__device__ void adapt_weights_fast(const CTA cta, const AdaptArgs &a, int d, int K, double *avg, double *tmp,
+                                   double *part)
 {
-    const int t = threadIdx.x, NT = (int)blockDim.x;
+    const int t = cta.t(), NT = cta.n();
     float *af = reinterpret_cast<float *>(tmp);   // [K] averages
     float *sf = af + K;                           // [K] smoothed (tmp holds 2K floats)
     float *pf = reinterpret_cast<float *>(part);
@@ -182,7 +202,7 @@ __device__ void adapt_weights_fast(const AdaptArgs &a, int d, int K, double *avg
             const_cast<unsigned long long *>(a.n_f)[d * a.ldi + i] = 0ull;
         }
     }
-    __syncthreads();
+    cta.sync();
     float mx = 0.f;
     for (int i = t; i < K; i += NT) {
         float v;
@@ -193,17 +213,17 @@ __device__ void adapt_weights_fast(const AdaptArgs &a, int d, int K, double *avg
         sf[i] = v;
         mx = fmaxf(mx, v);
     }
-    mx = block_reduce_f<true>(mx, pf, NT);
+    mx = block_reduce_f<true>(cta, mx, pf, NT);
     const float rmx = mx > 0.f ? 1.f / mx : 0.f;   // sum of values scaled by the max: no overflow
     float sp = 0.f;
     const int sum_nt = SUM_NT > 0 ? SUM_NT : NT;
     if (t < sum_nt)
         for (int i = t; i < K; i += sum_nt) sp += sf[i] * rmx;
-    sp = block_reduce_f<false>(sp, pf, sum_nt);
+    sp = block_reduce_f<false>(cta, sp, pf, sum_nt);
     for (int i = t; i < K; i += NT) {
         avg[i] = damped_weight_fast(sf[i], rmx, sp, a.alpha);
     }
-    __syncthreads();
+    cta.sync();
 }
 
 // One axis of AdaptiveMap.adapt.  avg (length >= max_old) holds the carried
@@ -211,16 +231,16 @@ __device__ void adapt_weights_fast(const AdaptArgs &a, int d, int K, double *avg
 // memory, max_old + 1 and max_old doubles) the axis' old nodes and
 // increments are staged there first, so new_grid / new_inc may be the grid
 // itself (adapt in place).
-template <int SUM_NT = 0>
+template <int SUM_NT = 0, typename CTA = WholeCta>
 __device__ void adapt_axis(const AdaptArgs &a, int d, double *avg, double *tmp, double *part,
-                           double *gs = nullptr, double *is = nullptr)
+                           double *gs = nullptr, double *is = nullptr, const CTA cta = CTA())
 {
     const int K = a.old_ninc[d];
     const int Kn = a.new_ninc[d];
-    const int t = threadIdx.x, NT = (int)blockDim.x;
+    const int t = cta.t(), NT = cta.n();
     const double alpha = a.alpha;
     if (alpha > 0 && K > 1 && a.fast && a.sum_f != nullptr) {
-        adapt_weights_fast<SUM_NT>(a, d, K, avg, tmp, part);
+        adapt_weights_fast<SUM_NT>(cta, a, d, K, avg, tmp, part);
     } else if (alpha != 0 && K > 1) {
         if (a.sum_f != nullptr) {
             for (int i = t; i < K; i += NT) {
@@ -236,7 +256,7 @@ __device__ void adapt_axis(const AdaptArgs &a, int d, double *avg, double *tmp, 
                     const_cast<unsigned long long *>(a.n_f)[d * a.ldi + i] = 0ull;
                 }
             }
-            __syncthreads();
+            cta.sync();
         }
         if (alpha > 0) {
             // smoothing, pyx:548-553
@@ -247,8 +267,8 @@ __device__ void adapt_axis(const AdaptArgs &a, int d, double *avg, double *tmp, 
                 else v = __dadd_rn(__dadd_rn(__dmul_rn(6., avg[i]), avg[i - 1]), avg[i + 1]);
                 tmp[i] = __dmul_rn(fabs(v), 0.125);   // == v / 8 exactly
             }
-            __syncthreads();
-            double s = block_sum(tmp, K, part);
+            cta.sync();
+            double s = block_sum(cta, tmp, K, part);
             // normalise + damp, pyx:554-562
             const double rs = (s > 0) ? 1.0 / s : 0.0;
             for (int i = t; i < K; i += NT) {
@@ -262,7 +282,7 @@ __device__ void adapt_axis(const AdaptArgs &a, int d, double *avg, double *tmp, 
                 }
                 avg[i] = v;
             }
-            __syncthreads();
+            cta.sync();
         }
     }
     // regrid, pyx:563-587: new node i sits where the running sum of avg_f
@@ -278,12 +298,12 @@ __device__ void adapt_axis(const AdaptArgs &a, int d, double *avg, double *tmp, 
         }
     }
     if (gs != nullptr && t == 0) gs[K] = gd[K];
-    __syncthreads();
+    cta.sync();
     if (gs != nullptr) {
         gd = gs;
         id = is;
     }
-    block_inclusive_scan(P, K, part);
+    block_inclusive_scan(cta, P, K, part);
     const double total = P[K - 1];
     const double f_ninc = a.fast ? div_fast(total, (double)Kn) : __ddiv_rn(total, (double)Kn);
     double *ng = a.new_grid + d * a.ldg_new;
@@ -309,10 +329,10 @@ __device__ void adapt_axis(const AdaptArgs &a, int d, double *avg, double *tmp, 
         }
         ng[i] = v;
     }
-    __syncthreads();
+    cta.sync();
     double *ni = a.new_inc + d * a.ldi_new;
     for (int i = t; i < Kn; i += NT) ni[i] = __dsub_rn(ng[i + 1], ng[i]);
-    __syncthreads();
+    cta.sync();
 }
 
 // ----------------------------------------------------------- cluster form

@@ -224,7 +224,13 @@ extern "C" int vg_batch_prepare(const vg_integrator *its, int njobs, int kind, c
             ad.max_old = max_old;
             ad.sequential = 1;
             ad.fast = f64 ? 0 : 1;
-            const size_t an = sizeof(double) * (2 * (size_t)max_old + 64);
+            // an axis per 256 threads at a time, fewer where the maps are so fine
+            // that their scratch would not fit
+            const size_t one = sizeof(double) * adapt_group_doubles(max_old);
+            int axes = C.ntb / vgadapt::GROUP_NT;
+            while (axes > 1 && one * axes > budget) axes--;
+            if (J.adapt) J.adapt = axes;
+            const size_t an = one * axes;
             need = an > need ? an : need;
         }
         J.out = out + (size_t)j * 3 * nitn;

@@ -24,7 +24,7 @@ struct BatchJob {
     double *res;                 // [4] weighted mean, sdev, chi2, dof
     unsigned int *sync;          // group barrier counter (group mode)
     int bucket;                  // dimension bucket: 0 (dim <= 4), 1 (<= 8), 2 (<= 16)
-    int adapt;                   // adapt the map after each iteration
+    int adapt;                   // adapt the map after each iteration: axes at a time (0: not)
     unsigned long long *stamp;   // instrumentation (or nullptr): [0] start, [1] end (globaltimer ns), [2] SM
 };
 
@@ -71,6 +71,9 @@ __device__ __forceinline__ bool group_barrier(unsigned int *ctr, unsigned int ta
     __syncthreads();
     return s_ok != 0;
 }
+
+// Shared memory of an axis' adaptation: weights, cumulative sums, partial sums.
+__host__ __device__ constexpr size_t adapt_group_doubles(int max_old) { return 2 * (size_t)max_old + 64; }
 
 constexpr int APER = 4;          // hypercubes per thread and pass of the allocation
 constexpr int F64_S = 2;         // samples per thread of the FP64 tiles
@@ -257,18 +260,27 @@ static __device__ __noinline__ void cta_finalize_f64(const IterArgs &a, int ngro
     __syncthreads();
 }
 
-// End of iteration: adapt the map (one axis after another), copy the new
-// grid back, clear the training histogram (vg_end_iteration's work).
+// End of iteration: adapt the map, copy the new grid back, clear the training
+// histogram (vg_end_iteration's work).  An axis is a chain of FP64 sums, scans
+// and searches, bound by their latency with 256 threads as with 1024, so the
+// CTA adapts an axis per 256 threads at a time.  (Only an axis of a single
+// increment would use the weights that pyx:533 carries from axis to axis, and
+// its nodes are fixed.)
 static __device__ __noinline__ void cta_adapt(const BatchJob &J, const IterArgs &a, unsigned char *smem)
 {
     const int tid = threadIdx.x, NTB = (int)blockDim.x;
     const vgadapt::AdaptArgs &ad = J.ad;
-    double *avg = (double *)smem;
-    double *tmp = avg + ad.max_old;
-    double *part = tmp + ad.max_old;
-    for (int i = tid; i < ad.max_old; i += NTB) avg[i] = 1.0;
-    __syncthreads();
-    for (int d = 0; d < ad.dim; d++) vgadapt::adapt_axis<256>(ad, d, avg, tmp, part);
+    const int ng = J.adapt, grp = tid / vgadapt::GROUP_NT;
+    if (grp < ng) {
+        double *avg = (double *)smem + (size_t)grp * adapt_group_doubles(ad.max_old);
+        double *tmp = avg + ad.max_old;
+        double *part = tmp + ad.max_old;
+        const vgadapt::PartOfCta part_of_cta;
+        for (int i = part_of_cta.t(); i < ad.max_old; i += vgadapt::GROUP_NT) avg[i] = 1.0;
+        part_of_cta.sync();
+        for (int d = grp; d < ad.dim; d += ng)
+            vgadapt::adapt_axis<vgadapt::GROUP_NT>(ad, d, avg, tmp, part, nullptr, nullptr, part_of_cta);
+    }
     __syncthreads();
     for (int d = 0; d < ad.dim; d++) {
         const int K = ad.old_ninc[d];
