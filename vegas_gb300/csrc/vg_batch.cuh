@@ -82,10 +82,21 @@ constexpr int F64_S = 2;         // samples per thread of the FP64 tiles
 // (its warps then stay together in the sample order), four in a group of CTAs.
 __device__ __forceinline__ int deal_chunks(int G) { return G > 1 ? 4 : 1; }
 
+// The arguments of the CTA's integral.  The functions that are not inlined into
+// the kernel name this variable and the dynamic shared memory themselves: through
+// a pointer parameter every access to the arguments, the grid table and the
+// histogram would be a generic one (the 16-dimensional lattice: 5.51 ms, 5.23 so).
+__device__ __forceinline__ IterArgs &job_args()
+{
+    __shared__ IterArgs sa;
+    return sa;
+}
+
 // Allocation of one iteration by one CTA: neval_h, offsets, tile heads,
 // totals in the integral's stats (the three allocation kernels' work).
-static __device__ __noinline__ void cta_alloc(const IterArgs &a, int64_t *scan /* one per warp */)
+static __device__ __noinline__ void cta_alloc(int64_t *scan /* one per warp */)
 {
+    const IterArgs &a = job_args();
     const int tid = threadIdx.x, NTB = (int)blockDim.x;
     build_tablef(a, tid, NTB);   // the FP32 grid table of this iteration
     vg_stats *st = a.stats;
@@ -158,8 +169,9 @@ static __device__ __noinline__ void cta_alloc(const IterArgs &a, int64_t *scan /
 // CTAs plus the Chan et al. merge of every hypercube cut by the ends of the
 // warps' ranges (the finalize kernels' work); sum_sigf and the constant-integrand
 // reset (pyx:2209-2215).
-static __device__ __noinline__ void cta_finalize(const IterArgs &a, int ngroup, int *flag)
+static __device__ __noinline__ void cta_finalize(int ngroup, int *flag)
 {
+    const IterArgs &a = job_args();
     const int tid = threadIdx.x, NTB = (int)blockDim.x;
     vg_stats *st = a.stats;
     float s6[6];
@@ -266,8 +278,10 @@ static __device__ __noinline__ void cta_finalize_f64(const IterArgs &a, int ngro
 // CTA adapts an axis per 256 threads at a time.  (Only an axis of a single
 // increment would use the weights that pyx:533 carries from axis to axis, and
 // its nodes are fixed.)
-static __device__ __noinline__ void cta_adapt(const BatchJob &J, const IterArgs &a, unsigned char *smem)
+static __device__ __noinline__ void cta_adapt(const BatchJob &J)
 {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const IterArgs &a = job_args();
     const int tid = threadIdx.x, NTB = (int)blockDim.x;
     const vgadapt::AdaptArgs &ad = J.ad;
     const int ng = J.adapt, grp = tid / vgadapt::GROUP_NT;
@@ -325,31 +339,32 @@ static __device__ __noinline__ void cta_ravg(const BatchJob &J, int nitn, int nw
 
 // The fused body of one integral, compiled for its dimension.
 template <int KIND, int DIM, int F>
-static __device__ __noinline__ void cta_range(const IterArgs &a, const VgParams &prm, unsigned char *smem, int rank,
-                                              int G)
+static __device__ __noinline__ void cta_range(const VgParams &prm, int rank, int G)
 {
-    range_body<MODE_FUSED, KIND, DIM, F>(a, prm, smem, rank, G, deal_chunks(G));
+    extern __shared__ __align__(16) unsigned char smem[];
+    range_body<MODE_FUSED, KIND, DIM, F>(job_args(), prm, smem, rank, G, deal_chunks(G));
 }
 
 template <int KIND, int DIMB>
-__device__ __forceinline__ void range_dispatch(const IterArgs &a, const VgParams &prm, unsigned char *smem, int rank,
-                                               int G)
+__device__ __forceinline__ void range_dispatch(const VgParams &prm, int rank, int G)
 {
+    const IterArgs &a = job_args();
     constexpr int ET = RF_EXACT | RF_TABLE;
-    if (a.wide || (a.train && !a.hist_smem) || (DIMB <= 8 && !a.table_smem)) return cta_range<KIND, DIMB, RF_GENERAL>(a, prm, smem, rank, G);
+    if (a.wide || (a.train && !a.hist_smem) || (DIMB <= 8 && !a.table_smem))
+        return cta_range<KIND, DIMB, RF_GENERAL>(prm, rank, G);
     if constexpr (DIMB == 4) {
-        if (a.dim == 4) cta_range<KIND, 4, ET>(a, prm, smem, rank, G);
-        else if (a.dim == 3) cta_range<KIND, 3, ET>(a, prm, smem, rank, G);
-        else if (a.dim == 2) cta_range<KIND, 2, ET>(a, prm, smem, rank, G);
-        else cta_range<KIND, 1, ET>(a, prm, smem, rank, G);
+        if (a.dim == 4) cta_range<KIND, 4, ET>(prm, rank, G);
+        else if (a.dim == 3) cta_range<KIND, 3, ET>(prm, rank, G);
+        else if (a.dim == 2) cta_range<KIND, 2, ET>(prm, rank, G);
+        else cta_range<KIND, 1, ET>(prm, rank, G);
     } else if constexpr (DIMB == 8) {
-        if (a.dim == 8) cta_range<KIND, 8, ET>(a, prm, smem, rank, G);
-        else if (a.dim == 7) cta_range<KIND, 7, ET>(a, prm, smem, rank, G);
-        else if (a.dim == 6) cta_range<KIND, 6, ET>(a, prm, smem, rank, G);
-        else cta_range<KIND, 5, ET>(a, prm, smem, rank, G);
+        if (a.dim == 8) cta_range<KIND, 8, ET>(prm, rank, G);
+        else if (a.dim == 7) cta_range<KIND, 7, ET>(prm, rank, G);
+        else if (a.dim == 6) cta_range<KIND, 6, ET>(prm, rank, G);
+        else cta_range<KIND, 5, ET>(prm, rank, G);
     } else {
-        if (a.table_smem) cta_range<KIND, DIMB, RF_TABLE>(a, prm, smem, rank, G);
-        else cta_range<KIND, DIMB, 0>(a, prm, smem, rank, G);
+        if (a.table_smem) cta_range<KIND, DIMB, RF_TABLE>(prm, rank, G);
+        else cta_range<KIND, DIMB, 0>(prm, rank, G);
     }
 }
 
@@ -371,7 +386,7 @@ __global__ void __launch_bounds__(MAXT, 1) batch_kernel(const BatchJob *__restri
                                                    int group, int *status)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ IterArgs sa;
+    IterArgs &sa = job_args();
     __shared__ int64_t scan[MAXT / 32];
     __shared__ VgKSum red[3 * (MAXT / 32)];
     __shared__ int s_q, s_flag;
@@ -410,25 +425,25 @@ __global__ void __launch_bounds__(MAXT, 1) batch_kernel(const BatchJob *__restri
         for (int it = 0; it < nitn && ok; it++) {
             if (tid == 0) sa.itn = itn0 + (uint32_t)it;
             __syncthreads();
-            if (rank == 0) cta_alloc(sa, scan);
+            if (rank == 0) cta_alloc(scan);
             if (G > 1 && !(ok = group_barrier(J.sync, (unsigned)G * ++rounds, sa.wait_iters))) break;
             if (sa.stats->ntiles > 0) {
                 if constexpr (sizeof(T) == 8)
                     tile_body<MODE_FUSED, KIND, DIMB, F64_S, MAXT>(sa, params[j], smem, rank, G, rank);
                 else
-                    range_dispatch<KIND, DIMB>(sa, params[j], smem, rank, G);
+                    range_dispatch<KIND, DIMB>(params[j], rank, G);
             }
             __syncthreads();
             if (G > 1 && !(ok = group_barrier(J.sync, (unsigned)G * ++rounds, sa.wait_iters))) break;
             if (rank == 0) {
                 if constexpr (sizeof(T) == 8) cta_finalize_f64(sa, G, red, &s_flag);
-                else cta_finalize(sa, G, &s_flag);
+                else cta_finalize(G, &s_flag);
                 if (tid == 0) {
                     J.out[3 * it] = sa.stats->mean;
                     J.out[3 * it + 1] = sa.stats->var;
                     J.out[3 * it + 2] = (double)sa.stats->neval;
                 }
-                if (J.adapt) cta_adapt(J, sa, smem);
+                if (J.adapt) cta_adapt(J);
             }
             __syncthreads();
         }

@@ -28,6 +28,8 @@
 // threads and its block-wide scans), and the loops are not unrolled over a
 // thread's samples, so the code fits the instruction cache.
 #pragma once
+#include <atomic>
+
 #include "vg_tile.cuh"
 
 namespace vg {
@@ -471,6 +473,10 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
             int before = 0;   // hypercube starts in the words before
 #pragma unroll 1
             for (int k = 0; k < CHUNK / 32; k++) {
+                // d * W formed anew for each sample: as loop invariants the axes'
+                // offsets into table and histogram take 20 registers, spilled
+                int Wk = W;
+                asm volatile("" : "+r"(Wk));
                 const int li = 32 * k + lane;
                 const unsigned int m = wb.mask[k];
                 const int cur = before + __popc(m & (0xffffffffu >> (31 - lane)));
@@ -495,6 +501,12 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
                             } else {
                                 VgUniform<float>::group(a.seed, a.stream, a.itn, (uint64_t)ig, g, u);
                             }
+                            // in the batched kernel the arguments are in shared memory:
+                            // not loaded ahead for all axes, to be spilled (beside 223 KB
+                            // of shared memory L1 holds few of 1024 threads' spills; with
+                            // the d * W above, dim 5 to 8: 7.22 -> 6.55 ms of the bucket,
+                            // dim 3 and 4: 6.66 -> 5.64)
+                            if (!(F & RF_CHAIN)) asm volatile("" ::: "memory");
 #pragma unroll
                             for (int q = 0; q < 4; q++) {
                                 const int d = 4 * g + q;
@@ -518,7 +530,7 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
                                 // y <= 1 (below 2^24 strata the product y0 + u = nstrat times 1 / nstrat
                                 // rounds to 1 at most), so iy <= ninc, and at y = 1 the table's last entry
                                 // has x and dy = 0
-                                const float2 e = table_smem ? table[d * W + iy] : __ldg(a.tablef + d * W + iy);
+                                const float2 e = table_smem ? table[d * Wk + iy] : __ldg(a.tablef + d * Wk + iy);
                                 float dy = yn - yfl;
                                 if (wide && iy >= ax.ninc) dy = 0.f;
                                 if (NEED_X) x[d] = fmaf(e.y, dy, e.x);
@@ -543,6 +555,7 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
                             }
                         }
                     }
+                    if (!(F & RF_CHAIN)) asm volatile("" ::: "memory");
                     // weight, pyx:1748-1749: jac *= dv_y / neval_hcube
                     const float wg = jac * win_w[cur];
                     if (MODE == MODE_POINTS) {
@@ -586,8 +599,8 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
                                     if (d >= dim) break;
                                     const unsigned int bin = (d & 1) ? bins[d >> 1] >> 16 : bins[d >> 1] & 0xffffu;
                                     if (!GENERAL || a.hist_smem) {
-                                        atomicAdd(my_hsum + d * W + bin, fd);
-                                        atomicAdd(hcnt + d * W + bin, 1u);
+                                        atomicAdd(my_hsum + d * Wk + bin, fd);
+                                        atomicAdd(hcnt + d * Wk + bin, 1u);
                                     } else if (bin < (unsigned int)a.ax[d].ninc) {
                                         atomicAdd(&a.sum_f[d * a.ldi + bin], (double)fd);
                                         atomicAdd(&a.n_f[d * a.ldi + bin], 1ull);
@@ -876,10 +889,13 @@ int launch_range_as(IterArgs &a, const VgParams *prm, size_t smem, cudaStream_t 
 {
     constexpr int NTB = range_threads(DIMB);
     auto kern = range_kernel<MODE, KIND, DIMB, F>;
-    static bool attr = false;   // once per kernel: always the largest
-    if (!attr) {
+    static std::atomic<uint64_t> attr{0};   // devices where it is set: once per kernel, always the largest
+    int dev = 0;
+    VG_CUDA_CHECK(cudaGetDevice(&dev));
+    const uint64_t bit = 1ull << (dev & 63);
+    if (!(attr.load(std::memory_order_relaxed) & bit)) {
         VG_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RANGE_SMEM));
-        attr = true;
+        if (dev < 64) attr.fetch_or(bit, std::memory_order_relaxed);
     }
     // one CTA per SM, fewer where there are fewer chunks
     int64_t grid = vg_num_sms();
