@@ -107,7 +107,18 @@ static __device__ __noinline__ void cta_alloc(int64_t *scan /* one per warp */)
     const int64_t mx = a.max_neval_hcube > a.min_neval_hcube ? a.max_neval_hcube : a.min_neval_hcube;
     const int64_t avg = (int64_t)((double)a.neval / (double)a.H);
     int64_t run = 0, mxn = 0;
-    for (int64_t base = 0; base < a.H; base += (int64_t)NTB * APER) {
+    if (!a.adaptive_alloc) {   // as many in every hypercube: offsets are products
+        for (int64_t h = tid; h < a.H; h += NTB) {
+            const int64_t off = h * avg;
+            a.neval_h[h] = (int32_t)avg;
+            a.offsets[h] = off;
+            for (int64_t tt = (off + BASE_TILE - 1) / BASE_TILE; tt * BASE_TILE < off + avg; tt++)
+                if (tt < a.ntiles_cap) a.tile_h0[tt] = h;
+        }
+        run = a.H * avg;
+        __syncthreads();   // the sentinel below comes after the tiles
+    }
+    for (int64_t base = a.adaptive_alloc ? 0 : a.H; base < a.H; base += (int64_t)NTB * APER) {
         int64_t loc[APER];
         int64_t s = 0;
 #pragma unroll
@@ -115,12 +126,8 @@ static __device__ __noinline__ void cta_alloc(int64_t *scan /* one per warp */)
             const int64_t h = base + (int64_t)tid * APER + k;
             int64_t n = 0;
             if (h < a.H) {
-                if (a.adaptive_alloc) {
-                    n = (int64_t)__dmul_rn(a.sigf[h], nsf) + a.min_neval_hcube;
-                    if (n > mx) n = mx;
-                } else {
-                    n = avg;
-                }
+                n = (int64_t)__dmul_rn(a.sigf[h], nsf) + a.min_neval_hcube;
+                if (n > mx) n = mx;
                 mxn = n > mxn ? n : mxn;
             }
             loc[k] = n;
@@ -141,7 +148,7 @@ static __device__ __noinline__ void cta_alloc(int64_t *scan /* one per warp */)
         }
         run += total;
     }
-    mxn = block_max(mxn, scan);
+    if (a.adaptive_alloc) mxn = block_max(mxn, scan);
     if (tid == 0) {
         const int64_t N = run;
         int64_t ntiles = (N + BASE_TILE - 1) / BASE_TILE;

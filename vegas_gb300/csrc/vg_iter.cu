@@ -71,24 +71,76 @@ __device__ __forceinline__ void st_release_u64(unsigned long long *p, unsigned l
     asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
+// The iteration's totals, by the thread that has them.
+__device__ __forceinline__ void alloc_totals(const IterArgs &a, int64_t N, int64_t mxn, unsigned int err)
+{
+    vg_stats *st = a.stats;
+    st->neval = N;
+    // neval_hcube_range starts at [mnh, mnh] and every count is >= mnh
+    // (pyx:1681, 1701-1704)
+    st->range_lo = a.min_neval_hcube;
+    st->range_hi = a.adaptive_alloc ? (mxn > a.min_neval_hcube ? mxn : a.min_neval_hcube) : a.min_neval_hcube;
+    int64_t ntiles = (N + BASE_TILE - 1) / BASE_TILE;
+    if (err) {
+        st->status = VG_ERR_TIMEOUT;
+        ntiles = 0;
+    } else if (N > a.ncap || ntiles + 1 > a.ntiles_cap) {
+        st->status = VG_ERR_MEMORY;
+        ntiles = 0;
+    } else {
+        st->status = VG_OK;
+        a.tile_h0[ntiles] = a.H;   // sentinel
+    }
+    a.offsets[a.H] = N;
+    st->ntiles = ntiles;
+    st->nan_seen = 0;
+    *a.counter = 0ull;
+    *a.fin_counter = 0u;
+}
+
+// offsets[h] and the tiles whose first sample falls in [run, run + n).
+__device__ __forceinline__ void place_hcube(const IterArgs &a, int64_t h, int64_t run, int64_t n)
+{
+    a.offsets[h] = run;
+    for (int64_t tt = (run + BASE_TILE - 1) / BASE_TILE; tt * BASE_TILE < run + n && tt < a.ntiles_cap; tt++)
+        a.tile_h0[tt] = h;
+}
+
 __global__ void __launch_bounds__(ALLOC_NT) alloc_kernel(const __grid_constant__ IterArgs a, int64_t nblk, int build_table)
 {
-    __shared__ int64_t wtot[ALLOC_NT / 32];
+    __shared__ int64_t wtot[ALLOC_NT / 32], wmax[ALLOC_NT / 32];
     __shared__ double s_nsf;
-    __shared__ int64_t s_avg, s_prefix;
+    __shared__ int64_t s_prefix;
     __shared__ unsigned int s_b, s_epoch;
     AllocSync *sy = reinterpret_cast<AllocSync *>(a.alloc_sync);
     unsigned long long *flags = reinterpret_cast<unsigned long long *>(a.bsum);
     const int t = threadIdx.x;
     vg_pdl_wait();
     vg_pdl_go();
+    if (!a.adaptive_alloc) {
+        // as many in every hypercube: offsets are products, and no block has to
+        // know of another (2e5 evaluations of dim 6, 85 blocks:
+        // an iteration of 39 us became one of 35)
+        const int64_t n = (int64_t)((double)a.neval / (double)a.H);
+        if (build_table)
+            build_tablef(a, (int64_t)blockIdx.x * ALLOC_NT + t, (int64_t)gridDim.x * ALLOC_NT);
+        for (int k = 0; k < ALLOC_PER; k++) {
+            const int64_t h = ((int64_t)blockIdx.x * ALLOC_PER + k) * ALLOC_NT + t;
+            if (h >= a.H) break;
+            a.neval_h[h] = (int32_t)n;
+            place_hcube(a, h, h * n, n);
+        }
+        if (blockIdx.x == 0 && t == 0) {
+            a.stats->neval_sigf = 0.0;
+            alloc_totals(a, a.H * n, n, 0u);
+        }
+        return;
+    }
     if (t == 0) {
         s_b = atomicAdd(&sy->ticket, 1u);
         s_epoch = *(volatile unsigned int *)&sy->epoch;
         const double sum_sigf = a.stats->sum_sigf;
-        s_nsf = (a.adaptive_alloc && sum_sigf > 0) ? __ddiv_rn(__dmul_rn(a.neval_frac, (double)a.neval), sum_sigf)
-                                                 : 0.0;
-        s_avg = (int64_t)((double)a.neval / (double)a.H);
+        s_nsf = sum_sigf > 0 ? __ddiv_rn(__dmul_rn(a.neval_frac, (double)a.neval), sum_sigf) : 0.0;
         if (s_b == 0) a.stats->neval_sigf = s_nsf;
     }
     if (build_table)
@@ -97,7 +149,6 @@ __global__ void __launch_bounds__(ALLOC_NT) alloc_kernel(const __grid_constant__
     const int64_t b = (int64_t)(s_b % (unsigned int)nblk);
     const unsigned int epoch = s_epoch;
     const double nsf = s_nsf;
-    const int64_t avg = s_avg;
     const int64_t mx = a.max_neval_hcube > a.min_neval_hcube ? a.max_neval_hcube : a.min_neval_hcube;
     // counts of this thread's ALLOC_PER consecutive hypercubes
     const int64_t h0 = (b * ALLOC_NT + t) * ALLOC_PER;
@@ -108,12 +159,8 @@ __global__ void __launch_bounds__(ALLOC_NT) alloc_kernel(const __grid_constant__
         const int64_t h = h0 + k;
         int64_t n = 0;
         if (h < a.H) {
-            if (a.adaptive_alloc) {
-                n = (int64_t)__dmul_rn(a.sigf[h], nsf) + a.min_neval_hcube;
-                if (n > mx) n = mx;
-            } else {
-                n = avg;
-            }
+            n = (int64_t)__dmul_rn(a.sigf[h], nsf) + a.min_neval_hcube;
+            if (n > mx) n = mx;
         }
         loc[k] = n;
         sum += n;
@@ -126,14 +173,33 @@ __global__ void __launch_bounds__(ALLOC_NT) alloc_kernel(const __grid_constant__
         for (int k = 0; k < ALLOC_PER; k++)
             if (h0 + k < a.H) a.neval_h[h0 + k] = (int32_t)loc[k];
     }
-    int64_t tot;
-    int64_t run = block_excl_scan(sum, wtot, &tot);
-    const int64_t bm = block_max(m, wtot);
+    // the block's exclusive scan and maximum, with one barrier
+    const int lane = t & 31, warp = t >> 5;
+    int64_t run = sum;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int64_t y = __shfl_up_sync(0xffffffffu, run, off);
+        if (lane >= off) run += y;
+        const int64_t z = __shfl_xor_sync(0xffffffffu, m, off);
+        m = z > m ? z : m;
+    }
+    if (lane == 31) {
+        wtot[warp] = run;
+        wmax[warp] = m;
+    }
+    run -= sum;
+    __syncthreads();
+    int64_t tot = 0, bm = 0;
+#pragma unroll
+    for (int w = 0; w < ALLOC_NT / 32; w++) {
+        if (w == warp) run += tot;
+        tot += wtot[w];
+        bm = wmax[w] > bm ? wmax[w] : bm;
+    }
     // warp 0: publish the block total, then look back 32 predecessors at a
     // time (each lane waits for one published word; the nearest inclusive
     // prefix ends the walk)
     if (t < 32) {
-        const int lane = t;
         if (lane == 0) {
             atomicMax(&sy->maxacc, (unsigned long long)bm);
             __threadfence();
@@ -183,40 +249,13 @@ __global__ void __launch_bounds__(ALLOC_NT) alloc_kernel(const __grid_constant__
     for (int k = 0; k < ALLOC_PER; k++) {
         const int64_t h = h0 + k;
         if (h >= a.H) break;
-        a.offsets[h] = run;
-        // tiles whose first sample falls in [run, run + n)
-        const int64_t n = loc[k];
-        for (int64_t tt = (run + BASE_TILE - 1) / BASE_TILE; tt * BASE_TILE < run + n && tt < a.ntiles_cap; tt++)
-            a.tile_h0[tt] = h;
-        run += n;
+        place_hcube(a, h, run, loc[k]);
+        run += loc[k];
     }
     if (b == nblk - 1 && t == 0) {   // every other block has published: totals, reset
         __threadfence();
-        const int64_t N = s_prefix + tot;
-        const int64_t mxn = (int64_t)*(volatile unsigned long long *)&sy->maxacc;
-        const unsigned int err = *(volatile unsigned int *)&sy->err;
-        vg_stats *st = a.stats;
-        st->neval = N;
-        // neval_hcube_range starts at [mnh, mnh] and every count is >= mnh
-        // (pyx:1681, 1701-1704)
-        st->range_lo = a.min_neval_hcube;
-        st->range_hi = a.adaptive_alloc ? (mxn > a.min_neval_hcube ? mxn : a.min_neval_hcube) : a.min_neval_hcube;
-        int64_t ntiles = (N + BASE_TILE - 1) / BASE_TILE;
-        if (err) {
-            st->status = VG_ERR_TIMEOUT;
-            ntiles = 0;
-        } else if (N > a.ncap || ntiles + 1 > a.ntiles_cap) {
-            st->status = VG_ERR_MEMORY;
-            ntiles = 0;
-        } else {
-            st->status = VG_OK;
-            a.tile_h0[ntiles] = a.H;   // sentinel
-        }
-        a.offsets[a.H] = N;
-        st->ntiles = ntiles;
-        st->nan_seen = 0;
-        *a.counter = 0ull;
-        *a.fin_counter = 0u;
+        alloc_totals(a, s_prefix + tot, (int64_t)*(volatile unsigned long long *)&sy->maxacc,
+                     *(volatile unsigned int *)&sy->err);
         sy->maxacc = 0ull;
         sy->err = 0u;
         sy->epoch = epoch + 1u;
