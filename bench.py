@@ -278,12 +278,12 @@ def dropin_line(dev, neval=10 ** 7, nitn=5, reps=5):
             'traffic_source': 'dram__bytes_read.sum + dram__bytes_write.sum per launch (ncu, '
                               'bench.py --device-loop-only --case dropin, about 9.3e6 evaluations)',
             'sample_kernel': {'bytes_per_eval': b_s, 'achieved': b_s * n / t_s / 1e9,
-                              'frac': b_s * n / t_s / 1e9 / hbm, 'traffic': 227.2e6,
+                              'frac': b_s * n / t_s / 1e9 / hbm, 'traffic': 224.0e6,
                               'writes': 'x (FP32, 4 dim B), Jacobian (4 B), training bins (2 dim B)'},
             'reduce_kernel': {'bytes_per_eval': b_r, 'achieved': b_r * n / t_r / 1e9,
-                              'frac': b_r * n / t_r / 1e9 / hbm, 'traffic': 179.3e6,
+                              'frac': b_r * n / t_r / 1e9 / hbm, 'traffic': 182.7e6,
                               'reads': 'f (4 B), Jacobian (4 B), training bins (2 dim B); forms the '
-                                       'two-pass hypercube sums and the training histogram'}},
+                                       'hypercube sums and the training histogram'}},
     }
 
 
@@ -753,14 +753,14 @@ def gpu_arm(args):
                 'per_call': {'value': e2e_call, 'unit': 'evals/s',
                              'call': '%d calls Integrator(f, nitn=1), host round trip each'
                                      % args.steps}},
-        # per timed step: allocation, fused tile kernel, finalize, adapt
-        'gpu_launches': 4 * args.steps,
+        # per timed step: allocation, fused iteration kernel, finalize + adapt
+        'gpu_launches': 3 * args.steps,
         'roofline': {'bound': 'issue (model)', 'achieved': model_rate / 1e12, 'peak': issue_peak / 1e12,
                      'unit': 'T thread-instr/s', 'frac': model_rate / issue_peak,
-                     'traffic': 1.70e6,
+                     'traffic': 3.41e6,
                      'traffic_source': 'dram__bytes_read.sum + dram__bytes_write.sum of one fused '
-                                       'tile_kernel launch (ncu, bench.py --device-loop-only)',
-                     'kernel': 'ridge iteration: fused tile_kernel (evaluate + reduce) + finalize '
+                                       'range_kernel launch (ncu, bench.py --device-loop-only)',
+                     'kernel': 'ridge iteration: fused range_kernel (evaluate + reduce) + finalize '
                                '(CUDA events on the launching stream, median over the timed steps)',
                      'algorithmic': 'thread instructions per evaluation from op counts (ridge_issue_model) '
                                     'x %d evaluations per launch' % neval_step,

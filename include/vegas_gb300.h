@@ -369,8 +369,8 @@ int vg_weight_points(int64_t n, const float *f, const float *jac, const float *l
  * nparams[j] values) -- run nitn iterations each in one persistent kernel
  * per dimension bucket (bucket 0: dim <= 4, 1: dim <= 8, 2: dim <= 16),
  * the buckets' kernels on forked streams joined back into `stream`.
- * cfg[3] picks each bucket's tile configuration (0 .. vg_batch_variants()-1:
- * samples per thread and CTAs per SM); vg_batch_prepare copies the job table
+ * cfg[3] picks each bucket's configuration (0 .. vg_batch_variants()-1:
+ * threads per CTA and CTAs per SM); vg_batch_prepare copies the job table
  * (vg_batch_table_bytes) to the device and returns each bucket's dynamic
  * shared memory smem[3] and co-resident grid grid[3] (0 for a bucket
  * without integrals).  Queue mode (group[b] <= 1): one CTA per integral at a
@@ -431,15 +431,14 @@ int vg_set_wait_budget(int64_t iters);
  * that reads it back. */
 int vg_set_eval_split(int policy);
 
-/* Tuning of the tile kernels: samples per thread of the fused FP32 ridge for
- * dim <= 4 (0 automatic = 2, four CTAs per SM; or 4); grid table and
- * training histogram in shared memory (-1 automatic, 0 off, 1 on where it
- * fits). */
+/* Tuning of the iteration kernels: grid table and training histogram in
+ * shared memory (-1 automatic, 0 off, 1 on where it fits).  s_dim4 (0, 2 or
+ * 4) was the samples per thread of an earlier FP32 kernel; it is checked and
+ * has no effect. */
 int vg_set_tile_tuning(int s_dim4, int table_smem, int hist_smem);
 
-/* Tuning of the drop-in path's FP32 kernels at dim <= 4: samples per thread
- * of vg_sample / vg_sample_keep (0 automatic, or 2, 4, 8) and of
- * vg_reduce_kept (0 automatic, or 2, 4). */
+/* Samples per thread of earlier FP32 kernels of the drop-in path (s_points 0,
+ * 2, 4 or 8; s_reduce 0, 2 or 4): checked, without effect. */
 int vg_set_dropin_tuning(int s_points, int s_reduce);
 
 /* ------------------------------------------------------------- probes */

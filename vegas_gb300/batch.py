@@ -7,8 +7,8 @@ their sigf, training histogram, iteration record) -- in a few device arenas,
 and runs ``nitn`` vegas+ iterations of all of them in one kernel
 (``vg_batch_launch``: one persistent kernel per dimension bucket -- dim
 <= 4, <= 8, <= 16 -- on forked streams), optionally replayed from a CUDA
-graph.  The tile configuration of each bucket's kernel (samples per thread,
-CTAs per SM) is picked by a small autotuner that times each configuration on
+graph.  The configuration of each bucket's kernel (threads per CTA, CTAs
+per SM) is picked by a small autotuner that times each configuration on
 a sample of the bucket's integrals.
 """
 import ctypes
@@ -47,7 +47,7 @@ class BatchIntegrator(object):
             from the weighted average (the reference's ``nitn`` of an adapt
             call followed by a final call).
         alpha, beta, seed: as ``Integrator``; integral j uses Philox stream j.
-        variant: tile configuration per dimension bucket, a sequence of 3
+        variant: kernel configuration per dimension bucket, a sequence of 3
             (or one int for all buckets); None: autotune.
         precision: 'fp32' (default: FP32 sampling, map and evaluation,
             float-float and FP64 sums) or 'fp64' (the parity configuration:

@@ -13,7 +13,10 @@
 //
 // Kernels on the 5th-generation tensor cores (CTA = 512 threads = 16 warps,
 // one per SM, TMEM accumulators; K in {16, 32}):
-//   flow_pass_umma_kernel   inference (sampling / density) and the training
+//   flow_pass_duo_kernel    inference and the training forward for more rows
+//                           than a 128-row tile per SM: two groups of 8 warps
+//                           on two tiles, activations as A operands in TMEM
+//   flow_pass_umma_kernel   the same for fewer rows: inference (sampling / density) and the training
 //                           forward (storing each layer's input)
 //   flow_bwd_umma_kernel    training backward of one layer: forward
 //                           recomputation, spline backward in registers,
@@ -1500,8 +1503,8 @@ __global__ void __launch_bounds__(UNT, 1) flow_pass_umma_kernel(FlowGeom g, cons
 // that finishes a layer's MMAs second starts the copy of the next layer's, under
 // the last splines.  Every wait is bounded; one that gives up sets a flag, after
 // which nothing waits any more and the loops run to their end.
-// The splines of 2^20 rows at dim 8: 1.60 ms with one group; see the launcher for
-// when this form is taken.
+// 2^20 rows at dim 8: 1.60 ms with one group of 16 warps, 1.31 ms so (with the
+// packed FP32 splines); see the launcher for when this form is taken.
 constexpr int DUO_NT = 256;      // threads of a group
 constexpr int DUO_D = 0, DUO_A = 160, DUO_COLS = 256;   // TMEM columns of a group
 

@@ -1,5 +1,5 @@
-// vg_fused.cuh -- dimension-bucket dispatch of the fused tile kernel for one
-// built-in integrand (included by one vg_fused_*.cu file per integrand so the
+// vg_fused.cuh -- dispatch of the fused iteration kernels for one built-in
+// integrand (included by one vg_fused_*.cu file per integrand so the
 // instantiations compile in parallel).
 #pragma once
 #include "vg_range.cuh"

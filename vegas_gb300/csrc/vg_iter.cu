@@ -3,26 +3,28 @@
 // Reference: src/vegas/_vegas.pyx (vegas 6.4.1), Integrator._random_batch
 // (pyx:1636-1765) and the batch loop of Integrator.__call__ (pyx:2096-2197).
 //
-// Layout of an iteration (all device-resident, no host round trip):
-//   1. allocation (one single-pass kernel): neval_h[h] from sigf
-//      (pyx:1692-1706), exclusive scan -> offsets[h], neval_hcube_range, the
-//      tile schedule tile_h0[t] (first hypercube of each tile of TILE
-//      samples).
-//   2. a persistent tile kernel: each CTA walks tiles t = blockIdx.x,
-//      += gridDim.x.  A tile is TILE consecutive samples (samples are ordered
-//      by hypercube, as in the reference).  Per sample: Philox uniforms (or
-//      injected ones), y = (y0 + u)/nstrat, the map y -> x, J from a grid
-//      table staged in shared memory, the integrand (fused built-in or read
-//      from an array), wf = wgt*f and the training histogram of
-//      fdv2 = (wf*n_h)^2 in shared memory.  Then the reference's two-pass
-//      per-hypercube mean/variance (with its EPSILON round-off guard) by a
-//      segmented scan over the tile.  Hypercubes cut by tile boundaries
-//      leave partial records (count, sum, sum of squared deviations).
-//   3. finalize (one CTA): merges the partial records with Chan's parallel
-//      variance formula, then sums the per-tile partials in tile order
-//      (compensated FP64) into the iteration mean / var / sum_sigf.
-// The tile kernel itself lives in vg_tile.cuh; its instantiations per
-// integrand are spread over vg_fused_*.cu and vg_dropin.cu.
+// Layout of an iteration (all device-resident, no host round trip; each kernel
+// is launched while the one before it drains):
+//   1. alloc_kernel: neval_h[h] from sigf (pyx:1692-1706), exclusive scan ->
+//      offsets[h], neval_hcube_range, the schedule tile_h0[t] (first hypercube
+//      of each 128 samples); without adaptive allocation the offsets are
+//      products.  FP32 mode: also the grid as an FP32 table.
+//   2. the iteration kernel over all samples (ordered by hypercube, as in the
+//      reference): Philox uniforms (or injected ones), y = (y0 + u)/nstrat, the
+//      map y -> x, J, the integrand (fused built-in or read from an array),
+//      wf = wgt*f, the training histogram of fdv2 = (wf*n_h)^2 and the
+//      per-hypercube mean and variance with the reference's EPSILON
+//      round-off guard.  FP32: warps on ranges of samples (vg_range.cuh); FP64:
+//      CTAs on tiles (vg_tile.cuh).  Hypercubes cut by the ends of ranges or
+//      tiles leave partial records (count, sum, sum of squared deviations).
+//   3. tail_kernel: one block (FP64: a few) merges the partial records with
+//      Chan's parallel variance formula and sums the partials into the
+//      iteration's mean / var / sum_sigf, while clusters of 8 CTAs adapt one
+//      axis each (finalize and adapt are separate kernels where the caller
+//      asks for one of them, or an axis has more increments than a cluster's
+//      threads).
+// The iteration kernels' instantiations per integrand are spread over
+// vg_fused_*.cu and vg_dropin.cu.
 #include <math.h>
 #include <string.h>
 

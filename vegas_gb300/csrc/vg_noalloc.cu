@@ -17,7 +17,13 @@
 
 #include "vg_common.cuh"
 
-static __device__ __align__(256) unsigned char g_vg_noalloc_scratch[VG_NOALLOC_SCRATCH_BYTES];
+// Beside the documented limit, room for the records and partial sums that a
+// workspace has at least (1024 and more, for the batched launch's groups of CTAs;
+// up to 170 KB that a small iteration does not use), so that they refuse no
+// iteration that the limit is meant to take.
+constexpr size_t SCRATCH_BYTES = (size_t)VG_NOALLOC_SCRATCH_BYTES + 256 * 1024;
+
+static __device__ __align__(256) unsigned char g_vg_noalloc_scratch[SCRATCH_BYTES];
 
 int vg_alloc_sync_reset(const vg_integrator *it, void *stream);   // vg_iter.cu
 
@@ -64,13 +70,13 @@ extern "C" int vg_iteration_noalloc(const vg_integrator *it, uint32_t itn, const
     local.work = nullptr;
     local.work_bytes = 0;
     const size_t need = vg_workspace_bytes(&local, 0);
-    if (need > (size_t)VG_NOALLOC_SCRATCH_BYTES)
+    if (need > SCRATCH_BYTES)
         return vg_fail(VG_ERR_MEMORY,
                        "vg_iteration_noalloc: this iteration needs %zu bytes of scratch, above the "
-                       "%d-byte static limit; use vg_allocate/vg_fused_iteration with a workspace",
-                       need, VG_NOALLOC_SCRATCH_BYTES);
+                       "%zu-byte static limit; use vg_allocate/vg_fused_iteration with a workspace",
+                       need, SCRATCH_BYTES);
     local.work = scratch;
-    local.work_bytes = (size_t)VG_NOALLOC_SCRATCH_BYTES;
+    local.work_bytes = SCRATCH_BYTES;
     // the scratch is shared by every geometry: start the allocation's
     // published words afresh
     if ((rc = vg_alloc_sync_reset(&local, stream))) return rc;
