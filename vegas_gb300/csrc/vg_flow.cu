@@ -933,11 +933,29 @@ __device__ __forceinline__ uint32_t relu_bf16x2(uint32_t v)
     return r;
 }
 
+// x a + c and y a + c
+template <bool PAIR>
+__device__ __forceinline__ void fma_pair(float &x, float &y, float a, float c)
+{
+    if constexpr (PAIR) {
+        f2_unpack(f2_fma(f2_pack(x, y), f2_pack(a, a), f2_pack(c, c)), x, y);
+    } else {
+        x = fmaf(x, a, c);
+        y = fmaf(y, a, c);
+    }
+}
+
 // ------------------------------------------------- tcgen05 inference pass
 // Spline of one coordinate with its 2K+1 logits in registers (compile-time
 // K, fully unrolled).  DIR 0: CDF at x; DIR 1: inverse CDF at x.  Returns
 // the transformed coordinate and lp = log pdf at the (input | output) point.
-template <int K, int DIR>
+// FEW: where a CTA has one tile, and latency counts rather than issue: the bin of
+// the block by a chain of selections beside the sums, and in DIR 0 scalar
+// operations.  The same bits.  Six layers, 5000 rows: dim 2 sampling 33.2 us
+// (34.8 with the form for many rows), dim 5 36.9 (38.8), dim 8 41.0 (43.0);
+// density of 19000 rows at dim 4 35.0 (36.9), dim 8 41.0 (43.0); from dim 9 on
+// the form for many rows is up to 2 us faster in density.
+template <int K, int DIR, bool FEW = false>
 __device__ __forceinline__ float spline_reg(float (&o)[2 * K + 1], float x, float &lp)
 {
     // Written for instruction-level parallelism: every reduction runs as 4
@@ -946,34 +964,51 @@ __device__ __forceinline__ float spline_reg(float (&o)[2 * K + 1], float x, floa
     static_assert(K % 8 == 0, "K must be a multiple of 8");
     constexpr int NB = K / 8;
     constexpr float c1 = 1.f - K * EPS_W;
-    float mx = o[0], mv = o[K], mx2 = o[1], mv2 = o[K + 1];   // two chains each
+    constexpr bool PAIR = !(FEW && DIR == 0);
+    float mx, mv;
+    if constexpr (PAIR) {   // two chains each
+        float mx2 = o[1], mv2 = o[K + 1];
+        mx = o[0];
+        mv = o[K];
 #pragma unroll
-    for (int k = 2; k < K; k += 4) {
-        mx = max3(mx, o[k], o[k + 1]);
-        if (k + 2 < K) mx2 = max3(mx2, o[k + 2], o[k + 3]);
-    }
+        for (int k = 2; k < K; k += 4) {
+            mx = max3(mx, o[k], o[k + 1]);
+            if (k + 2 < K) mx2 = max3(mx2, o[k + 2], o[k + 3]);
+        }
 #pragma unroll
-    for (int k = 2; k < K; k += 4) {
-        mv = max3(mv, o[K + k], o[K + k + 1]);
-        if (k + 2 < K) mv2 = max3(mv2, o[K + k + 2], o[K + k + 3]);
+        for (int k = 2; k < K; k += 4) {
+            mv = max3(mv, o[K + k], o[K + k + 1]);
+            if (k + 2 < K) mv2 = max3(mv2, o[K + k + 2], o[K + k + 3]);
+        }
+        mx = fmaxf(mx, mx2);
+        mv = max3(mv, mv2, o[2 * K]);
+    } else {
+        float m4[4], v4[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            m4[q] = o[q];
+            v4[q] = o[K + q];
+        }
+#pragma unroll
+        for (int k = 4; k < K; k++) m4[k & 3] = fmaxf(m4[k & 3], o[k]);
+#pragma unroll
+        for (int k = 4; k <= K; k++) v4[k & 3] = fmaxf(v4[k & 3], o[K + k]);
+        mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+        mv = fmaxf(fmaxf(v4[0], v4[1]), fmaxf(v4[2], v4[3]));
     }
-    mx = fmaxf(mx, mx2);
-    mv = max3(mv, mv2, o[2 * K]);
     // exponentials as 2^(v log2 e - max log2 e): one FMA and the MUFU each;
     // the vertex heights are stored halved (exponent - 1), which absorbs the
     // trapezoid's 1/2 in the segment areas (the partial-bin formulas at the
     // end restore the factor 2)
     constexpr float L2E = 1.4426950408889634f;
     const float mxl = mx * L2E, mvl = fmaf(mv, L2E, 1.f);
-    const uint64_t l2 = f2_pack(L2E, L2E);
-    const uint64_t nx2 = f2_pack(-mxl, -mxl), nv2 = f2_pack(-mvl, -mvl);
     // width exponentials, summed per block of 8 bins (NB independent chains)
     float sB[NB];
 #pragma unroll
     for (int b = 0; b < NB; b++) sB[b] = 0.f;
 #pragma unroll
     for (int k = 0; k < K; k += 2) {
-        f2_unpack(f2_fma(f2_pack(o[k], o[k + 1]), l2, nx2), o[k], o[k + 1]);
+        fma_pair<PAIR>(o[k], o[k + 1], L2E, -mxl);
         o[k] = vg_ex2_approx(o[k]);
         o[k + 1] = vg_ex2_approx(o[k + 1]);
         sB[k >> 3] += o[k];
@@ -983,12 +1018,11 @@ __device__ __forceinline__ float spline_reg(float (&o)[2 * K + 1], float x, floa
 #pragma unroll
     for (int b = 0; b < NB; b++) stot += sB[b];
     const float cw = __fdividef(c1, stot);
-    const uint64_t cw2 = f2_pack(cw, cw), ep2 = f2_pack(EPS_W, EPS_W);
 #pragma unroll
-    for (int k = 0; k < K; k += 2) f2_unpack(f2_fma(cw2, f2_pack(o[k], o[k + 1]), ep2), o[k], o[k + 1]);   // bin widths
+    for (int k = 0; k < K; k += 2) fma_pair<PAIR>(o[k], o[k + 1], cw, EPS_W);   // bin widths
 #pragma unroll
     for (int k = 0; k < K; k += 2) {   // vertex heights / 2
-        f2_unpack(f2_fma(f2_pack(o[K + k], o[K + k + 1]), l2, nv2), o[K + k], o[K + k + 1]);
+        fma_pair<PAIR>(o[K + k], o[K + k + 1], L2E, -mvl);
         o[K + k] = vg_ex2_approx(o[K + k]);
         o[K + k + 1] = vg_ex2_approx(o[K + k + 1]);
     }
@@ -1038,32 +1072,51 @@ __device__ __forceinline__ float spline_reg(float (&o)[2 * K + 1], float x, floa
 #pragma unroll
         for (int b = 1; b < NB; b++) usel[q] = bsel == b ? o[K + 8 * b + q] : usel[q];
     }
-    // the block's bins: their starts, then a binary descent over these (the
-    // first bin that ends above t, the last one where none does)
-    float Eq[8], Pq[8];
+    float Wb = 0.f, ub = 0.f, ub1 = 0.f, Eb = 0.f, Pb = 0.f;
+    if constexpr (FEW) {
+        bool f = false;
 #pragma unroll
-    for (int q = 0; q < 8; q++) {
-        const float wq = wsel[q], sq = (usel[q] + usel[q + 1]) * wq;
-        Eq[q] = E;
-        Pq[q] = P;
-        E += wq;
-        P += sq;
+        for (int q = 0; q < 8; q++) {
+            const float wq = wsel[q], sq = (usel[q] + usel[q + 1]) * wq;
+            // the last bin of the block takes t when no earlier bin did
+            const bool here = !f && (q == 7 || (DIR == 0 ? (t < E + wq) : (t < P + sq)));
+            Wb = here ? wq : Wb;
+            ub = here ? usel[q] : ub;
+            ub1 = here ? usel[q + 1] : ub1;
+            Eb = here ? E : Eb;
+            Pb = here ? P : Pb;
+            f = f || here;
+            E += wq;
+            P += sq;
+        }
+    } else {
+        // the block's bins: their starts, then a binary descent over these (the
+        // first bin that ends above t, the last one where none does)
+        float Eq[8], Pq[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            const float wq = wsel[q], sq = (usel[q] + usel[q + 1]) * wq;
+            Eq[q] = E;
+            Pq[q] = P;
+            E += wq;
+            P += sq;
+        }
+#pragma unroll
+        for (int n = 4; n > 0; n >>= 1) {
+            const bool up = DIR == 0 ? t >= Eq[n] : t >= Pq[n];
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (q < n) {
+                    wsel[q] = up ? wsel[n + q] : wsel[q];
+                    Eq[q] = up ? Eq[n + q] : Eq[q];
+                    Pq[q] = up ? Pq[n + q] : Pq[q];
+                }
+#pragma unroll
+            for (int q = 0; q <= 4; q++)
+                if (q <= n) usel[q] = up ? usel[n + q] : usel[q];
+        }
+        Wb = wsel[0], ub = usel[0], ub1 = usel[1], Eb = Eq[0], Pb = Pq[0];
     }
-#pragma unroll
-    for (int n = 4; n > 0; n >>= 1) {
-        const bool up = DIR == 0 ? t >= Eq[n] : t >= Pq[n];
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-            if (q < n) {
-                wsel[q] = up ? wsel[n + q] : wsel[q];
-                Eq[q] = up ? Eq[n + q] : Eq[q];
-                Pq[q] = up ? Pq[n + q] : Pq[q];
-            }
-#pragma unroll
-        for (int q = 0; q <= 4; q++)
-            if (q <= n) usel[q] = up ? usel[n + q] : usel[q];
-    }
-    const float Wb = wsel[0], ub = usel[0], ub1 = usel[1], Eb = Eq[0], Pb = Pq[0];
     // ub, ub1 are half the vertex heights: the area of the first al of the
     // bin is Wb (al 2 ub + al^2 (ub1 - ub)), the pdf 2 ((1 - al) ub + al ub1) / Z
     float al, xo;
@@ -1088,20 +1141,21 @@ __device__ __forceinline__ float spline_reg(float (&o)[2 * K + 1], float x, floa
 // logits with 16-byte loads.
 __host__ __device__ constexpr int bias_stride(int K) { return (2 * K + 1 + 3) / 4 * 4; }
 
-template <int K>
+template <int K, bool PAIR = true>
 __device__ __forceinline__ void add_bias(float (&o)[2 * K + 1], const float *bb)
 {
     constexpr int NR = 2 * K + 1;
 #pragma unroll
     for (int q = 0; q < NR; q += 4) {
         const float4 b = *reinterpret_cast<const float4 *>(bb + q);
-        if (q + 3 < NR) {
+        if (PAIR && q + 3 < NR) {
             f2_unpack(f2_add(f2_pack(o[q], o[q + 1]), f2_pack(b.x, b.y)), o[q], o[q + 1]);
             f2_unpack(f2_add(f2_pack(o[q + 2], o[q + 3]), f2_pack(b.z, b.w)), o[q + 2], o[q + 3]);
         } else {
             o[q] += b.x;
             if (q + 1 < NR) o[q + 1] += b.y;
             if (q + 2 < NR) o[q + 2] += b.z;
+            if (q + 3 < NR) o[q + 3] += b.w;
         }
     }
 }
@@ -1337,11 +1391,11 @@ __global__ void __launch_bounds__(UNT, 1) flow_pass_umma_kernel(FlowGeom g, cons
                     }
                     if (NR > 64) o[64] = umma::tmem_ld1(tmem + lane_base + col + 64u);
                 }
-                add_bias<K>(o, sb3 + j * bias_stride(K));
+                add_bias<K, DIR == 1>(o, sb3 + j * bias_stride(K));
                 const int cz = y.B[j];
                 const float xin = Zs[r * zst + cz];
                 float lp;
-                const float xo = spline_reg<K, DIR>(o, xin, lp);
+                const float xo = spline_reg<K, DIR, true>(o, xin, lp);
                 Zs[r * zst + cz] = fminf(fmaxf(xo, 0.f), 1.f);
                 sLD[(size_t)h * ST * FROWS + s * FROWS + r] += lp;
             };
