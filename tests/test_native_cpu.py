@@ -87,3 +87,16 @@ def test_flow_train_workspace_sizes(dim, K):
         prev = b
     s.hidden = 64   # unsupported width: the query reports an error
     assert int(L.vg_flow_train_bytes(ctypes.byref(s), 128)) < 0
+
+
+def test_kernels_read_no_memory_through_the_read_only_path():
+    """Non-coherent loads need data that nothing writes while the kernel lives.  An
+    iteration's kernels are placed while the one before them still writes, and the
+    batched kernel rewrites its grid table at each iteration."""
+    csrc = os.path.join(ROOT, 'vegas_gb300', 'csrc')
+    for name in sorted(os.listdir(csrc)):
+        if not name.endswith(('.cu', '.cuh')):
+            continue
+        txt = open(os.path.join(csrc, name)).read()
+        txt = re.sub(r'//[^\n]*', '', re.sub(r'/\*.*?\*/', '', txt, flags=re.S))
+        assert not re.search(r'__ldg\s*\(|ld\.global\.nc|global\.nc', txt), name

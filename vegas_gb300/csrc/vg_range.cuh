@@ -529,8 +529,10 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
                                                                ax.Kf, yd, yn, yfl);
                                 // y <= 1 (below 2^24 strata the product y0 + u = nstrat times 1 / nstrat
                                 // rounds to 1 at most), so iy <= ninc, and at y = 1 the table's last entry
-                                // has x and dy = 0
-                                const float2 e = table_smem ? table[d * Wk + iy] : __ldg(a.tablef + d * Wk + iy);
+                                // has x and dy = 0.  (An ordinary load: the batched kernel rewrites
+                                // the table at each iteration, and this kernel may be placed while
+                                // the allocation still writes it, so the read-only path is not open.)
+                                const float2 e = table_smem ? table[d * Wk + iy] : a.tablef[d * Wk + iy];
                                 float dy = yn - yfl;
                                 if (wide && iy >= ax.ninc) dy = 0.f;
                                 if (NEED_X) x[d] = fmaf(e.y, dy, e.x);
@@ -543,13 +545,14 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
                             }
                         }
                     } else {
-                        jac = __ldg((const float *)a.keep_jac + ig);
+                        // (ordinary loads, for the kernel may be placed while the sampler writes these)
+                        jac = ((const float *)a.keep_jac)[ig];
                         if (a.train) {
                             const uint2 *src = reinterpret_cast<const uint2 *>(a.keep_bins + (size_t)ig * a.keep_bstride);
 #pragma unroll
                             for (int g = 0; 4 * g < DIMB; g++) {
                                 if (4 * g >= dim) break;
-                                const uint2 t = __ldg(src + g);
+                                const uint2 t = src[g];
                                 bins[2 * g] = t.x;
                                 bins[2 * g + 1] = t.y;
                             }
