@@ -38,8 +38,11 @@ constexpr int CHUNK = 128;      // samples per chunk
 constexpr int WCAP = 68;        // hypercube starts a chunk can see (every count is >= 2), padded
 static_assert(CHUNK == BASE_TILE, "tile_h0 gives the first hypercube of each chunk");
 
+constexpr int OPEN = WCAP - 1;  // a chunk sees WCAP - 2 hypercubes at the most
+
 // Per-warp shared memory.  res holds (D, Q) of the hypercubes that end in the
-// chunk; the sampling weights dv_y / neval_h use the same space before.
+// chunk, the sampling weights dv_y / neval_h use the same space before; its
+// last element holds (D, Q) of the one that began before the chunk.
 struct WarpBuf {
     float4 res[WCAP];
     float wf[CHUNK];
@@ -167,39 +170,79 @@ struct LaneSums {
     float mh, ml, vh, vl, sh, sl;
 };
 
-// A hypercube whose squares leave the float range, in FP64 from its samples
-// (x != nullptr: all of them are in the chunk) or from its float-float sums.
-static __device__ __noinline__ double3 finish_big(const float *x, int n, float c, DQ v, double beta_half, int adaptive,
-                                                  double *sigf_h, int want_var)
+// Beyond this a sum Q of squares goes to FP64 (also where it is infinite or NaN).
+constexpr float BIG_Q = 1e30f;
+
+// D and Q in FP64 of the piece at samples o to oe of the chunk about c; with o < 0 it
+// began earlier, and wb.res[OPEN] has the sums of its samples before the chunk.
+__device__ __forceinline__ void sums_f64(const WarpBuf &wb, int o, int oe, float c, double &D, double &Q)
 {
+    D = Q = 0.0;
+    if (o < 0) {
+        const float4 v = wb.res[OPEN];
+        D = vg_ff_value(v.x, v.y);
+        Q = vg_ff_value(v.z, v.w);
+    }
+    for (int i = max(o, 0); i < oe; i++) {
+        const double d = (double)wb.wf[i] - (double)c;
+        D += d;
+        Q = fma(d, d, Q);
+    }
+}
+
+// A hypercube of n samples whose squares leave the float range, in FP64.
+static __device__ __noinline__ double3 finish_big(const WarpBuf &wb, int o, int oe, float c, double beta_half,
+                                                  int adaptive, double *sigf_h, int want_var)
+{
+    const int n = oe - o;
     const double nd = (double)n;
     double S, D = 0.0, Q = 0.0;
-    if (x != nullptr) {
+    if (o >= 0) {
         S = 0.0;
-        for (int i = 0; i < n; i++) S += (double)x[i];
+        for (int i = o; i < oe; i++) S += (double)wb.wf[i];
         const double m = S / nd;
-        for (int i = 0; i < n; i++) {
-            const double d = (double)x[i] - m;
+        for (int i = o; i < oe; i++) {
+            const double d = (double)wb.wf[i] - m;
             D += d;
             Q = fma(d, d, Q);
         }
     } else {
-        D = vg_ff_value(v.dh, v.dl);
-        Q = vg_ff_value(v.qh, v.ql);
+        sums_f64(wb, o, oe, c, D, Q);
         S = nd * (double)c;
     }
     return finish_f64(S, D, Q, n, beta_half, adaptive, sigf_h, want_var);
 }
 
+// A piece of n samples of which those before oe in the chunk are the last, and whose squares
+// about c leave the float range: its sums about its mean, which is returned, to
+// wb.res[OPEN].  Q is then near the variance and no longer up to n times as large (c an
+// outlier), so a piece that goes on stays in the range that its variance has.  One lane.
+static __device__ __noinline__ float recentre_big(WarpBuf &wb, int o, int oe, int n, float c)
+{
+    double D, Q;
+    sums_f64(wb, o, oe, c, D, Q);
+    const double nd = (double)n;
+    const float m = (float)((double)c + D / nd);
+    const double t = (double)c - (double)m;
+    Q += t * (2.0 * D + nd * t);
+    D += nd * t;
+    float4 v;
+    ff_from_double(D, v.x, v.y);
+    ff_from_double(Q, v.z, v.w);
+    wb.res[OPEN] = v;
+    return m;
+}
+
 // One whole hypercube: mean, variance (n Q - D^2) / (n - 1) and sigf =
 // |var|^(beta/2) (pyx:2174-2186) into the lane's sums; FP64 only where the
-// squares leave the float range.  x: its samples, when all are in the chunk.
-__device__ __forceinline__ void finish_hcube(const IterArgs &a, int64_t h, int n, float c, const DQ &v, const float *x,
-                                             float beta_half_f, LaneSums &s)
+// squares leave the float range.  It is at samples o (< 0: it began earlier) to oe
+// of the chunk.
+__device__ __forceinline__ void finish_hcube(const IterArgs &a, int64_t h, const WarpBuf &wb, int o, int oe, float c,
+                                             const DQ &v, float beta_half_f, LaneSums &s)
 {
-    const float fn = (float)n;
-    if (!(fabsf(v.qh) < 1e30f)) {
-        const double3 r = finish_big(x, n, c, v, a.beta_half, a.adaptive, a.sigf + h, a.train_hc);
+    const float fn = (float)(oe - o);
+    if (!(fabsf(v.qh) < BIG_Q)) {
+        const double3 r = finish_big(wb, o, oe, c, a.beta_half, a.adaptive, a.sigf + h, a.train_hc);
         float rh, rl;
         ff_from_double(r.x, rh, rl);
         ff_add_pair(s.mh, s.ml, rh, rl);
@@ -249,9 +292,10 @@ struct Piece {
         if (qh == 0.f) {
             qh = guard_q(n, sh);
         } else {
-            float d2h, d2l, th, tl;
-            ff_sqr(r.dh, r.dl, d2h, d2l);
-            ff_div_f(d2h, d2l, n, th, tl);
+            // Q - D (D / n), at most Q: D^2 would leave the float range before it
+            float mh, ml, th, tl;
+            ff_div_f(r.dh, r.dl, n, mh, ml);
+            ff_mul(r.dh, r.dl, mh, ml, th, tl);
             ff_add_pair(qh, ql, -th, -tl);
         }
     }
@@ -294,7 +338,7 @@ struct Piece {
 static __device__ __noinline__ void finish_cut(const IterArgs &a, int64_t h, const Piece &p, float (&s6)[6])
 {
     float vh, vl;
-    if (fabsf(p.qh) < 1e30f) {
+    if (fabsf(p.qh) < BIG_Q) {
         ff_mul_f(p.qh, p.ql, p.n, vh, vl);
         ff_div_f(vh, vl, p.n - 1.f, vh, vl);
     } else {   // squares beyond the float range: this hypercube in FP64
@@ -636,7 +680,10 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
                 float c = o0 < 0 ? c_open : wb.wf[o0];
                 DQ v, vfirst;
                 v.zero();
-                if (lane == 0) v = v_open;
+                if (lane == 0) {
+                    v = v_open;
+                    wb.res[OPEN] = make_float4(v.dh, v.dl, v.qh, v.ql);
+                }
                 bool started = lane == 0 || (nib & 1u);
                 int kfirst = -1;
 #pragma unroll
@@ -680,19 +727,33 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
                 // ---- the hypercubes that end here, one lane each
                 for (int k = lane; k < nfin; k += 32) {
                     const float4 t = wb.res[k];
-                    const DQ q = {t.x, t.y, t.z, t.w};
+                    DQ q = {t.x, t.y, t.z, t.w};
                     const int o = wb.off[k], oe = wb.off[k + 1];
-                    const float ck = o < 0 ? c_open : wb.wf[o];
-                    if (k == 0 && cut0)
-                        rec[0] = RangeRec{h, (int)(b + oe - s0), ck, q.dh, q.dl, q.qh, q.ql};
-                    else
-                        finish_hcube(a, h + k, oe - o, ck, q, o < 0 ? nullptr : wb.wf + o, beta_half_f, sums);
+                    float ck = o < 0 ? c_open : wb.wf[o];
+                    if (k == 0 && cut0) {
+                        const int n = (int)(b + oe - s0);
+                        if (!(fabsf(q.qh) < BIG_Q)) {
+                            ck = recentre_big(wb, o, oe, n, ck);
+                            q = DQ{wb.res[OPEN].x, wb.res[OPEN].y, wb.res[OPEN].z, wb.res[OPEN].w};
+                        }
+                        rec[0] = RangeRec{h, n, ck, q.dh, q.dl, q.qh, q.ql};
+                    } else {
+                        finish_hcube(a, h + k, wb, o, oe, ck, q, beta_half_f, sums);
+                    }
                 }
                 if (nfin > 0) cut0 = false;   // its first piece is recorded
-                v_open = v_next;
-                c_open = c_next;
                 open = !ended;
                 n_open = len - wb.off[nw - 1];
+                v_open = v_next;
+                c_open = c_next;
+                if (open && !(fabsf(v_next.qh) < BIG_Q)) {
+                    if (lane == 0)
+                        c_open = recentre_big(wb, wb.off[nw - 1], len, cut0 ? (int)(b + len - s0) : n_open, c_next);
+                    __syncwarp();
+                    const float4 t = wb.res[OPEN];
+                    v_open = DQ{t.x, t.y, t.z, t.w};
+                    c_open = __shfl_sync(0xffffffffu, c_open, 0);
+                }
             }
             h += nfin;
             __syncwarp();
