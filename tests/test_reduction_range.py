@@ -79,3 +79,42 @@ def test_outliers_near_the_float_range(nstrat, neval, beta, every, X, kept):
     if adaptive:
         np.testing.assert_allclose(sigf, want, rtol=2e-5)
         assert abs(st.sum_sigf - ss) <= 2e-5 * ss
+
+
+def _divide(a, b):
+    """a / b as float-float: quotient by the correctly rounded reciprocal, corrected once."""
+    r = np.float32(1) / np.float32(b)
+    q1 = np.float32(np.float32(a) * r)
+    q2 = np.float32(np.float32(float(a) - float(q1) * b) * r)
+    return float(q1) + float(q2)
+
+
+def test_variance_divides_by_the_rounded_reciprocal():
+    """One hypercube of n small whole numbers, 0 the first and the sum of each chunk of 128:
+    n Q is a whole number below 2^24 and exact on every way to the variance n Q / (n - 1),
+    whose bits are then those of the division.  (A reciprocal to an ulp is another float
+    for one whole number in eight, and its quotient's error up to twice as large.)"""
+    rng = np.random.default_rng(2)
+    for n in range(129, 801):
+        I = vg.Integrator([[0, 1]], neval=n, nstrat=[1], maxinc_axis=2, seed=n, beta=0.0, alpha=0.0)
+        want = np.zeros(n, np.float32)
+
+        def values(x, w, nh):
+            w0 = np.float32(w[0].item())
+            q = np.arange(1, 6).astype(np.float32)   # those that are products of floats and the weight
+            f = np.stack([q / w0, np.nextafter(q / w0, np.float32(100)), np.nextafter(q / w0, np.float32(0))])
+            hit = (f * w0 == q).any(axis=0)
+            f = f[(f * w0 == q).argmax(axis=0), np.arange(len(q))]
+            out = np.zeros(n, np.float32)
+            for b in range(0, n, 128):
+                m = (min(n, b + 128) - b - 1) // 2   # pairs after the first
+                pick = rng.choice(np.flatnonzero(hit), m)
+                want[b + 1:b + 1 + m], out[b + 1:b + 1 + m] = q[pick], f[pick]
+                want[b + 1 + m:b + 1 + 2 * m], out[b + 1 + m:b + 1 + 2 * m] = -q[pick], -f[pick]
+            return torch.from_numpy(out).to(x.device)
+
+        st, _, nh, wf = _reduce(I, values, False)
+        assert list(nh) == [n] and np.array_equal(wf, want)
+        num = n * int((want.astype(np.int64) ** 2).sum())
+        assert st.status == 0 and 0 < num < 2 ** 24
+        assert st.var == _divide(num, n - 1), n

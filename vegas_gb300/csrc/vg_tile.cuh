@@ -364,12 +364,16 @@ __device__ __forceinline__ void ff_sqr(float ah, float al, float &h, float &l)
     l = __fsub_rn(e, __fsub_rn(h, p));
 }
 
-// (h, l) = (ah, al) / b in float-float: head quotient, its remainder by fma,
-// one correction term.
+// (h, l) = (ah, al) / b in float-float, b a count: head quotient, its remainder by
+// fma, one correction term.  The reciprocal is the correctly rounded one, by a Newton
+// step on the special-function unit's (as that is, to an ulp, the quotient's error is up
+// to twice as large).  The step gives __frcp_rn's bits for every count below 2^31, and
+// __frcp_rn itself, whose path is for all floats, took 2 % of the dim-4 ridge's call.
 __device__ __forceinline__ void ff_div_f(float ah, float al, float b, float &h, float &l)
 {
-    float rb;   // to an ulp: the remainder term corrects it
+    float rb;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rb) : "f"(b));
+    rb = __fmaf_rn(rb, __fmaf_rn(-b, rb, 1.f), rb);
     const float q1 = __fmul_rn(ah, rb);
     const float r = __fadd_rn(__fmaf_rn(-q1, b, ah), al);
     const float q2 = __fmul_rn(r, rb);
