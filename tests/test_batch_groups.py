@@ -63,3 +63,29 @@ def test_groups_agree_after_adapting(kind, dim, variant, group):
     np.testing.assert_allclose(ob[:, 0, :2], oa[:, 0, :2], rtol=1e-6)
     np.testing.assert_allclose(ob[:, 1, 0], oa[:, 1, 0], rtol=2e-3)
     np.testing.assert_allclose(ob[:, 1, 1], oa[:, 1, 1], rtol=4e-3)
+
+
+@pytest.mark.parametrize('dim,variant,group', [(16, 0, 3), (8, 0, 3), (4, 2, 5), (7, 1, 2)])
+def test_groups_agree_when_adapting_to_errors(dim, variant, group):
+    """adapt_to_errors (a field of the C record): the finalize adds the hypercubes cut by
+    ranges to the training histogram that the group's other CTAs then adapt from.  The
+    variances are float-float and the sums FP64; their averages are rounded to FP32,
+    6e-8, so 6e-8 of 1000 increments is the most that a node moves where its weight is the
+    average: a thousandth of an increment is allowed."""
+    from vegas_gb300.batch import BatchIntegrator
+    runs = []
+    for g in (1, group):
+        B = BatchIntegrator(_lorentz(dim, 3, dim), [100003, 150000, 120001], nitn=1, nwarm=0, beta=0.0, seed=31,
+                            variant=variant, group=g)
+        for it in B.its:
+            it.adapt_to_errors = 1
+        B.set_variant(variant)
+        B.run()
+        runs.append(B)
+    a, b = runs
+    np.testing.assert_allclose(b.iterations()[:, 0], a.iterations()[:, 0], rtol=1e-6)
+    for j in range(3):
+        ga, gb = (x.state(j)['grid'].cpu().numpy() for x in (a, b))
+        assert np.abs(ga - gb).max() <= 1e-3 / a.ninc[j].min()
+        for d, k in enumerate(a.ninc[j]):
+            assert np.abs(ga[d, :k + 1] - np.linspace(0.0, 1.0, k + 1)).max() > 0.01

@@ -385,7 +385,7 @@ __device__ __forceinline__ void range_dispatch(const VgParams &prm, int rank, in
 // Group mode (group = G >= 2, cooperative launch): CTA c works on integral
 // order[c / G] as rank c % G; rank 0 allocates and finalizes, all G
 // ranks share the samples and the axes to adapt, with three group barriers per
-// iteration.
+// iteration (four under adapt_to_errors).
 template <typename T, int KIND, int DIMB, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) batch_kernel(const BatchJob *__restrict__ jobs,
                                                    const VgParams *__restrict__ params,
@@ -452,6 +452,10 @@ __global__ void __launch_bounds__(MAXT, 1) batch_kernel(const BatchJob *__restri
                     J.out[3 * it + 2] = (double)sa.stats->neval;
                 }
             }
+            // adapt_to_errors: the finalize still trains the map on the hypercubes
+            // cut by ranges, and the other ranks are not to read or clear before
+            if (G > 1 && J.adapt && sa.train_hc &&
+                !(ok = group_barrier(J.sync, (unsigned)G * ++rounds, sa.wait_iters))) break;
             if (J.adapt) cta_adapt(J, rank, G);
             __syncthreads();
             if (G > 1 && J.adapt && !(ok = group_barrier(J.sync, (unsigned)G * ++rounds, sa.wait_iters))) break;
