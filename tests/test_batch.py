@@ -114,3 +114,20 @@ def test_batch_lattice_scan_against_transfer_matrix():
     exact = np.array([f.exact(4) for f in fs])
     pulls = (res[:, 0] - exact) / res[:, 1]
     assert np.max(np.abs(pulls)) < 5, pulls
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('ninc', [14048, 14049, 14203])
+def test_batch_maps_up_to_the_shared_memory_of_an_adapt(ninc, monkeypatch):
+    """The weights and cumulative sums of one axis fill a CTA's shared memory at 14203
+    increments (16 bytes each)."""
+    import functools
+    from vegas_gb300 import batch
+    monkeypatch.setattr(batch, 'strata', functools.partial(vg.strata, maxinc_axis=ninc))
+    f = vg.LorentzianProduct([0.4], [0.05])
+    B = batch.BatchIntegrator([f], [160000], nitn=3, nwarm=1, seed=5, variant=0, group=1)
+    assert int(B.ninc[0][0]) == ninc
+    res = B.run()
+    assert abs(res[0, 0] - f.exact(1)) < 5 * res[0, 1]
+    out = B.iterations()
+    assert out[0, 2, 1] < out[0, 0, 1]   # adapted

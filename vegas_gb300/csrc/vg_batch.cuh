@@ -72,8 +72,9 @@ __device__ __forceinline__ bool group_barrier(unsigned int *ctr, unsigned int ta
     return s_ok != 0;
 }
 
-// Shared memory of an axis' adaptation: weights, cumulative sums, partial sums.
-__host__ __device__ constexpr size_t adapt_group_doubles(int max_old) { return 2 * (size_t)max_old + 64; }
+// Shared memory of an axis' adaptation: weights, cumulative sums, partial sums
+// (block_sum takes 33).
+__host__ __device__ constexpr size_t adapt_group_doubles(int max_old) { return 2 * (size_t)max_old + 34; }
 
 constexpr int APER = 4;          // hypercubes per thread and pass of the allocation
 constexpr int F64_S = 2;         // samples per thread of the FP64 tiles
@@ -488,12 +489,18 @@ int launch_one(int ntb, const BatchJob *jobs, const VgParams *prm, const int *or
     return VG_OK;
 }
 
-// sets the kernel's shared-memory attribute (outside any stream capture)
+// sets the kernel's shared-memory attribute (outside any stream capture): always
+// all that the kernel may have, so that plans of one batch do not lower another's
 template <typename T, int KIND, int DIMB, int MAXT>
 int occupancy_one(int ntb, size_t smem, int *per_sm)
 {
     auto k = batch_kernel<T, KIND, DIMB, MAXT>;
-    VG_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    int dev = 0, most = 0;
+    cudaFuncAttributes fa;
+    VG_CUDA_CHECK(cudaGetDevice(&dev));
+    VG_CUDA_CHECK(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    VG_CUDA_CHECK(cudaFuncGetAttributes(&fa, k));
+    VG_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes));
     VG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k, ntb, smem));
     return VG_OK;
 }
