@@ -359,7 +359,7 @@ __device__ __forceinline__ void range_dispatch(const VgParams &prm, int rank, in
 {
     const IterArgs &a = job_args();
     constexpr int ET = RF_EXACT | RF_TABLE;
-    if (a.wide || (a.train && !a.hist_smem) || (DIMB <= 8 && !a.table_smem))
+    if (a.wide || a.few || (a.train && !a.hist_smem) || (DIMB <= 8 && !a.table_smem))
         return cta_range<KIND, DIMB, RF_GENERAL>(prm, rank, G);
     if constexpr (DIMB == 4) {
         if (a.dim == 4) cta_range<KIND, 4, ET>(prm, rank, G);

@@ -540,6 +540,7 @@ int fill_args(IterArgs &a, const vg_integrator *it, uint32_t itn, const double *
     const int ate = it->adapt_to_errors ? 1 : 0;
     a.adaptive_alloc = (it->beta > 0 && it->nhcube > 1 && !ate) ? 1 : 0;
     a.adaptive = (a.adaptive_alloc && it->adapt) ? 1 : 0;
+    a.few = (a.adaptive_alloc ? (double)it->min_neval_hcube : (double)it->neval / (double)it->nhcube) < 2.0;
     a.train = (it->adapt && it->alpha > 0 && !ate) ? 1 : 0;
     a.train_hc = (ate && it->adapt) ? 1 : 0;
     a.sum_f = it->sum_f;

@@ -374,6 +374,34 @@ __device__ __forceinline__ bool scan_pieces(Piece &cur, bool started)
     return heads != 0u;
 }
 
+// Hypercubes of one sample or none: the hypercube of the sample b, at h or after it, and
+// a length of the chunk there such that it sees no more hypercubes than the warp's
+// buffer takes, and none without samples (two that start at the same sample).
+struct Windows {
+    int64_t h;
+    int len;
+};
+static __device__ __noinline__ Windows few_windows(const IterArgs &a, int64_t b, int64_t N, int64_t h, int len)
+{
+    const int lane = threadIdx.x & 31;
+    auto start = [&](int64_t k) {   // of hypercube k, relative to b
+        const int64_t dif = (k <= a.H ? a.offsets[k] : N) - b;
+        return dif > CHUNK ? CHUNK + 1 : (dif < -1 ? -1 : (int)dif);
+    };
+    for (;;) {   // pass those that end at b or before
+        const int64_t next = h + 1 + lane;
+        const unsigned int m = __ballot_sync(0xffffffffu, next < a.H && start(next) <= 0);
+        h += __popc(m);
+        if (m != 0xffffffffu) break;
+    }
+    int cut = len;
+    for (int k = 1 + lane; k < WCAP - 1; k += 32) {
+        const int s = start(h + k);
+        if (s < cut && (k == WCAP - 2 || start(h + k + 1) == s)) cut = s;
+    }
+    return Windows{h, __reduce_min_sync(0xffffffffu, cut)};
+}
+
 // ------------------------------------------------------------------ kernel
 constexpr int RF_CHAIN = 8;   // a kernel of its own, launched with vg_launch_pdl
 
@@ -392,8 +420,8 @@ struct IndexType<true> {
 // warp instructions).
 constexpr int RF_EXACT = 1;   // dim == DIMB
 constexpr int RF_TABLE = 2;   // the grid table is in shared memory (else: read through L1)
-constexpr int RF_GENERAL = 4; // injected uniforms, 2^31 hypercubes or samples, 2^24 strata on an axis, the table
-                              // and the histogram in either place
+constexpr int RF_GENERAL = 4; // injected uniforms, 2^31 hypercubes or samples, 2^24 strata on an axis, hypercubes
+                              // of fewer than two samples, the table and the histogram in either place
 
 // The work of CTA `rank` of `nranks` on one integral's iteration; its partial
 // sums go to a.parts[rank].  deal > 0 (the batched launch): units of `deal`
@@ -487,8 +515,15 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
         float c_open = 0.f;
         DQ v_open;
         v_open.zero();
-        for (Idx b = s0; b < s1; b += CHUNK) {
-            const int len = (int)(s1 - b < CHUNK ? s1 - b : CHUNK);
+        int len = CHUNK;
+        for (Idx b = s0; b < s1; b += GENERAL ? len : CHUNK) {
+            len = (int)(s1 - b < CHUNK ? s1 - b : CHUNK);
+            if constexpr (GENERAL)
+                if (a.few) {
+                    const Windows w = few_windows(a, b, N, h, len);
+                    h = w.h;
+                    len = w.len;
+                }
             // ---- the hypercubes of the chunk
             int nw = 0;
             if (lane < CHUNK / 32) wb.mask[lane] = 0u;
@@ -986,7 +1021,7 @@ int launch_range(IterArgs &a, const VgParams *prm, int tab_len, cudaStream_t st)
     const RangePlan p = range_fit(range_threads(a.dim), a.dim, a.maxK, tab_len, train, NEED_MAP && g_tile_table != 0,
                                   RANGE_SMEM, &a.table_smem, &a.hist_smem);
     if (p.total > RANGE_SMEM) return vg_fail(VG_ERR_UNSUPPORTED, "shared memory plan too large");
-    if ((!NEED_MAP || a.u == nullptr) && !a.wide && (!NEED_RED || !a.train || a.hist_smem)) {
+    if ((!NEED_MAP || a.u == nullptr) && !a.wide && !a.few && (!NEED_RED || !a.train || a.hist_smem)) {
         if (!NEED_MAP || a.table_smem) {
             switch (a.dim) {
             case 1: return launch_range_as<MODE, KIND, 1, ET>(a, prm, p.total, st);

@@ -132,7 +132,7 @@ struct IterArgs {
     double dv_y;              // 1 / nhcube (pyx:1639)
     double beta_half;         // beta / 2 (pyx:2185)
     uint32_t wait_iters;      // polls of a bounded wait before it gives up (vg_set_wait_budget)
-    uint32_t pad_wait;
+    int few;                  // hypercubes may have fewer than two samples
 };
 
 struct SmemPlan {
@@ -1010,7 +1010,9 @@ int launch_tile(IterArgs &a, const VgParams *prm, cudaStream_t st)
     // many, so that the FP64 work (19 cycles per warp instruction and SM) spreads
     // over more SMs; a CTA then has too few samples to stage the grid or a
     // histogram for.  1e4 evaluations at dim 4: 75 us on 18 SMs before.
-    if (MODE != MODE_POINTS && (a.ncap + NT * S - 1) / (NT * S) < vg_num_sms())
+    // (Not where hypercubes may have one sample or none: a tile takes as many
+    // hypercubes as samples.)
+    if (MODE != MODE_POINTS && !a.few && (a.ncap + NT * S - 1) / (NT * S) < vg_num_sms())
         return launch_tile_as<MODE, KIND, DIMB, 1, BASE_TILE>(a, prm, st, 0);
     return launch_tile_as<MODE, KIND, DIMB, S, NT>(a, prm, st, 1);
 }
