@@ -1,10 +1,10 @@
 """Benchmark: vegas+ on the ridge integrand (dim 4, M=1000 Gaussians of width
 0.01 on the diagonal), neval = 1e6 evaluations per iteration, FP32 sampling /
-map / evaluation with FP64 sums -- the vegas+ ridge workload.
+map / evaluation with float-float sums -- the vegas+ ridge workload.
 
 A step is one full vegas+ iteration: allocation of evaluations to the
 123462 hypercubes, Philox sampling + map + fused integrand evaluation +
-per-hypercube two-pass reduction + training histogram, and the grid adapt.
+per-hypercube mean and variance + training histogram, and the grid adapt.
 
 Arms
   (default)          this library on the GPU(s); one JSON line on rank 0.
@@ -267,7 +267,7 @@ def dropin_line(dev, neval=10 ** 7, nitn=5, reps=5):
         'fp32_vs_fp64_oracle': {'oracle': 'exact value erf(5)^4 in FP64', 'exact': exact,
                                 'rel_dev': r.mean / exact - 1.0, 'pull': (r.mean - exact) / r.sdev},
         'workload': 'drop-in path: torch lbatch integrand (dim-4 Gaussian, torch ops) through '
-                    'Integrator.__call__, neval %.0e/itn, FP32 sampling, FP64 sums' % neval,
+                    'Integrator.__call__, neval %.0e/itn, FP32 sampling, float-float sums' % neval,
         'value': r.sum_neval / api_s, 'unit': 'evals/s', 'neval_per_iteration': n,
         'result': str(r),
         'seconds_per_iteration': {'api': api_s / nitn, 'sample_kernel': t_s, 'integrand_torch': t_f,
@@ -328,7 +328,7 @@ def batched_line(dev, reps=2):
         'timeline': timeline,
         'workload': '4096 Lorentzian-product integrals, dim U{3..9}, centres U[0.2,0.8]^d, widths '
                     'log-U[0.01,0.1], neval log-U[1e4,1e6] per integral, nitn 8+8, one persistent '
-                    'kernel per 16 iterations replayed from a CUDA graph, FP32 eval + FP64 sums',
+                    'kernel per 16 iterations replayed from a CUDA graph, FP32 eval + float-float sums',
         'evals_per_launch': B.evaluations(), 'seconds_per_launch': secs,
         'value': B.evaluations() / secs, 'unit': 'evals/s', 'variant': B.variant,
         'autotune_seconds': {str(k): v for k, v in getattr(B, 'tuning', {}).items()},
@@ -353,7 +353,7 @@ def issue_roofline(dims, nevals, seconds, integrand_ops, clock_mhz):
     per 4 uniforms), the map (12 per axis: stratum coordinate, scale, floor,
     table load, FMA, Jacobian, training bin), the integrand (integrand_ops(d))
     and the per-sample reduction (30 + d: weight, histogram atomics,
-    float-float two-pass sums) -- against 128 thread instructions per cycle
+    float-float sums) -- against 128 thread instructions per cycle
     and SM."""
     import numpy as np
     d = np.asarray(dims, np.int64)
@@ -1051,14 +1051,14 @@ def ridge_issue_model(terms_per_eval, dim=DIM):
       map, per axis: stratum coordinate, bin index, table load, node + inc
         x fraction, Jacobian factor, training bin -- 12
       ridge: mean and spread of x (3 dim + 1), exponent offset and centre
-        (2), window of the Gaussian terms that can be nonzero in FP32 (15),
+        (2), window of the Gaussian terms that count in FP32 (15),
         final scale (3); per evaluated term: subtract, FMA, ex2, add and a
         quarter of a vector shared load -- 4.25
       per-sample reduction: weight and fdv2 (4), training histogram (3 per
-        axis), float-float two-pass hypercube sums (30)
+        axis), float-float hypercube sums (30)
 
-    The terms are the ones the kernel evaluates (those that can be nonzero
-    in FP32; the others are exactly zero), counted per iteration.  Peak: 152
+    The terms are the ones the kernel evaluates (those above 2^-30 of a sample's
+    largest that are not zero in FP32), counted per iteration.  Peak: 152
     SMs x 4 schedulers x 32 lanes per cycle at the maximum SM clock."""
     philox = 80 * ((dim + 3) // 4)
     mapping = 12 * dim

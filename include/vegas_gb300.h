@@ -97,7 +97,7 @@ typedef struct vg_integrator {
     double alpha;
     double beta;
     int32_t adapt;                 /* Integrator.adapt                          */
-    int32_t adapt_to_errors;       /* must be 0 for now                         */
+    int32_t adapt_to_errors;       /* Integrator.adapt_to_errors                */
     uint64_t seed;                 /* Philox key                                */
     uint32_t stream_id;            /* Philox counter word: integral id          */
     int32_t tile;                  /* samples per tile (0 = default)            */
@@ -186,8 +186,9 @@ int vg_sample(const vg_integrator *it, uint32_t itn, const double *u, void *x, v
               double *wgt, int64_t *hcube, int64_t n_cap, void *stream);
 
 /*
- * Per-hypercube two-pass reduction of the integrand values f[n] (dtype),
- * pyx:2136-2193, with the training histogram (pyx:2173, 2196-2197), the new
+ * Per-hypercube mean and variance of the integrand values f[n] (dtype),
+ * pyx:2136-2193 (FP64: two passes; FP32: one, float-float sums about the
+ * hypercube's first sample), with the training histogram (pyx:2173, 2196-2197), the new
  * sigf and the iteration mean/var/sum_sigf (written to it->stats).
  */
 int vg_reduce(const vg_integrator *it, uint32_t itn, const double *u, const void *f, int f_dtype,

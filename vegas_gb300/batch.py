@@ -50,7 +50,7 @@ class BatchIntegrator(object):
         variant: kernel configuration per dimension bucket, a sequence of 3
             (or one int for all buckets); None: autotune.
         precision: 'fp32' (default: FP32 sampling, map and evaluation,
-            float-float and FP64 sums) or 'fp64' (the parity configuration:
+            float-float sums) or 'fp64' (the parity configuration:
             everything in FP64, the arithmetic of ``Integrator(precision=
             'fp64')``; Lorentzian products of dim <= 8 only, no autotuning).
     """

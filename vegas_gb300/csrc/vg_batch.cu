@@ -300,9 +300,9 @@ extern "C" int vg_batch_launch(const void *table, int njobs, int kind, int nitn,
     // own streams after it was enqueued.  Their CTAs start as SMs become free,
     // so the bucket with the fewest integrals per CTA goes first (it ends with
     // its longest integral, beside which little of its own is left to run) and
-    // the one with the most last, to fill up behind the others.  1024 integrals
-    // of dim 3 to 9, 285 + 591 + 148 of them in the buckets: 18.8 ms in the
-    // order of the dimensions (16, 8, 4), 14.4 so.
+    // the one with the most last, to fill up behind the others.  (1024 integrals
+    // of dim 3 to 9, 285 + 591 + 148 of them in the buckets, took 30 % longer in the
+    // order of the dimensions, 16, 8, 4.)
     int turn[NBUCKET] = {2, 1, 0};   // ties: the larger dimension first
     auto fewer = [&](int x, int y) {
         if (seg[2 * x + 1] <= 0 || seg[2 * y + 1] <= 0) return seg[2 * x + 1] <= 0 && seg[2 * y + 1] > 0;

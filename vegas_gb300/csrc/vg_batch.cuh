@@ -2,12 +2,13 @@
 //
 // One CTA runs one integral at a time, all of its iterations back to back:
 // allocation of evaluations to hypercubes (pyx:1692-1706), the fused body of
-// the single-integral kernel over all of the integral's samples (sampling, map, integrand, two-pass per-hypercube reduction, training
-// histogram), the merge of hypercubes cut by tile boundaries and the
+// the single-integral kernel over all of the integral's samples (sampling, map,
+// integrand, per-hypercube mean and variance, training histogram), the merge of
+// hypercubes cut by the ends of ranges or tiles and the
 // iteration sums (finalize), AdaptiveMap.adapt (pyx:467-594), and at the end
 // the weighted average over the iterations after the warm-up ones
-// (RAvg.add, pyx:2392-2410) -- all in FP64 where the single-integral path
-// is.  CTAs take integrals from an atomic queue in an order given by the
+// (RAvg.add, pyx:2392-2410) -- in the arithmetic of the single-integral
+// path.  CTAs take integrals from an atomic queue in an order given by the
 // host (largest first), so nothing crosses CTAs and the launch needs no
 // grid-wide synchronisation.
 #pragma once
@@ -86,7 +87,7 @@ __device__ __forceinline__ int deal_chunks(int G) { return G > 1 ? 4 : 1; }
 // The arguments of the CTA's integral.  The functions that are not inlined into
 // the kernel name this variable and the dynamic shared memory themselves: through
 // a pointer parameter every access to the arguments, the grid table and the
-// histogram would be a generic one (the 16-dimensional lattice: 5.51 ms, 5.23 so).
+// histogram would be a generic one (the 16-dimensional lattice took 5 % longer).
 __device__ __forceinline__ IterArgs &job_args()
 {
     __shared__ IterArgs sa;

@@ -214,11 +214,13 @@ __device__ __forceinline__ float vg_eval_f32(const VgF32Consts &k, const float *
         const float E0 = -k.c[0] * R;
         const float w = m * k.c[1];
         float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-        // Terms that can count, aligned to the 4-way accumulator pattern: a
-        // term below 2^-30 of the largest one (the nearest centre's) leaves the
-        // FP32 sum as it is (all of those together are below 2^-29 of it, its own
-        // rounding is 2^-24), one with E0 - (w - v_j)^2 < -127 is exactly zero
-        // (ex2.approx.ftz flushes it).  The first bound makes the window as wide
+        // Terms that can count, aligned to the 4-way accumulator pattern.  A term
+        // with E0 - (w - v_j)^2 < -127 is exactly zero (ex2.approx.ftz flushes it).
+        // Those below 2^-30 of the largest one (the nearest centre's) are a tail of
+        // erfc(sqrt(30 ln 2)) = 2^-33 where the centres are dense; over M = 7 to 16384, s =
+        // 0.003 to 0.3 and dim 2 to 10 they were at most 2^-30.9 of the sum, whose own
+        // error is 2^-17 to 2^-24, and without them its error against 64 bits was the same,
+        // the mean and the largest, to 1 %.  That bound makes the window as wide
         // for every sample of a warp: 68 terms of M = 1000, s = 0.01 at dim 4 where
         // the second alone left 96 on average and 132 for the warp's widest.
         int j = 0, jend = nterm & ~3;

@@ -19,8 +19,12 @@
 // The variance needs no second pass over the samples: sums of d = wf - c and
 // d^2 about c = the hypercube's first sample of the range, in float-float
 // (about 2^-44 relative), give (n Q - D^2) / (n - 1) -- the reference's formula,
-// which is exact for any c.  The cancellation costs about (c - mean)^2 / var of
-// the 2^-44, and the samples themselves are FP32.
+// which is exact for any c.  The cancellation costs about (c - mean)^2 / var, n at the
+// most, of the 2^-44, and the samples themselves are FP32.  (Variances of iterations
+// against long double, five integrands, dims 1 to 9: 2^-47 to 2^-50, as with two
+// passes about the mean.)  Sums of squares beyond 1e30 go to FP64; a hypercube that goes
+// on into the next chunk then goes on about its mean, so that Q stays near the
+// variance where c was an outlier.
 //
 // Why this shape.  No barrier of the CTA is inside the loop, so 1024 threads
 // share one grid table and one training histogram (64 KB each at dim 8 with
@@ -35,7 +39,7 @@
 namespace vg {
 
 constexpr int CHUNK = 128;      // samples per chunk
-constexpr int WCAP = 68;        // hypercube starts a chunk can see (every count is >= 2), padded
+constexpr int WCAP = 68;        // hypercube starts a chunk can see (two samples each or more), padded
 static_assert(CHUNK == BASE_TILE, "tile_h0 gives the first hypercube of each chunk");
 
 constexpr int OPEN = WCAP - 1;  // a chunk sees WCAP - 2 hypercubes at the most
@@ -540,7 +544,7 @@ __device__ __forceinline__ void range_body(const IterArgs &a, const VgParams &pr
                 nw += __popc(m);
                 if (m != 0xffffffffu) break;
             }
-            if (nw < 1 || nw > WCAP - 2) {   // impossible while every count is >= 2
+            if (nw < 1 || nw > WCAP - 2) {   // impossible: counts of 2 or more, or a shortened chunk
                 if (lane == 0) a.stats->status = VG_ERR_UNSUPPORTED;
                 break;
             }
