@@ -820,26 +820,32 @@ class Integrator(object):
             sigf.copy_(s_, non_blocking=True)
             cur.synchronize()
 
-        enqueue(0)
-        for k in range(nitn):
-            ahead = k + 1 < nitn
-            if ahead:
-                enqueue(k + 1)
-            done[k % 2].synchronize()
-            st = N.VgStats.from_buffer_copy(host[k % 2].numpy().tobytes()[:sz])
-            self._itn = itn0 + k + 1
-            try:
-                self._take_record(st)
-            except Exception:
+        try:
+            enqueue(0)
+            for k in range(nitn):
+                ahead = k + 1 < nitn
                 if ahead:
-                    undo(k)
-                raise
-            result.add(gv.gvar(st.mean, st.var ** 0.5))
-            result.sum_neval += self.last_neval
-            if result.converged(self.rtol, self.atol):
-                if ahead:
-                    undo(k)
-                break
+                    enqueue(k + 1)
+                done[k % 2].synchronize()
+                st = N.VgStats.from_buffer_copy(host[k % 2].numpy().tobytes()[:sz])
+                self._itn = itn0 + k + 1
+                try:
+                    self._take_record(st)
+                except Exception:
+                    if ahead:
+                        undo(k)
+                    raise
+                result.add(gv.gvar(st.mean, st.var ** 0.5))
+                result.sum_neval += self.last_neval
+                if result.converged(self.rtol, self.atol):
+                    if ahead:
+                        undo(k)
+                    break
+        except BaseException:
+            # an iteration in flight writes its record to memory that may be
+            # freed (and used again) once this call is left
+            cur.synchronize()
+            raise
         return result
 
     # --------------------------------------------------------------- report
